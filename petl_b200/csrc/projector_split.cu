@@ -11,17 +11,21 @@
 // * k_xshift writes X for a chunk of views into FP32 scratch, [view][y][z][c]
 //   (memory bound: one write of a volume per view; each volume row is read
 //   once per chunk);
-// * k_fwd_zsum applies the z taps.  CTA = one view x 16 slopes x 32 rows x 64
-//   columns, 16 warps of 4 slopes x 8 rows x 2 columns per lane.  The staged
-//   rows of each plane arrive by a tiled TMA copy (no multicast) into a ring
-//   of two stages of two planes with full/empty mbarriers; the copy of a stage is
-//   started by a rotating warp once every warp has released the slot, so no
-//   CTA-wide barrier sits in the plane loop.  The window offset, tap offsets
-//   and weights of every (plane, slope group) are tabulated once per CTA.
-//   The tap offsets of a warp's four consecutive slopes move by at most one
-//   row from slope to slope, so they form one of 15 monotone patterns: one
-//   dispatch per plane selects a fully unrolled form (four per-slope
-//   dispatches measured 10 % slower); other groups take the per-slope form.
+// * k_fwd_zsum applies the z taps: persistent CTAs of twelve consumer warps
+//   and a producer warp that stages planes by tiled TMA copies (no multicast)
+//   into a ring with full/empty mbarriers, across tile borders.  The tap
+//   offsets of a warp's four consecutive slopes move by at most one row from
+//   slope to slope, so they form one of 15 monotone patterns: one dispatch per
+//   plane selects a fully unrolled form.
+//
+// 256x256x128, planogram (65, 129, 128, 256): 7.7 ms for the z taps and 0.7
+// for the x pass (before: 10.0 and 0.9, with one 16-warp CTA per tile, tables
+// built by every CTA, scalar FMAs on 8 rows per warp and tiles that started at
+// bin 0).  What the steps gave on the z taps: twelve warps x 12 rows against
+// eight x 16 9 %, tiles handed out by a counter against a fixed stride 18 % (the
+// stride of 148 met the period of the column blocks, whose last is often
+// empty), a rolled epilogue 10 % and its loads in batches another 25 % where
+// the MLEM ratio is computed.
 //
 // Both kernels do the float operations of project_tma in the same order (x
 // taps fmaf(w1, b, w0 * a); per ray, the z taps of the live planes in
@@ -42,6 +46,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstdlib>
+#include <cstring>
 #include <mutex>
 #include <string>
 
@@ -50,32 +55,62 @@
 #include "shear.cuh"
 #include "storage.cuh"
 #include "tma.cuh"
+#include "ztaps.cuh"
 
 namespace petl {
 namespace shear {
 
 namespace {
 
-constexpr int ZV = 4;                 // slopes per warp
-constexpr int ZK = 8;                 // rows per warp
-constexpr int ZSG = 4;                // slope groups of a full block (warps along v1)
-constexpr int ZSL = ZV * ZSG;         // slopes of a full block
-constexpr int ZCOLS = 64;             // columns per CTA, two per lane
-constexpr int ZWARPS = 16;
-constexpr int ZNT = 32 * ZWARPS;
-constexpr int ZDMAX = 3;              // largest shift difference among a warp's slopes
-constexpr int ZWN = ZK + ZDMAX + 1;   // register window rows
-// ring stages (of two planes each): three measured 0.9 % faster than two at
-// the 256x256x128 workload once the tap offsets were dispatched per plane
-// (before that, deeper rings ran 1-3 % slower)
-constexpr int ZNSMAX = 3;
-constexpr int ZMAXPLANES = 1024;      // planes the per-CTA tables hold
+constexpr int ZSLOPES = 16;           // slopes per block at most (a table record holds 16 weights)
+constexpr int ZMAXROWS = 15000;       // rows of volume and planogram at most (16-bit row shifts)
+constexpr int XZB = 8;                // volume rows z per k_xshift block
+constexpr int XMAXNX = 1024;          // longest volume row k_xshift stages
 
-// code word of a (plane, slope group): tap offsets (2 bits per slope), the
-// window's first staged row (bits 8..15), per row group "window outside the
-// volume" (bits 16..31)
-constexpr int kCodeRowShift = 8;
-constexpr int kCodeSkipShift = 16;
+// Table record of one (slope block, plane), staged with the plane: the second
+// tap's weight of each slope, and per slope group (warp) the tap offsets (2
+// bits per slope), the window's first staged row << 8 and the shift of that
+// row << 16.
+struct __align__(16) ZRec {
+    float w[ZSLOPES];
+    uint32_t code[kZWarps];
+};
+
+// Blocks of slopes that share a launch shape: sg slope groups (warps along
+// v1) x rg row groups (warps along u1).
+struct ZKind {
+    int v1_first, v1_end;
+    int sg, rg, rows;  // rows = NK * rg
+    int nblk;          // slope blocks
+    int n_rowblk;      // row blocks at most (the visible rows of a block need fewer)
+    int nrb;           // staged rows per plane (rows + shift spread of the block + 1)
+    int pstride;       // floats per staged plane (nrb + kZSpread rows of 64)
+    int pps;           // planes per stage: two, or one of the tail's tall planes
+    int blk0;          // index of the first block in the tables
+    int ntile;
+};
+
+struct ZsumArgs {
+    petl_geom G;
+    int step;       // view step of the members' view ranges
+    int nw;         // consumer warps
+    int nslot;      // view slots of all members
+    int n_colblk;   // column blocks at most
+    int ns;         // ring stages, two planes each
+    int stage;      // bytes per stage (planes, then two records)
+    ZKind k[2];     // full blocks, and the tail of at most half a block
+    ZRec* rec;      // [block][plane]
+    int* dz;        // [block][plane] smallest shift of the block
+    int* next;      // tiles handed out beyond one per CTA
+    Tables T;
+    int* err;
+    unsigned wait_limit;  // bound of the waits on staged data (wait_limit(): kWaitLimit or 0)
+    Members M;            // planograms (out), measured planograms (meas) and views of the chunk
+};
+
+struct ZMaps {
+    CUtensorMap m[2];  // X with the box of each kind
+};
 
 struct XshiftArgs {
     petl_geom G;
@@ -83,15 +118,64 @@ struct XshiftArgs {
     int NXc;   // scratch row pitch (columns, a multiple of 4)
     Tables T;
     Members M;  // volumes (in) and views of the chunk
+    ZKind k[2];
+    int nv;     // slopes per group
+    ZRec* rec;
+    int* dz;
+    int* next;
+    int* err;
 };
 
-constexpr int XZB = 8;      // volume rows z per k_xshift block
-constexpr int XMAXNX = 1024;  // longest volume row k_xshift stages
+// Table records of plane y for every slope block of the call.
+__device__ void z_records(const XshiftArgs& A, int y)
+{
+    const int NY = A.G.numY, nv = A.nv;
+    const int nblk = A.k[0].nblk + A.k[1].nblk;
+    for (int e = threadIdx.x; e < nblk * kZWarps; e += blockDim.x) {
+        const int blk = e / kZWarps, q = e - blk * kZWarps;
+        const ZKind& K = A.k[blk < A.k[0].nblk ? 0 : 1];
+        const int v1a = K.v1_first + (blk - K.blk0) * nv * K.sg;
+        const int v1b = min(v1a + nv * K.sg, K.v1_end);
+        // the shifts are monotone in v1
+        const int da = A.T.zt[size_t(v1a) * NY + y].d, db = A.T.zt[size_t(v1b - 1) * NY + y].d;
+        const int dmin = min(da, db);
+        ZRec* R = A.rec + size_t(blk) * NY + y;
+        uint32_t code = 0;
+        const int j0 = v1a + q * nv, j1 = min(j0 + nv, v1b);
+        if (j0 < v1b) {
+            int base = 1 << 30;
+            for (int j = j0; j < j1; j++) base = min(base, A.T.zt[size_t(j) * NY + y].d);
+            int xoff = base - dmin;
+            bool bad = xoff < 0 || max(da, db) - dmin + K.rows + 1 > K.nrb;
+            code = (uint32_t(uint16_t(int16_t(base))) << 16);
+            for (int j = j0; j < j1; j++) {
+                const Shift zs = A.T.zt[size_t(j) * NY + y];
+                if (zs.d - base > kZSpread) bad = true;
+                code |= uint32_t(min(zs.d - base, kZSpread)) << (2 * (j - j0));
+                R->w[q * nv + j - j0] = zs.w;
+            }
+            if (bad) {  // a host-side bound does not hold: stay inside the staged rows
+                atomicOr(A.err, kErrLayout);
+                xoff = 0;
+            }
+            // slopes beyond the last one: a pattern of the present ones, no weight
+            for (int j = j1; j < j0 + nv; j++) {
+                code |= ((code >> (2 * (j1 - 1 - j0))) & 3u) << (2 * (j - j0));
+                R->w[q * nv + j - j0] = 0.0f;
+            }
+            code |= uint32_t(xoff) << 8;
+        }
+        if (q < K.sg) R->code[q] = code;
+        if (q == 0) A.dz[size_t(blk) * NY + y] = dmin;
+    }
+}
 
 // X rows of a chunk of views.  A block stages rows z0..z0+7 of plane y of
 // one member's volume in shared memory once and writes them shifted for
 // every view of that member in the chunk, one float4 of columns per thread
-// and step.  Grid (ceil(NZ / 8), NY, members).
+// and step; columns whose rays are all masked are left out.  Bound by its
+// writes of the scratch.  The first block of a plane also writes the plane's
+// table records.  Grid (ceil(NZ / 8), NY, members).
 template <class TF, int NM>
 __global__ void __launch_bounds__(256) k_xshift(float* __restrict__ X, const XshiftArgs A)
 {
@@ -101,7 +185,6 @@ __global__ void __launch_bounds__(256) k_xshift(float* __restrict__ X, const Xsh
     const int y = blockIdx.y, z0 = blockIdx.x * XZB;
     const int b = NM == 1 ? 0 : int(blockIdx.z);
     const int nz = min(XZB, NZ - z0);
-    const int nq = A.NXc >> 2;  // float4 columns per row
     const TF* __restrict__ f = static_cast<const TF*>(member_pick<NM>(A.M.in, b));
     for (int e = threadIdx.x; e < nz * NX; e += blockDim.x) {
         const int r = e / NX, x = e - r * NX;
@@ -110,11 +193,15 @@ __global__ void __launch_bounds__(256) k_xshift(float* __restrict__ X, const Xsh
     __syncthreads();
     const int first = member_pick<NM>(A.M.first, b), nvb = member_pick<NM>(A.M.nv, b);
     for (int iv = 0; iv < nvb; iv++) {
-        const Shift xs = A.T.xt[size_t(first + iv * A.step) * NY + y];
+        const int v0 = first + iv * A.step;
+        const Shift xs = A.T.xt[size_t(v0) * NY + y];
+        const int2 ub0 = A.T.ub0[v0];
+        const int c0 = ub0.x & ~3;
+        const int nq = ub0.y < ub0.x ? 0 : ((ub0.y - c0) >> 2) + 1;  // float4 columns per row
         const float w1 = xs.w, w0 = 1.0f - xs.w;
         float* Xv = X + (size_t(b * A.M.nvm + iv) * NY + y) * NZ * A.NXc;
         for (int e = threadIdx.x; e < nz * nq; e += blockDim.x) {
-            const int r = e / nq, c = (e - r * nq) * 4;
+            const int r = e / nq, c = c0 + (e - r * nq) * 4;
             const float* fr = rowbuf + r * NX;
             float v[5];
 #pragma unroll
@@ -128,397 +215,384 @@ __global__ void __launch_bounds__(256) k_xshift(float* __restrict__ X, const Xsh
             __stcs(reinterpret_cast<float4*>(Xv + size_t(z0 + r) * A.NXc + c), o);
         }
     }
+    if (blockIdx.x == 0 && b == 0) z_records(A, y);
+    if (blockIdx.x == 0 && y == 0 && b == 0 && threadIdx.x == 0) *A.next = 0;
 }
 
-struct ZsumArgs {
-    petl_geom G;
-    int step;      // view step of the members' view ranges
-    int v1_first;  // first slope of the launch's slope blocks
-    int v1_end;    // one past its last slope
-    int sg;        // slope groups per CTA (4; 1 or 2 for a tail block of at most 8 slopes)
-    int n_colblk;  // ceil(N_u0 / 64)
-    int n_rowblk;  // ceil(N_u1 / rows per CTA)
-    int nrb;       // staged rows per plane (rows per CTA + CTA shift spread + 1, bounded on the host)
-    int ns;        // ring stages, two planes each
-    int pstride;   // floats per staged plane (nrb + ZDMAX rows of 64; a multiple of 32)
-    // shared-memory layout (byte offsets, set by the host): weights, codes,
-    // live planes, barriers
-    unsigned off_w, off_code, off_plane, off_bar;
-    Tables T;
-    int* err;
-    unsigned wait_limit;  // bound of the waits on staged data (wait_limit(): kWaitLimit or 0)
-    Members M;  // planograms (out), measured planograms (meas) and views of the chunk
-};
-
-// z taps of one slope: all first-tap FMAs, then all second-tap FMAs (16
-// independent chains per pass)
-template <int O>
-__device__ __forceinline__ void zsum_taps(float2 (&acc)[ZK], const float2 (&W)[ZWN], float2 w0, float2 w1)
-{
-#pragma unroll
-    for (int k = 0; k < ZK; k++) acc[k] = fma2(w0, W[k + O], acc[k]);
-#pragma unroll
-    for (int k = 0; k < ZK; k++) acc[k] = fma2(w1, W[k + O + 1], acc[k]);
-}
-
-// z taps of the four slopes of a warp with compile-time tap offsets
-// (PC: 2 bits per slope), each slope's FMAs as zsum_taps orders them.
-template <int PC>
-__device__ __forceinline__ void zsum4(float2 (&acc)[ZV][ZK], const float2 (&W)[ZWN], const float (&wj)[ZV])
-{
-    zsum_taps<(PC >> 0) & 3>(acc[0], W, dup(1.0f - wj[0]), dup(wj[0]));
-    zsum_taps<(PC >> 2) & 3>(acc[1], W, dup(1.0f - wj[1]), dup(wj[1]));
-    zsum_taps<(PC >> 4) & 3>(acc[2], W, dup(1.0f - wj[2]), dup(wj[2]));
-    zsum_taps<(PC >> 6) & 3>(acc[3], W, dup(1.0f - wj[3]), dup(wj[3]));
-}
-
+// The z taps: g[v1][v0][iu1][c] = S sum_y (1 - w) X[y][iu1 + d] + w X[y][iu1 + d + 1].
+//
+// Persistent CTAs of nw consumer warps and a producer warp.  A tile is one
+// view x one slope block x rows x 64 columns, placed at the first visible row
+// of the block and the first visible column of the view (masked rays are
+// written as zeros by the tiles at the edge, not computed); a warp sums NV
+// slopes x NK rows x 2 columns per lane over the planes.  The producer walks
+// the tiles and stages their planes two at a time, rows by a tiled TMA copy
+// (no multicast) and the planes' table records by a bulk copy, ahead of the
+// consumers across tile borders, so set-up and epilogue of a warp overlap the
+// sums of the others.
+//
+// Bound by FP32 issue: a plane costs a warp 96 packed FMAs (192 cycles of its
+// scheduler, which holds three such warps) and 16 eight-byte window loads (32
+// cycles of the SM's shared memory, of which twelve warps take 384 of the 576
+// cycles the FMAs take).  Measured 850 cycles per plane: the dispatch, the
+// window's first loads and the ring's waits are not fully covered.  4 slopes x
+// 16 rows in eight warps need fewer loads per FMA but ran at 800 cycles for
+// 512 of FMAs; 8 rows and 16 warps are bound by the loads.
 // TG: planogram storage (float or bfloat16); X and the arithmetic are FP32.
-// Warp w: slope group w % sg, row group w / sg.  The copy of stage j is
-// started by lane 0 of warp j % 16 once every warp has released the slot.
-template <class TG, int NM>
-__global__ void __launch_bounds__(ZNT, 1)
-k_fwd_zsum(const __grid_constant__ CUtensorMap xmap, const ZsumArgs A)
+template <class TG, int NM, int NV, int NK>
+__global__ void __launch_bounds__(kZThreads, 1)
+k_fwd_zsum(const __grid_constant__ ZMaps maps, const __grid_constant__ ZsumArgs A)
 {
+    constexpr int WN = NK + kZSpread + 1;
     extern __shared__ __align__(128) unsigned char smem[];
+    ZCtl* ctl = reinterpret_cast<ZCtl*>(smem + size_t(A.ns) * A.stage);
+    ZStage* s_info = ctl->info;
+    uint64_t *full = ctl->full, *empty = ctl->empty;
+    volatile int* s_abort = &ctl->abort;
     const petl_geom& G = A.G;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int sg = A.sg, rows = ZK * (ZWARPS / sg);
-    const int gv = warp % sg, gr = warp / sg;
-    const int vi = blockIdx.y;  // view slot within the chunk
-    const int mb = NM == 1 ? 0 : vi / A.M.nvm, mv = vi - mb * A.M.nvm;
-    if (mv >= member_pick<NM>(A.M.nv, mb)) return;  // a member with fewer views than the slots
-    const int iv0 = member_pick<NM>(A.M.first, mb) + mv * A.step;
-    TG* __restrict__ g = static_cast<TG*>(member_pick<NM>(A.M.out, mb));
-    const TG* __restrict__ meas = static_cast<const TG*>(member_pick<NM>(A.M.meas, mb));
-    int t = blockIdx.x;
-    const int colblk = t % A.n_colblk;
-    t /= A.n_colblk;
-    const int rowblk = t % A.n_rowblk;
-    t /= A.n_rowblk;
-    const int v1a = A.v1_first + t * (ZV * sg);
-    const int v1b = min(v1a + ZV * sg, A.v1_end) - 1;  // last slope of the CTA
-    const int nsl = v1b - v1a + 1;
-    const int cta_row0 = rowblk * rows, col0 = colblk * ZCOLS;
-    const int jw = gv * ZV;              // first slope of this warp, relative to v1a
-    const int row0 = cta_row0 + gr * ZK;  // first row of this warp
-    const int NY = G.numY, NZ = G.numZ, NX = G.numX;
-    const int ns = A.ns, npl = min(NY, ZMAXPLANES);
-
-    float* ringp = reinterpret_cast<float*>(smem);                      // [ns][2][pstride]
-    float4* s_w1 = reinterpret_cast<float4*>(smem + A.off_w);            // [npl][4]
-    uint32_t* s_code = reinterpret_cast<uint32_t*>(smem + A.off_code);   // [npl][4]
-    int2* s_plane = reinterpret_cast<int2*>(smem + A.off_plane);         // [npl] (y, first staged row)
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + A.off_bar);      // [ZNSMAX]
-    uint64_t* empty = full + ZNSMAX;                                     // [ZNSMAX]
-    int* s_n = reinterpret_cast<int*>(empty + ZNSMAX);
-    volatile int* s_abort = s_n + 1;  // a consumer gave up a wait: start no further copies
-    int* s_round = s_n + 2;           // [ZNSMAX] round of the copy last started in a slot
-
-    // a tile outside the visible bins of every slope stays zero
-    const int2 ub0 = A.T.ub0[iv0];
-    bool any_row = false;
-    for (int v1 = v1a; v1 <= v1b; v1++) {
-        const int2 u = A.T.ub1[v1];
-        any_row |= !(cta_row0 > u.y || cta_row0 + rows - 1 < u.x);
+    const int NY = G.numY, NZ = G.numZ, NX = G.numX, ns = A.ns;
+    if (tid == 0) {
+        *s_abort = 0;
+        for (int s = 0; s < ns; s++) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], A.nw);
+        }
+        fence_barrier_init();
     }
-    const bool live = any_row && !(col0 > ub0.y || col0 + ZCOLS - 1 < ub0.x);
+    __syncthreads();
 
-    // slopes of this warp whose rows can be visible
-    unsigned wmask = 0;
-#pragma unroll
-    for (int j = 0; j < ZV; j++) {
-        if (jw + j < nsl) {
-            const int2 u = A.T.ub1[v1a + jw + j];
-            if (!(row0 > u.y || row0 + ZK - 1 < u.x)) wmask |= 1u << j;
+    if (warp >= A.nw) {
+        producer_registers();
+        if (warp > A.nw) {
+            __syncthreads();
+            return;
         }
-    }
-
-    float2 acc[ZV][ZK];
-#pragma unroll
-    for (int j = 0; j < ZV; j++)
-#pragma unroll
-        for (int k = 0; k < ZK; k++) acc[j][k] = make_float2(0.0f, 0.0f);
-
-    if (live) {  // CTA-uniform
-        // planes whose staged window meets the volume, compacted in order
-        if (warp == 0) {
-            int n = 0;
-            for (int yb = 0; yb < NY; yb += 32) {
-                const int y = yb + lane;
-                bool ok = false;
-                int wlo = 0;
-                if (y < NY) {
-                    const Shift xs = A.T.xt[size_t(iv0) * NY + y];
-                    const int da = A.T.zt[size_t(v1a) * NY + y].d, db = A.T.zt[size_t(v1b) * NY + y].d;
-                    const int dzmin = min(da, db);
-                    const int nr = rows + (max(da, db) - dzmin) + 1;
-                    const int cx = col0 + xs.d;
-                    wlo = cta_row0 + dzmin;
-                    ok = !(cx + ZCOLS < 0 || cx >= NX || wlo + nr - 1 < 0 || wlo >= NZ);
-                    if (ok && nr > A.nrb) {
-                        atomicOr(A.err, kErrLayout);
-                        ok = false;
-                    }
-                }
-                const unsigned b = __ballot_sync(0xffffffffu, ok);
-                const int idx = n + __popc(b & ((1u << lane) - 1u));
-                if (ok && idx < npl) s_plane[idx] = make_int2(y, wlo);
-                n += __popc(b);
-            }
-            if (lane == 0) {
-                if (n > npl) {  // the host bounds numY; never index past the tables
-                    atomicOr(A.err, kErrLayout);
-                    n = npl;
-                }
-                s_n[0] = n;
-                *s_abort = 0;
-                for (int s = 0; s < ns; s++) {
-                    mbar_init(&full[s], 1);
-                    mbar_init(&empty[s], ZWARPS);
-                    s_round[s] = -1;
-                }
-                fence_barrier_init();
-            }
-        }
-        __syncthreads();
-        const int nlive = s_n[0];
-
-        // per (plane, slope group): window row, tap offsets, skip bits, weights
-        for (int e = tid; e < nlive * sg; e += ZNT) {
-            const int li = e / sg, q = e - li * sg;
-            const int2 pl = s_plane[li];
-            const int y = pl.x, wlo = pl.y;
-            const int dzmin = wlo - cta_row0;
-            int d[ZV];
-            float w[ZV];
-            int base = 1 << 30;
-#pragma unroll
-            for (int j = 0; j < ZV; j++) {
-                d[j] = 0;
-                w[j] = 0.0f;
-                if (q * ZV + j < nsl) {
-                    const Shift zs = A.T.zt[size_t(v1a + q * ZV + j) * NY + y];
-                    d[j] = zs.d;
-                    w[j] = zs.w;
-                    base = min(base, zs.d);
-                }
-            }
-            uint32_t code = 0xffffu << kCodeSkipShift;  // no slope in this group
-            if (base != (1 << 30)) {
-                const int xoff = base - dzmin;  // >= 0: the shifts are monotone in v1
-                // the window of the last row group ends inside the plane's rows (nrb + ZDMAX)
-                if (xoff < 0 || xoff + rows - ZK + ZWN > A.nrb + ZDMAX || xoff > 255) {
-                    atomicOr(A.err, kErrLayout);
-                } else {
-                    code = uint32_t(xoff) << kCodeRowShift;
-#pragma unroll
-                    for (int j = 0; j < ZV; j++) {
-                        if (q * ZV + j >= nsl) continue;
-                        const int o = d[j] - base;
-                        if (o > ZDMAX) atomicOr(A.err, kErrLayout);
-                        code |= uint32_t(min(o, ZDMAX)) << (2 * j);
-                    }
-                    for (int r = 0; r < ZWARPS / sg; r++) {
-                        const int iz0 = wlo + xoff + r * ZK;  // volume row of window row 0
-                        if (iz0 + ZWN - 1 < 0 || iz0 >= NZ) code |= 1u << (kCodeSkipShift + r);
-                    }
-                }
-            }
-            s_code[li * 4 + q] = code;
-            s_w1[li * 4 + q] = make_float4(w[0], w[1], w[2], w[3]);
-        }
-        __syncthreads();
-
-        const int nst = (nlive + 1) / 2;  // ring stages of this CTA
-        const uint32_t box_bytes = uint32_t(ZCOLS) * uint32_t(A.nrb) * 4u;
+        int j = 0;       // stages started
         bool dead = false;
-        // stage j holds planes 2j and 2j + 1; it reuses its slot once every
-        // warp has released stage j - ns
-        auto issue = [&](int j) {
+        const int ntile = A.k[0].ntile + A.k[1].ntile;
+        // waits until the slot of stage j is free (lane 0)
+        auto claim = [&]() {
             const int slot = j % ns, round = j / ns;
-            if (round > 0 && !mbar_wait(&empty[slot], uint32_t((round - 1) & 1), A.err, A.wait_limit)) return false;
-            if (*s_abort) return false;
-            fence_proxy_async_smem();
-            const int np = min(2, nlive - 2 * j);
-            mbar_arrive_expect_tx(&full[slot], box_bytes * uint32_t(np));
-            for (int h = 0; h < np; h++) {
-                const int2 pl = s_plane[2 * j + h];
-                tma_load_4d(ringp + size_t(2 * slot + h) * A.pstride, &xmap, &full[slot], col0, pl.y, pl.x, vi);
-            }
-            s_round[slot] = round;
-            return true;
+            if (round > 0 && !ring_wait(&empty[slot], uint32_t((round - 1) & 1), A.err, s_abort, A.wait_limit))
+                return false;
+            return *s_abort == 0;
         };
-        if (tid == 0)
-            for (int j = 0; j < ns - 1 && j < nst; j++) issue(j);
-        // the next stage this warp starts: the first j >= ns - 1 with j % 16 == warp
-        int my_next = warp + ZWARPS * ((ns - 1 - warp + ZWARPS - 1) / ZWARPS);
-        if (my_next < ns - 1) my_next += ZWARPS;
-        int slot = 0;
-        uint32_t phase = 0;
-        for (int j = 0; j < nst; j++) {
-            if (j + ns - 1 == my_next) {
-                if (lane == 0 && !dead && my_next < nst && !issue(my_next)) dead = true;
-                my_next += ZWARPS;
+        int after = 0;  // the tile after the current one (lane 0)
+        for (int tile = blockIdx.x; tile < ntile && !dead; tile = __shfl_sync(0xffffffffu, after, 0)) {
+            if (lane == 0) after = int(gridDim.x) + atomicAdd(A.next, 1);
+            const int kind = tile < A.k[0].ntile ? 0 : 1;
+            const ZKind& K = A.k[kind];
+            int t = tile - (kind ? A.k[0].ntile : 0);
+            const int colblk = t % A.n_colblk;
+            t /= A.n_colblk;
+            const int rowblk = t % K.n_rowblk;
+            t /= K.n_rowblk;
+            const int blk = t % K.nblk, vi = t / K.nblk;  // slope block, view slot
+            const int mb = NM == 1 ? 0 : vi / A.M.nvm, mv = vi - mb * A.M.nvm;
+            if (mv >= member_pick<NM>(A.M.nv, mb)) continue;  // a member with fewer views than the slots
+            const int iv0 = member_pick<NM>(A.M.first, mb) + mv * A.step;
+            const int nsl = NV * K.sg, v1a = K.v1_first + blk * nsl, v1b = min(v1a + nsl, K.v1_end);
+            // visible columns of the view and visible rows of the block
+            const int2 ub0 = A.T.ub0[iv0];
+            int lo = 1 << 30, hi = -1;
+            if (v1a + lane < v1b) {
+                const int2 u = A.T.ub1[v1a + lane];
+                if (u.x <= u.y) lo = u.x, hi = u.y;
             }
-            if (!dead) dead = !mbar_wait(&full[slot], phase, A.err, A.wait_limit);
-            if (dead) *s_abort = 1;  // before this warp releases the slot
-#pragma unroll 1
-            for (int h = 0; h < 2 && !dead; h++) {
-                const int li = 2 * j + h;
-                if (li >= nlive) break;
-                const uint32_t code = s_code[li * 4 + gv];
-                if (!wmask || ((code >> (kCodeSkipShift + gr)) & 1u)) continue;
-                const float4 w1 = s_w1[li * 4 + gv];
-                const float wj[ZV] = {w1.x, w1.y, w1.z, w1.w};
-                const float* Xr = ringp + size_t(2 * slot + h) * A.pstride +
-                                  (int((code >> kCodeRowShift) & 0xffu) + gr * ZK) * ZCOLS + 2 * lane;
-                float2 W[ZWN];
-#pragma unroll
-                for (int i = 0; i < ZWN; i++) W[i] = *reinterpret_cast<const float2*>(Xr + i * ZCOLS);
-                // the offsets of four consecutive slopes move by at most one
-                // row per slope: one dispatch over the 15 monotone patterns
-                bool done = wmask == 0xFu;
-                if (done) {
-                    switch (code & 0xffu) {
-                        case 0x00: zsum4<0x00>(acc, W, wj); break;
-                        case 0x40: zsum4<0x40>(acc, W, wj); break;
-                        case 0x50: zsum4<0x50>(acc, W, wj); break;
-                        case 0x90: zsum4<0x90>(acc, W, wj); break;
-                        case 0x54: zsum4<0x54>(acc, W, wj); break;
-                        case 0x94: zsum4<0x94>(acc, W, wj); break;
-                        case 0xA4: zsum4<0xA4>(acc, W, wj); break;
-                        case 0xE4: zsum4<0xE4>(acc, W, wj); break;
-                        case 0x01: zsum4<0x01>(acc, W, wj); break;
-                        case 0x05: zsum4<0x05>(acc, W, wj); break;
-                        case 0x15: zsum4<0x15>(acc, W, wj); break;
-                        case 0x06: zsum4<0x06>(acc, W, wj); break;
-                        case 0x16: zsum4<0x16>(acc, W, wj); break;
-                        case 0x1A: zsum4<0x1A>(acc, W, wj); break;
-                        case 0x1B: zsum4<0x1B>(acc, W, wj); break;
-                        default: done = false;
-                    }
-                }
-                if (!done) {
-#pragma unroll
-                    for (int jj = 0; jj < ZV; jj++) {
-                        if (!((wmask >> jj) & 1u)) continue;
-                        const float2 a1 = dup(wj[jj]), a0 = dup(1.0f - wj[jj]);
-                        switch ((code >> (2 * jj)) & 3u) {
-                            case 0: zsum_taps<0>(acc[jj], W, a0, a1); break;
-                            case 1: zsum_taps<1>(acc[jj], W, a0, a1); break;
-                            case 2: zsum_taps<2>(acc[jj], W, a0, a1); break;
-                            default: zsum_taps<3>(acc[jj], W, a0, a1); break;
+            lo = __reduce_min_sync(0xffffffffu, lo);
+            hi = __reduce_max_sync(0xffffffffu, hi);
+            const bool vis = lo <= hi && ub0.x <= ub0.y;
+            const int rlo = vis ? lo : 0, clo = vis ? ub0.x & ~3 : 0;
+            const int nrow = vis ? (hi - rlo) / K.rows + 1 : 1, ncol = vis ? (ub0.y - clo) / kZCols + 1 : 1;
+            if (rowblk >= nrow || colblk >= ncol) continue;
+            const int row0 = rlo + rowblk * K.rows, col0 = clo + colblk * kZCols;
+            // planes whose staged window meets the volume
+            int ya = NY, ye = 0;
+            const int* dz = A.dz + size_t(K.blk0 + blk) * NY;
+            if (vis)
+                for (int yb = 0; yb < NY; yb += 32) {
+                    const int y = yb + lane;
+                    if (y < NY) {
+                        const int cx = col0 + A.T.xt[size_t(iv0) * NY + y].d, wlo = row0 + dz[y];
+                        if (cx + kZCols >= 0 && cx < NX && wlo + K.nrb > 0 && wlo < NZ) {
+                            ya = min(ya, y);
+                            ye = y + 1;
                         }
                     }
                 }
+            ya = __reduce_min_sync(0xffffffffu, ya);
+            ye = __reduce_max_sync(0xffffffffu, ye);
+            const int edge = (kind ? kZTail : 0) | (rowblk == 0 ? kZRow0 : 0) | (rowblk == nrow - 1 ? kZRowN : 0) |
+                             (colblk == 0 ? kZCol0 : 0) | (colblk == ncol - 1 ? kZColN : 0);
+            const int nst = max(1, (ye - ya + K.pps - 1) / K.pps);  // a tile without planes still writes its zeros
+            if (lane == 0) {
+                const uint32_t box = uint32_t(K.nrb) * kZCols * 4u;
+                for (int i = 0; i < nst; i++) {
+                    if (!claim()) {
+                        dead = true;
+                        break;
+                    }
+                    const int slot = j % ns, y = ya + K.pps * i, np = max(0, min(K.pps, ye - y));
+                    unsigned char* st = smem + size_t(slot) * A.stage;
+                    s_info[slot] = ZStage{y, np | edge | (i == 0 ? kZFirst : 0) | (i == nst - 1 ? kZLast : 0), v1a, vi,
+                                          row0, col0, 0.0f, 0.0f};
+                    fence_proxy_async_smem();
+                    mbar_arrive_expect_tx(&full[slot], uint32_t(np) * (box + uint32_t(sizeof(ZRec))));
+                    for (int h = 0; h < np; h++)
+                        tma_load_4d(st + size_t(h) * K.pstride * 4, &maps.m[kind], &full[slot], col0, row0 + dz[y + h],
+                                    y + h, vi);
+                    if (np)
+                        bulk_load(st + A.stage - 2 * sizeof(ZRec), A.rec + size_t(K.blk0 + blk) * NY + y,
+                                  uint32_t(np) * uint32_t(sizeof(ZRec)), &full[slot]);
+                    j++;
+                }
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&empty[slot]);
-            if (++slot == ns) {
-                slot = 0;
-                phase ^= 1u;
+            dead = __shfl_sync(0xffffffffu, int(dead), 0) != 0;
+        }
+        if (lane == 0) {
+            if (!dead && claim()) {
+                const int slot = j % ns;
+                s_info[slot].flags = kZEnd;
+                mbar_arrive(&full[slot]);
+                j++;
+            } else {
+                *s_abort = 1;
             }
         }
-        if (__syncthreads_or(dead)) {
-            // a wait gave up: drain the copies still in flight, write nothing
-            if (tid == 0)
-                for (int s = 0; s < ns; s++)
-                    if (s_round[s] >= 0) mbar_wait(&full[s], uint32_t(s_round[s] & 1), nullptr);
-            return;
-        }
+        __syncthreads();
+        // a wait gave up: drain the copies still in flight
+        if (lane == 0 && *s_abort)
+            for (int i = max(0, j - ns); i < j; i++) mbar_wait(&full[i % ns], uint32_t((i / ns) & 1), nullptr);
+        return;
     }
 
-    // epilogue: scale, ray masks, optional MLEM ratio
-    const int colA = col0 + 2 * lane;
-    const bool pairs = (G.N_u0 & 1) == 0;  // float2 accesses stay 8-byte aligned
-#pragma unroll
-    for (int j = 0; j < ZV; j++) {
-        const int v1 = v1a + jw + j;
-        if (jw + j >= nsl) continue;
-        const float S = A.T.S[size_t(v1) * G.N_v0 + iv0];
-        const int2 u1r = A.T.ub1[v1];
-#pragma unroll
-        for (int k = 0; k < ZK; k++) {
-            const int iu1 = row0 + k;
-            if (iu1 >= G.N_u1) break;
-            const bool rv = iu1 >= u1r.x && iu1 <= u1r.y;
-            const size_t o = ((size_t(v1) * G.N_v0 + iv0) * G.N_u1 + iu1) * G.N_u0 + colA;
-            const bool v0ok = rv && colA >= ub0.x && colA <= ub0.y;
-            const bool v1ok = rv && colA + 1 >= ub0.x && colA + 1 <= ub0.y;
-            float2 val = make_float2(v0ok ? acc[j][k].x * S : 0.0f, v1ok ? acc[j][k].y * S : 0.0f);
-            if (pairs && colA + 1 < G.N_u0) {
-                if (meas) {
-                    const float2 m = Store<TG>::ld2(meas + o);
-                    val = make_float2(ratio_rule(m.x, val.x), ratio_rule(m.y, val.y));
+    {
+        consumer_registers();
+        int slot = 0;
+        uint32_t phase = 0;
+        auto wait = [&]() {
+            return __all_sync(0xffffffffu, ring_wait(&full[slot], phase, A.err, s_abort, A.wait_limit)) != 0;
+        };
+        bool dead = !wait();
+        while (!dead) {  // tiles
+            const ZStage in = s_info[slot];
+            if (in.flags & kZEnd) break;
+            const ZKind& K = A.k[in.flags & kZTail ? 1 : 0];
+            const int gv = warp % K.sg, gr = warp / K.sg, row0 = in.row0 + gr * NK;
+            bool have = false;  // some slope of this warp has visible rows in the tile
+            if (gr < K.rg)
+                for (int v1 = in.a + gv * NV; v1 < min(in.a + (gv + 1) * NV, K.v1_end); v1++) {
+                    const int2 u = A.T.ub1[v1];
+                    have |= row0 <= u.y && row0 + NK - 1 >= u.x;
                 }
-                Store<TG>::st2(g + o, val);
-            } else {
-                if (colA < G.N_u0) g[o] = Store<TG>::st(meas ? ratio_rule(Store<TG>::ld(meas[o]), val.x) : val.x);
-                if (colA + 1 < G.N_u0)
-                    g[o + 1] = Store<TG>::st(meas ? ratio_rule(Store<TG>::ld(meas[o + 1]), val.y) : val.y);
+            f2x acc[NV][NK];
+#pragma unroll
+            for (int j = 0; j < NV; j++)
+#pragma unroll
+                for (int k = 0; k < NK; k++) acc[j][k] = 0ull;
+            const int pbytes = K.pstride * 4;
+            for (;;) {  // stages
+                const int flags = s_info[slot].flags;
+                if (have) {
+                    const unsigned char* st = smem + size_t(slot) * A.stage;
+                    const ZRec* rec = reinterpret_cast<const ZRec*>(st + A.stage - 2 * sizeof(ZRec));
+#pragma unroll 1
+                    for (int h = flags & 3; h > 0; h--, rec++, st += pbytes) {
+                        const uint32_t code = rec->code[gv];
+                        f2x wa[NV], wb[NV];
+#pragma unroll
+                        for (int j = 0; j < NV; j++) {
+                            const float w = rec->w[gv * NV + j];
+                            wa[j] = f2_dup(1.0f - w);
+                            wb[j] = f2_dup(w);
+                        }
+                        const int iz0 = row0 + int(int16_t(code >> 16));  // volume row of window row 0
+                        if (iz0 + WN - 1 < 0 || iz0 >= NZ) continue;
+                        const f2x* W = reinterpret_cast<const f2x*>(st) +
+                                       (int((code >> 8) & 0xffu) + gr * NK) * (kZCols / 2) + lane;
+                        // the offsets of consecutive slopes are monotone and
+                        // (four slopes) at most one row apart: one dispatch
+                        // per plane over the patterns that occur
+                        if constexpr (NV == 4) {
+                            switch (code & 0xffu) {
+#define PETL_ZCASE(PC) case PC: z_taps<PC, true>(acc, W, wa, wb); break;
+                                PETL_ZCASE(0x00) PETL_ZCASE(0x40) PETL_ZCASE(0x50) PETL_ZCASE(0x90) PETL_ZCASE(0x54)
+                                PETL_ZCASE(0x94) PETL_ZCASE(0xA4) PETL_ZCASE(0xE4) PETL_ZCASE(0x01) PETL_ZCASE(0x05)
+                                PETL_ZCASE(0x15) PETL_ZCASE(0x06) PETL_ZCASE(0x16) PETL_ZCASE(0x1A) PETL_ZCASE(0x1B)
+                            }
+                        } else {
+                            switch (code & 0xfu) {
+                                PETL_ZCASE(0x0) PETL_ZCASE(0x4) PETL_ZCASE(0x8) PETL_ZCASE(0xC) PETL_ZCASE(0x1)
+                                PETL_ZCASE(0x2) PETL_ZCASE(0x3)
+#undef PETL_ZCASE
+                            }
+                        }
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&empty[slot]);
+                if (++slot == ns) {
+                    slot = 0;
+                    phase ^= 1u;
+                }
+                if (flags & kZLast) break;
+                if (!wait()) {
+                    dead = true;
+                    break;
+                }
             }
+            if (dead) break;
+            if (gr < K.rg) {
+            // epilogue: scale, ray masks, optional MLEM ratio; zeros for the
+            // masked rays beyond the tiles
+            const int mb = NM == 1 ? 0 : in.b / A.M.nvm, mv = in.b - mb * A.M.nvm;
+            const int iv0 = member_pick<NM>(A.M.first, mb) + mv * A.step;
+            TG* __restrict__ g = static_cast<TG*>(member_pick<NM>(A.M.out, mb));
+            const TG* __restrict__ meas = static_cast<const TG*>(member_pick<NM>(A.M.meas, mb));
+            const int2 ub0 = A.T.ub0[iv0];
+            const int colA = in.col0 + 2 * lane;
+            const int row1 = min(row0 + NK, G.N_u1);
+            const bool pairs = (G.N_u0 & 1) == 0;  // float2 accesses stay 8-byte aligned
+            const bool ok0 = colA >= ub0.x && colA <= ub0.y, ok1 = colA + 1 >= ub0.x && colA + 1 <= ub0.y;
+            f2x* out = ctl->out[warp][0] + lane;
+#pragma unroll 1
+            for (int i = 0; i < NV * NK / kZOut; i++) {
+                out_rows(acc, out, i);
+                const int v1 = in.a + gv * NV + i / (NK / kZOut), r0 = row0 + i % (NK / kZOut) * kZOut;
+                if (v1 >= min(in.a + NV * K.sg, K.v1_end)) break;
+                const float S = A.T.S[size_t(v1) * G.N_v0 + iv0];
+                const int2 u1r = A.T.ub1[v1];
+                const size_t o0 = (size_t(v1) * G.N_v0 + iv0) * G.N_u1 * G.N_u0;
+                if (pairs && colA + 1 < G.N_u0) {
+                    float2 m[kZOut];
+                    if (meas)
+#pragma unroll
+                        for (int k = 0; k < kZOut; k++)
+                            if (r0 + k < G.N_u1) m[k] = Store<TG>::ld2(meas + o0 + size_t(r0 + k) * G.N_u0 + colA);
+#pragma unroll
+                    for (int k = 0; k < kZOut; k++) {
+                        if (r0 + k >= G.N_u1) break;
+                        const bool rv = r0 + k >= u1r.x && r0 + k <= u1r.y;
+                        const float2 a = f2_unpack(out[k * 32]);
+                        float2 val = make_float2(rv && ok0 ? a.x * S : 0.0f, rv && ok1 ? a.y * S : 0.0f);
+                        if (meas) val = make_float2(ratio_rule(m[k].x, val.x), ratio_rule(m[k].y, val.y));
+                        Store<TG>::st2(g + o0 + size_t(r0 + k) * G.N_u0 + colA, val);
+                    }
+                } else {  // odd rows, or the row's last column
+#pragma unroll 1
+                    for (int k = 0; k < min(kZOut, G.N_u1 - r0); k++) {
+                        const bool rv = r0 + k >= u1r.x && r0 + k <= u1r.y;
+                        const size_t o = o0 + size_t(r0 + k) * G.N_u0 + colA;
+                        const float2 a = f2_unpack(out[k * 32]);
+                        const float2 val = make_float2(rv && ok0 ? a.x * S : 0.0f, rv && ok1 ? a.y * S : 0.0f);
+                        if (colA < G.N_u0) g[o] = Store<TG>::st(meas ? ratio_rule(Store<TG>::ld(meas[o]), val.x) : val.x);
+                        if (colA + 1 < G.N_u0)
+                            g[o + 1] = Store<TG>::st(meas ? ratio_rule(Store<TG>::ld(meas[o + 1]), val.y) : val.y);
+                    }
+                }
+            }
+            // masked rays around the tiles
+            const int cz0 = in.flags & kZCol0 ? 0 : in.col0;
+            const int cz1 = in.flags & kZColN ? G.N_u0 : min(in.col0 + kZCols, G.N_u0);
+            const int rz0 = (in.flags & kZRow0) && gr == 0 ? 0 : row0;
+            const int rz1 = (in.flags & kZRowN) && gr == K.rg - 1 ? G.N_u1 : row1;
+            if (cz0 < in.col0 || cz1 > in.col0 + kZCols || rz0 < row0 || rz1 > row1)
+#pragma unroll 1
+                for (int v1 = in.a + gv * NV; v1 < min(in.a + (gv + 1) * NV, K.v1_end); v1++)
+#pragma unroll 1
+                    for (int r = rz0; r < rz1; r++) {
+                        TG* row = g + ((size_t(v1) * G.N_v0 + iv0) * G.N_u1 + r) * G.N_u0;
+                        const bool inside = r >= row0 && r < row1;
+#pragma unroll 1
+                        for (int c = cz0 + lane; c < cz1; c += 32)
+                            if (!inside || c < in.col0 || c >= in.col0 + kZCols) row[c] = Store<TG>::st(0.0f);
+                    }
+            }
+            dead = !wait();
         }
+        if (dead) *s_abort = 1;
     }
+    __syncthreads();
 }
 
-// Scratch budget of the x-shift pass (bytes of FP32 X per chunk of views);
-// PETL_SPLIT_SCRATCH_MB overrides it.
-
-// Launch layout of k_fwd_zsum for one range of slope blocks.
-struct ZsumLaunch {
+// Launch shape of the z kernel for a call: false when a layout rule fails.
+struct ZPlan {
     ZsumArgs A;
-    CUtensorMap map;
+    int nv, nk;        // slopes and rows per warp
     size_t smem;
-    unsigned nblk;  // CTAs per view
+    size_t table_bytes;
 };
 
-// Layout of the blocks of slopes [v1_first, v1_end) with sg slope groups per
-// CTA: false when it breaks a layout rule.
-bool zsum_layout(const petl_geom& G, const ViewRange& vr, int v1_first, int v1_end, int sg, double step,
-                 const float* X, int NXc, int nv, const Tables& T, int* err, ZsumLaunch& L)
+bool zsum_plan(const petl_geom& G, const ViewRange& vr, double step, int nslot, ZPlan& P)
 {
-    const int rows = ZK * (ZWARPS / sg);
-    const int nrb = rows + shift_spread(ZV * sg - 1, step) + 1;
-    if (nrb > 256 - ZDMAX) return false;  // TMA box rows; the window row fits 8 bits
-    ZsumArgs& A = L.A;
+    ZsumArgs& A = P.A;
     A = ZsumArgs{};
     A.G = G;
     A.step = vr.iv0_step;
-    A.v1_first = v1_first;
-    A.v1_end = v1_end;
-    A.sg = sg;
-    A.n_colblk = int(ceil_div(G.N_u0, ZCOLS));
-    A.n_rowblk = int(ceil_div(G.N_u1, rows));
-    A.nrb = nrb;
-    A.pstride = ((nrb + ZDMAX) * ZCOLS + 31) & ~31;  // 128-byte aligned planes
-    A.T = T;
-    A.err = err;
+    A.nslot = nslot;
+    A.n_colblk = int(ceil_div(G.N_u0, kZCols));
     A.wait_limit = wait_limit();
-    // shared memory: the ring, then the per-CTA tables and the barriers
-    const size_t np = size_t(std::min(G.numY, ZMAXPLANES));
-    const size_t b_w = np * 4 * sizeof(float4), b_code = np * 4 * 4, b_plane = np * 8;
-    const size_t b_bar = 2 * ZNSMAX * 8 + (2 + ZNSMAX) * 4;
-    auto al = [](size_t b) { return (b + 15) & ~size_t(15); };
-    const size_t fixed = al(b_w) + al(b_code) + al(b_plane) + al(b_bar);
-    const size_t stage = size_t(2) * A.pstride * 4;
-    A.ns = int(std::min<size_t>(ZNSMAX, (227 * 1024 - std::min<size_t>(fixed, 227 * 1024)) / stage));
+    // four slopes share a window of 16 rows where their shifts differ by at
+    // most three rows (steps below one row per slope); steeper slopes (a volume
+    // that reaches beyond the panels) take two per warp and a window of 28
+    // rows, whose loads then bound them; steps of three rows and more are left
+    // to the first-generation kernel.  192x192x96 at 1.1 to 1.4 rows per
+    // slope: 3.3 ms for 67 views here, 6.0 on the first-generation kernel
+    P.nv = shift_spread(3, step) <= kZSpread ? 4 : 2;
+    P.nk = P.nv == 4 ? 12 : 24;
+    if (shift_spread(P.nv - 1, step) > kZSpread) return false;
+    const int nv1 = vr.iv1_end - vr.iv1_begin;
+    const int ngrp = int(ceil_div(nv1, P.nv));
+    // Twelve consumer warps; four where twelve would leave SMs without a tile
+    // (an ordered subset of a small volume: a third of the rows per tile, and a
+    // warp alone on its scheduler).
+    for (A.nw = kZWarps;; A.nw = 4) {
+        const int sg = P.nv == 4 || A.nw == 4 ? 4 : 6;
+        // full blocks of sg slope groups; a tail of at most half a block
+        // takes fewer slope groups over more rows instead of idle warps
+        const int ntail = ngrp % sg;
+        const int tail_sg = ntail == 0 ? 0 : ntail == 1 ? 1 : 2 * ntail <= sg ? sg / 2 : 0;
+        const int v1_split = tail_sg ? vr.iv1_begin + (ngrp - ntail) * P.nv : vr.iv1_end;
+        int tiles = 0;
+        for (int i = 0; i < 2; i++) {
+            ZKind& K = A.k[i];
+            K.v1_first = i ? v1_split : vr.iv1_begin;
+            K.v1_end = i ? vr.iv1_end : v1_split;
+            K.sg = i ? std::max(tail_sg, 1) : sg;
+            K.rg = std::min(A.nw / K.sg, int(ceil_div(G.N_u1, P.nk)));
+            K.rows = P.nk * K.rg;
+            K.nblk = int(ceil_div(K.v1_end - K.v1_first, P.nv * K.sg));
+            K.n_rowblk = int(ceil_div(G.N_u1, K.rows));
+            K.nrb = K.rows + shift_spread(P.nv * K.sg - 1, step) + 1;
+            K.pstride = (K.nrb + kZSpread) * kZCols;
+            K.pps = i ? 1 : 2;
+            K.blk0 = i ? A.k[0].nblk : 0;
+            if (K.nrb > 256 - kZSpread) return false;  // TMA box rows; the window row fits 8 bits
+            const long long nt = (long long)nslot * K.nblk * K.n_rowblk * A.n_colblk;
+            if (nt > (1 << 30)) return false;
+            K.ntile = int(nt);
+            tiles += K.ntile;
+        }
+        if (A.nw == 4 || tiles >= sm_count()) break;
+    }
+    A.stage = 0;
+    for (const ZKind& K : A.k)
+        if (K.nblk > 0) A.stage = std::max(A.stage, K.pstride * K.pps * 4);
+    A.stage += 2 * int(sizeof(ZRec));
+    A.stage = (A.stage + 127) & ~127;
+    A.ns = std::min(kZStages, (227 * 1024 - int(sizeof(ZCtl))) / A.stage);
     if (A.ns < 2) return false;
-    const size_t ring = size_t(A.ns) * stage;
-    A.off_w = unsigned(ring);
-    A.off_code = unsigned(A.off_w + al(b_w));
-    A.off_plane = unsigned(A.off_code + al(b_code));
-    A.off_bar = unsigned(A.off_plane + al(b_plane));
-    L.smem = A.off_bar + al(b_bar);
-    if (L.smem > 227 * 1024) return false;
-    L.nblk = unsigned(A.n_colblk) * unsigned(A.n_rowblk) * ceil_div(v1_end - v1_first, ZV * sg);
-    const uint64_t dims[4] = {uint64_t(NXc), uint64_t(G.numZ), uint64_t(G.numY), uint64_t(nv)};
-    const uint64_t strides[3] = {uint64_t(NXc) * 4, uint64_t(NXc) * G.numZ * 4, uint64_t(NXc) * G.numZ * G.numY * 4};
-    const uint32_t box[4] = {uint32_t(ZCOLS), uint32_t(nrb), 1u, 1u};
-    return encode_tensor_map(&L.map, X, 4, dims, strides, box, 4);
+    P.smem = size_t(A.ns) * A.stage + sizeof(ZCtl);
+    const size_t nrec = size_t(A.k[0].nblk + A.k[1].nblk) * G.numY;
+    P.table_bytes = nrec * (sizeof(ZRec) + sizeof(int)) + sizeof(int);
+    return true;
 }
 
 }  // namespace
 
+// Scratch budget of the x-shift pass (bytes of FP32 X per chunk of views);
+// PETL_SPLIT_SCRATCH_MB overrides it.
 size_t split_scratch_budget()
 {
     static const long long env_mb = [] {
@@ -563,9 +637,9 @@ int project_split_m(const petl_geom& G, const Members& M0, const ViewRange& vr, 
     // the x pass writes a volume per view whatever the slope count: below
     // about ten slopes the single-pass kernel is cheaper than that round trip
     if (nv1 < kSplitMinSlopes) return kNotApplicable;
-    if (G.numY > ZMAXPLANES || G.numZ > 65535 * 4) return kNotApplicable;
+    if (std::max(G.numZ, G.N_u1) > ZMAXROWS) return kNotApplicable;
     const double step = double(G.T_v1) * plane_ymax(G) / double(G.T_z);  // shift change per slope
-    if (shift_spread(ZV - 1, step) > ZDMAX) return kNotApplicable;
+    if (!(step * std::max(G.N_v1, 1) < ZMAXROWS)) return kNotApplicable;
     int* err = device_error_ptr();
     if (!err) return kNotApplicable;
 
@@ -581,37 +655,45 @@ int project_split_m(const petl_geom& G, const Members& M0, const ViewRange& vr, 
         nchunks = (nvmax + nv - 1) / nv;
         nv = (nvmax + nchunks - 1) / nchunks;
     } else {
-        if (size_t(nb) * nvmax > fit || size_t(nb) * nvmax > 65535 || chunk_cap > 0) return kNotApplicable;
+        if (size_t(nb) * nvmax > fit || chunk_cap > 0) return kNotApplicable;
         nv = nvmax;
         nchunks = 1;
     }
+    ZPlan P;
+    if (!zsum_plan(G, vr, step, nv * nb, P)) return kNotApplicable;
 
+    // X, then the table records and the blocks' smallest shifts
     float* X = nullptr;
-    if (scratch_alloc(reinterpret_cast<void**>(&X), per_view * nv * nb, st) != cudaSuccess) {
+    const size_t x_bytes = per_view * nv * nb;  // a multiple of 16
+    if (scratch_alloc(reinterpret_cast<void**>(&X), x_bytes + P.table_bytes, st) != cudaSuccess) {
         cudaGetLastError();  // out of memory is not sticky: the caller takes the fused kernel
         return kNotApplicable;
     }
-    // full blocks of 16 slopes; a tail of at most 8 slopes takes CTAs of 1 or
-    // 2 slope groups over 128 or 64 rows instead of a mostly idle full block
-    const int ntail = nv1 % ZSL;
-    const int tail_sg = ntail == 0 ? 0 : ntail <= ZV ? 1 : ntail <= 2 * ZV ? 2 : 0;
-    const int v1_split = vr.iv1_end - (tail_sg ? ntail : 0);
-    ZsumLaunch L[2];
-    int nl = 0;
+    ZsumArgs& A = P.A;
+    A.T = T;
+    A.err = err;
+    A.rec = reinterpret_cast<ZRec*>(reinterpret_cast<unsigned char*>(X) + x_bytes);
+    A.dz = reinterpret_cast<int*>(A.rec + size_t(A.k[0].nblk + A.k[1].nblk) * G.numY);
+    A.next = A.dz + size_t(A.k[0].nblk + A.k[1].nblk) * G.numY;
+    ZMaps maps;
+    std::memset(&maps, 0, sizeof(maps));
+    const uint64_t dims[4] = {uint64_t(NXc), uint64_t(G.numZ), uint64_t(G.numY), uint64_t(nv * nb)};
+    const uint64_t strides[3] = {uint64_t(NXc) * 4, uint64_t(NXc) * G.numZ * 4, uint64_t(NXc) * G.numZ * G.numY * 4};
     bool ok = true;
-    if (v1_split > vr.iv1_begin)
-        ok = zsum_layout(G, vr, vr.iv1_begin, v1_split, ZSG, step, X, NXc, nv * nb, T, err, L[nl++]);
-    if (ok && tail_sg) ok = zsum_layout(G, vr, v1_split, vr.iv1_end, tail_sg, step, X, NXc, nv * nb, T, err, L[nl++]);
+    for (int i = 0; i < 2 && ok; i++) {
+        if (A.k[i].nblk == 0) continue;
+        const uint32_t box[4] = {uint32_t(kZCols), uint32_t(A.k[i].nrb), 1u, 1u};
+        ok = encode_tensor_map(&maps.m[i], X, 4, dims, strides, box, 4);
+    }
     if (!ok) {
         cudaFreeAsync(X, st);
         return kNotApplicable;
     }
     // kernels compiled for one member where there is one
-    auto kz = nb == 1 ? k_fwd_zsum<TG, 1> : k_fwd_zsum<TG, kMaxMembers>;
+    auto kz = nb == 1 ? (P.nv == 4 ? k_fwd_zsum<TG, 1, 4, 12> : k_fwd_zsum<TG, 1, 2, 24>)
+                      : (P.nv == 4 ? k_fwd_zsum<TG, kMaxMembers, 4, 12> : k_fwd_zsum<TG, kMaxMembers, 2, 24>);
     auto kx = nb == 1 ? k_xshift<TF, 1> : k_xshift<TF, kMaxMembers>;
-    size_t smem_max = 0;
-    for (int l = 0; l < nl; l++) smem_max = std::max(smem_max, L[l].smem);
-    cudaError_t e = cudaFuncSetAttribute(kz, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_max));
+    cudaError_t e = cudaFuncSetAttribute(kz, cudaFuncAttributeMaxDynamicSharedMemorySize, int(P.smem));
     for (int c = 0; c < nchunks && e == cudaSuccess; c++) {
         Members M = M0;
         const int vi0 = c * nv;
@@ -622,14 +704,15 @@ int project_split_m(const petl_geom& G, const Members& M0, const ViewRange& vr, 
             M.nv[0] = nvc;
         }
         M.nvm = nvc;
-        XshiftArgs XA{G, vr.iv0_step, NXc, T, M};
+        XshiftArgs XA{G, vr.iv0_step, NXc, T, M, {A.k[0], A.k[1]}, P.nv, A.rec, A.dz, A.next, err};
         kx<<<dim3(ceil_div(G.numZ, XZB), unsigned(G.numY), unsigned(nb)), 256, 0, st>>>(X, XA);
         note_launch();
-        for (int l = 0; l < nl; l++) {
-            L[l].A.M = M;
-            kz<<<dim3(L[l].nblk, unsigned(nvc * nb)), ZNT, L[l].smem, st>>>(L[l].map, L[l].A);
-            note_launch();
-        }
+        A.M = M;
+        A.nslot = nvc * nb;
+        int tiles = 0;
+        for (ZKind& K : A.k) tiles += K.ntile = A.nslot * K.nblk * K.n_rowblk * A.n_colblk;
+        kz<<<std::min(tiles, sm_count()), 32 * (A.nw + 4), P.smem, st>>>(maps, A);
+        note_launch();
         e = cudaGetLastError();
         if (e == cudaSuccess && hook && hook->fn) hook->fn(hook->ctx, vi0, nvc);
     }

@@ -40,9 +40,7 @@ struct Store<__nv_bfloat16> {
     }
 };
 
-// Two scalar FMAs on a column pair.  Scalar FFMA issues at the full FP32
-// rate with two warps per scheduler; the packed f32x2 form needs about four
-// times the warps to reach the same rate on this part.
+// Two scalar FMAs on a column pair (the single-pass kernels).
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
 {
     return make_float2(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y));
