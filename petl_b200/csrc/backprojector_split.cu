@@ -9,12 +9,11 @@
 // two interpolations are separate kernels:
 //
 // * k_bwd_zgather sums the z taps over the slopes of one view into FP32
-//   scratch B[view][y][z][c] (c = planogram column).  CTA = views of a group x
-//   16 planes x 32 rows x 64 columns, 16 warps of 4 planes x 8 rows x 2
-//   columns per lane; per slope the planogram rows the tile needs arrive by a
-//   tiled TMA copy (no multicast) into a ring of two-slope stages with
-//   full/empty mbarriers and a rotating copy issuer; window offsets, modes,
-//   masks and weights are tabulated once per CTA.
+//   scratch B[view][y][z][c] (c = planogram column): persistent CTAs of twelve
+//   consumer warps and a producer warp that stages the slopes' planogram rows
+//   into a ring with full/empty mbarriers, by tiled TMA copies (no multicast)
+//   or, where rows are no multiple of 16 bytes, by copies of column pairs;
+//   k_gather_records tabulates window offsets, masks and weights once per call.
 // * k_bwd_xgather applies the x taps and sums the views of a chunk into the
 //   volume (or an FP32 partial sum between chunks).
 //
@@ -25,6 +24,11 @@
 // of one geometry (one tensor map per member's planogram).  A single slope
 // at v1 = 0 (the rebinned planogram of FBP) takes k_bwd_zflat: its z sums
 // do not depend on the plane.
+//
+// 256x256x128, planogram (65, 129, 128, 256): 8.7 ms for the z taps and 0.9
+// for the x pass (before: 12.5 and 0.9, with one 16-warp CTA per tile, tables
+// built by every CTA and scalar FMAs).  FBP's single slope: 0.42 ms (0.72 with
+// a thread per x).
 // Every wait is bounded: a wait that gives up sets the device error word, the
 // CTA drains its copies in flight and returns without writing.
 #include <cuda.h>
@@ -43,70 +47,53 @@
 #include "shear.cuh"
 #include "storage.cuh"
 #include "tma.cuh"
+#include "ztaps.cuh"
 
 namespace petl {
 namespace shear {
 
 namespace {
 
-constexpr int GP = 4;               // planes per warp
-constexpr int GK = 8;               // rows per warp
-constexpr int GPG = 4;              // plane groups per CTA
-constexpr int GRG = 4;              // row groups per CTA
-constexpr int GPL = GP * GPG;       // planes per CTA
-constexpr int GROWS = GK * GRG;     // rows per CTA
-constexpr int GCOLS = 64;           // columns per CTA, two per lane
-constexpr int GWARPS = GPG * GRG;
-constexpr int GNT = 32 * GWARPS;
-constexpr int GDW = 2;              // largest shift difference among a warp's planes
-constexpr int GWN = GK + GDW + 1;   // register window rows
-// ring stages: two (of two slopes each) measured fastest; deeper rings
-// (3-8 stages) ran 3-10 % slower at the 256x256x128 workload
-constexpr int GNSMAX = 2;
+constexpr int GPLMAX = 16;          // planes per block at most (a table record holds 16 weights)
 constexpr int GV1MAX = 128;         // slopes per call at most
-constexpr int GVG = 4;              // views per CTA at most
-constexpr int kPatGen = 15;         // no straight-line pattern: per-plane taps
+constexpr int GMAXROWS = 15000;     // rows of volume and planogram at most
 
-// Window offsets of a plane group's 4 planes when all are fully visible and
-// their shifts differ by at most one row: o0 | o1 << 2 | o2 << 4 | o3 << 6.
-constexpr int kNumPat = 7;
-__host__ __device__ constexpr int gpat_offsets(int pid)
-{
-    return pid == 0 ? 0x00 : pid == 1 ? 0x40 : pid == 2 ? 0x50 : pid == 3 ? 0x54
-         : pid == 4 ? 0x01 : pid == 5 ? 0x05 : 0x15;
-}
-
-// Entry of a (slope, warp).  code: plane modes and offsets (4 bits per
-// plane: mode 0 none / 1 full / 2 masked rows, offset << 2), path << 16
-// (0..6: the straight-line pattern of fully visible planes; 8..14: the same
-// pattern with per-plane row intervals; kPatGen: per-plane taps), window row
-// in the stage << 20.  vm: window rows holding visible bins (adjoint).  ivl:
-// per plane (8 bits each) the mask of output rows that receive the slope:
-// the rows inside the visible range (adjoint: all) or passing the voxel
-// test (reference).
-struct __align__(16) GEntry {
-    uint32_t code;
-    uint32_t vm;
-    uint32_t ivl;
-    uint32_t pad;
+// Table record of one (plane block, row block, slope), staged with the slope:
+// the second tap's weight of each plane; per warp a code word (window offsets,
+// 2 bits per plane; kind << 8: 0 no rows, 1 every row, 2 edge of the visible
+// range; the window's first staged row << 16) and a mask for the edge: the
+// output rows of each plane that receive the slope (64 / NV bits per plane;
+// reference semantics) or the window rows that hold visible bins (adjoint).
+struct __align__(16) GRec {
+    float w[GPLMAX];
+    uint32_t code[kZWarps];
+    unsigned long long mask[kZWarps];
 };
 
 struct ZgatherArgs {
     petl_geom G;
-    ViewRange vr;  // slopes and view step (the members hold their views)
-    int vg;        // views per CTA
-    int gpm;       // CTAs along y per member: ceil(view slots per member / vg)
-    int n_colblk;  // ceil(N_u0 / 64)
-    int n_rowblk;  // ceil(numZ / 32)
-    int brb;       // staged planogram rows per slope (33 + CTA shift spread, bounded on the host)
-    int ns;        // ring stages, two slopes each
-    int sstride;   // elements per staged slope (brb + 2 rows of 64; 128-byte multiple)
-    int NUc;       // scratch row pitch (columns)
-    int v1cap;     // slopes the per-CTA tables hold (the call's slope count)
+    ViewRange vr;   // slopes and view step (the members hold their views)
+    int nw;         // consumer warps
+    int pg, rg;     // plane groups x row groups of a CTA (pg * rg = nw)
+    int planes, rows;  // planes and rows per tile
+    int nslot;      // view slots of all members
+    int n_plblk, n_rowblk, n_colblk;
+    int nrb;        // staged planogram rows per slope (rows + 1 + shift spread of the planes)
+    int ns;         // ring stages, two slopes each
+    int sbytes;     // bytes per staged slope (nrb + kZSpread rows of 64, a multiple of 128)
+    int stage;      // bytes per stage (slopes, then two records)
+    int NUc;        // scratch row pitch (columns)
+    int nv1;        // slopes of the call
+    int ntile;
+    GRec* rec;      // [plane block][row block][nv1], the slopes that reach the tile first
+    int2* list;     // same layout: (v1, first staged row)
+    int* cnt;       // [plane block][row block] slopes that reach the tile
+    int* next;      // tiles handed out beyond one per CTA, per chunk
+    int nchunks;
     Tables T;
     int* err;
     unsigned wait_limit;  // bound of the waits on staged data (wait_limit(): kWaitLimit or 0)
-    Members M;  // views of the chunk per member (the planograms are the tensor maps)
+    Members M;            // planograms (in) and views of the chunk
 };
 
 // tensor maps of the members' planograms
@@ -115,108 +102,18 @@ struct GMaps {
     CUtensorMap m[NM];
 };
 
-// z taps of one plane (two columns): Z[k] += w0 W[O + k + 1] then w1 W[O + k],
-// with per-row 0/1 masks when MASK (vm: window rows, om: output rows).
-template <int O, bool MASK>
-__device__ __forceinline__ void g_taps(float2 (&Z)[GK], const float2 (&W)[GWN], float w0, float w1, uint32_t vm,
-                                       uint32_t om)
+// The slopes that reach each tile of planes and rows, compacted in order, and
+// their records.  Grid (plane blocks, row blocks), 256 threads.
+template <bool ADJ>
+__global__ void __launch_bounds__(256) k_gather_records(const ZgatherArgs A, int NV, int NK)
 {
-    if (MASK) {
-#pragma unroll
-        for (int k = 0; k < GK; k++) {
-            const bool kb = (vm >> (O + k + 1)) & (om >> k) & 1u, ka = (vm >> (O + k)) & (om >> k) & 1u;
-            const float2 b = kb ? W[O + k + 1] : make_float2(0.0f, 0.0f);
-            const float2 a = ka ? W[O + k] : make_float2(0.0f, 0.0f);
-            Z[k] = make_float2(fmaf(w1, a.x, fmaf(w0, b.x, Z[k].x)), fmaf(w1, a.y, fmaf(w0, b.y, Z[k].y)));
-        }
-    } else {
-        const float2 a0 = dup(w0), a1 = dup(w1);
-#pragma unroll
-        for (int k = 0; k < GK; k++) Z[k] = fma2(a0, W[O + k + 1], Z[k]);
-#pragma unroll
-        for (int k = 0; k < GK; k++) Z[k] = fma2(a1, W[O + k], Z[k]);
-    }
-}
-
-template <int PID>
-__device__ __forceinline__ void g_taps4(float2 (&Z)[GP][GK], const float2 (&W)[GWN], float4 wa, float4 wb)
-{
-    constexpr int o = gpat_offsets(PID);
-    g_taps<(o >> 0) & 3, false>(Z[0], W, wa.x, wa.y, 0u, 0u);
-    g_taps<(o >> 2) & 3, false>(Z[1], W, wa.z, wa.w, 0u, 0u);
-    g_taps<(o >> 4) & 3, false>(Z[2], W, wb.x, wb.y, 0u, 0u);
-    g_taps<(o >> 6) & 3, false>(Z[3], W, wb.z, wb.w, 0u, 0u);
-}
-
-// z taps of one plane restricted to the output rows of mask m (predicated;
-// rows outside receive nothing, as the masked taps' zero operands give)
-template <int O>
-__device__ __forceinline__ void g_taps_ivl(float2 (&Z)[GK], const float2 (&W)[GWN], float w0, float w1,
-                                           uint32_t m)
-{
-    const float2 a0 = dup(w0), a1 = dup(w1);
-#pragma unroll
-    for (int k = 0; k < GK; k++)
-        if ((m >> k) & 1u) Z[k] = fma2(a0, W[O + k + 1], Z[k]);
-#pragma unroll
-    for (int k = 0; k < GK; k++)
-        if ((m >> k) & 1u) Z[k] = fma2(a1, W[O + k], Z[k]);
-}
-
-template <int PID>
-__device__ __forceinline__ void g_taps4_ivl(float2 (&Z)[GP][GK], const float2 (&W)[GWN], float4 wa, float4 wb,
-                                            uint32_t ivl)
-{
-    constexpr int o = gpat_offsets(PID);
-    g_taps_ivl<(o >> 0) & 3>(Z[0], W, wa.x, wa.y, ivl);
-    g_taps_ivl<(o >> 2) & 3>(Z[1], W, wa.z, wa.w, ivl >> 8);
-    g_taps_ivl<(o >> 4) & 3>(Z[2], W, wb.x, wb.y, ivl >> 16);
-    g_taps_ivl<(o >> 6) & 3>(Z[3], W, wb.z, wb.w, ivl >> 24);
-}
-
-// TG: planogram storage (float or bfloat16); B and the arithmetic are FP32.
-// Warp w: plane group w % 4, row group w / 4.
-template <bool ADJ, class TG, int NM>
-__global__ void __launch_bounds__(GNT, 1)
-k_bwd_zgather(const __grid_constant__ GMaps<NM> gmaps, float* __restrict__ B, const ZgatherArgs A)
-{
-    extern __shared__ __align__(128) unsigned char smem[];
     const petl_geom& G = A.G;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int q = warp % GPG, r = warp / GPG;
-    int t = blockIdx.x;
-    const int colblk = t % A.n_colblk;
-    t /= A.n_colblk;
-    const int rowblk = t % A.n_rowblk;
-    const int plblk = t / A.n_rowblk;
-    const int p0 = plblk * GPL, r0 = rowblk * GROWS, col0 = colblk * GCOLS;
-    const int z0 = r0 + r * GK;  // first row of this warp
-    const int mb = NM == 1 ? 0 : blockIdx.y / A.gpm;  // member
-    const int vfirst = (blockIdx.y - mb * A.gpm) * A.vg;  // first view of this CTA in the member's chunk
-    const int nvw = min(A.vg, member_pick<NM>(A.M.nv, mb) - vfirst);  // views of this CTA
-    if (nvw <= 0) return;  // a member with fewer views than the slots
-    const int vbase = member_pick<NM>(A.M.first, mb) + vfirst * A.vr.iv0_step;  // view of k = 0
-    const int sbase = mb * A.M.nvm + vfirst;                                // its scratch slot
-    const CUtensorMap* gmap = &gmaps.m[0];
-#pragma unroll
-    for (int i = 1; i < NM; i++)
-        if (mb == i) gmap = &gmaps.m[i];
-    const int NY = G.numY, NZ = G.numZ, NU1 = G.N_u1;
-    const int ns = A.ns;
-
-    TG* ringp = reinterpret_cast<TG*>(smem);                                           // [ns][2][sstride]
-    const int vcap = A.v1cap;
-    GEntry* s_ent = reinterpret_cast<GEntry*>(smem + size_t(ns) * 2 * A.sstride * sizeof(TG));  // [vcap][16]
-    float2* s_wt = reinterpret_cast<float2*>(s_ent + vcap * GWARPS);                    // [vg][vcap][16]
-    int2* s_sl = reinterpret_cast<int2*>(s_wt + size_t(A.vg) * vcap * GPL);             // (v1, first staged row)
-    uint64_t* full = reinterpret_cast<uint64_t*>(s_sl + vcap);                          // [GNSMAX]
-    uint64_t* empty = full + GNSMAX;                                                    // [GNSMAX]
-    int* s_n = reinterpret_cast<int*>(empty + GNSMAX);
-    volatile int* s_abort = s_n + 1;
-    int* s_round = s_n + 2;  // [GNSMAX]
-
-    // ---- slopes whose rows reach the tile (warp 0), compacted in order
-    if (warp == 0) {
+    const int NY = G.numY, NU1 = G.N_u1;
+    const int p0 = blockIdx.x * A.planes, r0 = blockIdx.y * A.rows;
+    const size_t base = (size_t(blockIdx.x) * gridDim.y + blockIdx.y) * A.nv1;
+    __shared__ int s_n;
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
         int n = 0;
         for (int vb = A.vr.iv1_begin; vb < A.vr.iv1_end; vb += 32) {
             const int v1 = vb + lane;
@@ -224,314 +121,343 @@ k_bwd_zgather(const __grid_constant__ GMaps<NM> gmaps, float* __restrict__ B, co
             int grow = 0;
             if (v1 < A.vr.iv1_end) {
                 int dmin = 1 << 30, dmax = -(1 << 30);
-                for (int p = 0; p < GPL && p0 + p < NY; p++) {
+                const int2 ub1 = A.T.ub1[v1];
+                for (int p = 0; p < A.planes && p0 + p < NY; p++) {
                     const int d = A.T.zt[size_t(v1) * NY + p0 + p].d;
                     dmin = min(dmin, d);
                     dmax = max(dmax, d);
-                }
-                grow = r0 - dmax - 1;
-                const int2 ub1 = A.T.ub1[v1];
-                for (int p = 0; p < GPL && p0 + p < NY && !ok; p++) {
-                    const int d = A.T.zt[size_t(v1) * NY + p0 + p].d;
-                    // rows of the CTA that can receive this slope on plane p
-                    const int lo = r0 - d - 1, hi = r0 + GROWS - 1 - d;
+                    // planogram rows that the tile touches on plane p
+                    const int lo = r0 - d - 1, hi = r0 + A.rows - 1 - d;
                     if (hi < 0 || lo >= NU1) continue;
                     if (ADJ) {
-                        ok = !(hi < ub1.x || lo > ub1.y);
+                        ok |= !(hi < ub1.x || lo > ub1.y);
                     } else {
                         const int2 zv = A.T.zvis[size_t(v1) * NY + p0 + p];
-                        ok = !(r0 + GROWS - 1 < zv.x || r0 > zv.y);
+                        ok |= !(r0 + A.rows - 1 < zv.x || r0 > zv.y);
                     }
                 }
-                if (ok && dmax - dmin > A.brb - (GROWS + 1)) {
+                grow = r0 - dmax - 1;
+                if (ok && dmax - dmin + A.rows + 1 > A.nrb) {  // a host-side bound does not hold
                     atomicOr(A.err, kErrLayout);
                     ok = false;
                 }
             }
             const unsigned bal = __ballot_sync(0xffffffffu, ok);
-            const int idx = n + __popc(bal & ((1u << lane) - 1u));
-            if (ok && idx < vcap) s_sl[idx] = make_int2(v1, grow);
+            if (ok) A.list[base + n + __popc(bal & ((1u << lane) - 1u))] = make_int2(v1, grow);
             n += __popc(bal);
         }
         if (lane == 0) {
-            if (n > vcap) {  // the host sizes the tables; never index past them
-                atomicOr(A.err, kErrLayout);
-                n = vcap;
-            }
-            s_n[0] = n;
-            *s_abort = 0;
-            for (int s = 0; s < ns; s++) {
-                mbar_init(&full[s], 1);
-                mbar_init(&empty[s], GWARPS);
-                s_round[s] = -1;
-            }
-            fence_barrier_init();
+            s_n = n;
+            A.cnt[blockIdx.x * gridDim.y + blockIdx.y] = n;
         }
     }
     __syncthreads();
-    const int nlive = s_n[0];
-
-    // ---- per (slope, warp): plane modes, window offsets, pattern, masks
-    for (int e = tid; e < nlive * GWARPS; e += GNT) {
-        const int li = e / GWARPS, w = e - li * GWARPS;
-        const int wq = w % GPG, wr = w / GPG;
-        const int2 sl = s_sl[li];
+    if (blockIdx.x == 0 && blockIdx.y == 0)
+        for (int i = threadIdx.x; i < A.nchunks; i += blockDim.x) A.next[i] = 0;
+    const int nlive = s_n;
+    for (int e = threadIdx.x; e < nlive * kZWarps; e += blockDim.x) {
+        const int li = e / kZWarps, w = e - li * kZWarps;
+        if (w >= A.pg * A.rg) continue;
+        const int2 sl = A.list[base + li];
         const int v1 = sl.x, grow = sl.y;
-        const int zr = r0 + wr * GK;  // first row of warp w
+        GRec* R = A.rec + base + li;
+        const int q = w % A.pg, zr = r0 + (w / A.pg) * NK;  // first row of the warp
         const int2 ub1 = A.T.ub1[v1];
-        int dz[GP], mode[GP];
-        int2 zv[GP];
         int dmx = -(1 << 30);
-#pragma unroll
-        for (int u = 0; u < GP; u++) {
-            const int y = p0 + wq * GP + u;
-            dz[u] = 0;
-            mode[u] = 0;
-            zv[u] = make_int2(0, -1);
-            if (y >= NY) continue;
-            dz[u] = A.T.zt[size_t(v1) * NY + y].d;
-            const int lo = zr - dz[u] - 1, hi = zr + GK - 1 - dz[u];  // g rows touched
+        for (int u = 0; u < NV; u++) dmx = max(dmx, A.T.zt[size_t(v1) * NY + min(p0 + q * NV + u, NY - 1)].d);
+        uint32_t offs = 0;
+        unsigned long long rows = 0;
+        int full = 0, some = 0;
+        bool bad = false;
+        for (int u = 0; u < NV; u++) {
+            const int yq = p0 + q * NV + u, y = min(yq, NY - 1);
+            const Shift zs = A.T.zt[size_t(v1) * NY + y];
+            const int o = dmx - zs.d;
+            bad |= o > kZSpread;
+            offs |= uint32_t(min(o, kZSpread)) << (2 * u);
+            if (w < A.pg) R->w[q * NV + u] = zs.w;
+            if (yq >= NY) continue;
+            const int lo = zr - zs.d - 1, hi = zr + NK - 1 - zs.d;  // planogram rows touched
             if (hi < 0 || lo >= NU1) continue;
             if (ADJ) {
                 if (hi < ub1.x || lo > ub1.y) continue;
-                mode[u] = (lo >= ub1.x && hi <= ub1.y) ? 1 : 2;
+                some++;
+                full += lo >= ub1.x && hi <= ub1.y;
             } else {
-                zv[u] = A.T.zvis[size_t(v1) * NY + y];
-                if (zr + GK - 1 < zv[u].x || zr > zv[u].y) continue;
-                mode[u] = (zr >= zv[u].x && zr + GK - 1 <= zv[u].y) ? 1 : 2;
-            }
-            dmx = max(dmx, dz[u]);
-        }
-        GEntry en{0u, 0u, 0u, 0u};
-        if (dmx != -(1 << 30)) {
-            const int wfirst = zr - dmx - 1;  // g row of window row 0
-            const int wrow = wfirst - grow;   // its row in the stage
-            bool bad = wrow < 0 || wrow + GWN > A.brb + 2;
-            uint32_t code = 0, ivl = 0, vm = 0;
-            bool allfull = true;
-            int offs = 0, olast = -1;
-            for (int i = 0; i < GWN; i++)
-                if (wfirst + i >= ub1.x && wfirst + i <= ub1.y) vm |= 1u << i;
-#pragma unroll
-            for (int u = 0; u < GP; u++) {
-                const int o = dmx - dz[u];
-                uint32_t iv = 0u;  // no rows
-                if (mode[u]) {
-                    if (o > GDW) bad = true;
-                    code |= uint32_t(mode[u] | (min(o, 3) << 2)) << (4 * u);
-                    if (ADJ || mode[u] == 1) {
-                        iv = 0xffu;  // rows 0..7 (adjoint: invisible window rows are zeroed instead)
-                    } else {
-                        const int ka = max(zv[u].x - zr, 0), kb = min(zv[u].y - zr, GK - 1);
-                        iv = kb >= ka ? (0xffu >> (7 - kb)) & (0xffu << ka) & 0xffu : 0u;
-                    }
-                }
-                ivl |= iv << (8 * u);
-                allfull = allfull && mode[u] == 1;
-                // planes that receive nothing take a neighbour's offset
-                // (monotone), so that a pattern can cover the group
-                const int oe = mode[u] ? o : (olast >= 0 ? olast : dmx - dz[u]);
-                if (mode[u]) olast = o;
-                offs |= (min(oe, 3) & 3) << (2 * u);
-            }
-            // leading planes without rows: the offset of the first active one
-            if (!mode[0]) {
-                int ofirst = 0;
-                for (int u = GP - 1; u >= 0; u--)
-                    if (mode[u]) ofirst = dmx - dz[u];
-                for (int u = 0; u < GP && !mode[u]; u++) offs = (offs & ~(3 << (2 * u))) | ((ofirst & 3) << (2 * u));
-            }
-            int pid = kPatGen;
-            for (int c = 0; c < kNumPat; c++)
-                if (gpat_offsets(c) == offs) pid = allfull ? c : c + 8;
-            if (bad) {
-                atomicOr(A.err, kErrLayout);
-            } else {
-                en.code = code | uint32_t(pid) << 16 | uint32_t(wrow) << 20;
-                en.vm = vm;
-                en.ivl = ivl;
+                const int2 zv = A.T.zvis[size_t(v1) * NY + y];
+                const int ka = max(zv.x - zr, 0), kb = min(zv.y - zr, NK - 1);
+                if (kb < ka) continue;
+                some++;
+                full += ka == 0 && kb == NK - 1;
+                const unsigned long long bits = ((~0ull >> (63 - kb)) >> ka) << ka;
+                rows |= bits << (64 / NV * u);
             }
         }
-        s_ent[li * GWARPS + w] = en;
+        const int wfirst = zr - dmx - 1, wrow = wfirst - grow;  // planogram row and staged row of window row 0
+        if (ADJ)
+            for (int i = 0; i < NK + kZSpread + 1; i++)
+                if (wfirst + i >= ub1.x && wfirst + i <= ub1.y) rows |= 1ull << i;
+        bad |= wrow < 0 || wrow + NK + 1 > A.nrb;
+        if (bad) atomicOr(A.err, kErrLayout);
+        R->code[w] = bad || !some ? 0u : offs | uint32_t(full == NV ? 1 : 2) << 8 | uint32_t(wrow) << 16;
+        R->mask[w] = rows;
     }
-    // ---- weights (S (1 - w), S w) per view, slope and plane
-    for (int e = tid; e < nvw * nlive * GPL; e += GNT) {
-        const int k = e / (nlive * GPL), rem = e - k * (nlive * GPL);
-        const int li = rem / GPL, p = rem - li * GPL;
-        const int v1 = s_sl[li].x;
-        const int v0 = vbase + k * A.vr.iv0_step;
-        const int y = min(p0 + p, NY - 1);
-        const float S = A.T.S[size_t(v1) * G.N_v0 + v0];
-        const float w = A.T.zt[size_t(v1) * NY + y].w;
-        s_wt[(k * vcap + li) * GPL + p] = make_float2(S * (1.0f - w), S * w);
+}
+
+// The z taps of the transpose: B[view][y][z][c] = sum over the slopes of
+// S (1 - w) g[v1][v0][z - d][c] + S w g[v1][v0][z - d - 1][c].
+//
+// Persistent CTAs as in k_fwd_zsum, with planes and slopes exchanged: a tile
+// is one view x a block of planes x rows x 64 columns (from the first column
+// that a voxel of those planes reads), a warp sums NV planes x NK rows x 2
+// columns per lane over the slopes that reach the tile, and the producer
+// stages the planogram rows of two slopes at a time with their table records.
+// Bound as k_fwd_zsum by FP32 issue (measured 820 cycles per slope for 576 of
+// packed FMAs).  At the edges of the visible range (a quarter to a third of
+// the (warp, slope) pairs) the taps are predicated per output row (reference
+// semantics) or take zeros for masked window rows (adjoint), a plane at a
+// time.
+//
+// TG: planogram storage (float or bfloat16); B and the arithmetic are FP32.
+// BULK: planogram rows are multiples of 16 bytes and arrive by a tiled TMA copy
+// (no multicast); else the producer's lanes copy a column pair each.
+template <bool ADJ, class TG, int NM, bool BULK, int NV, int NK>
+__global__ void __launch_bounds__(kZThreads, 1)
+k_bwd_zgather(const __grid_constant__ GMaps<NM> gmaps, float* __restrict__ B, const __grid_constant__ ZgatherArgs A)
+{
+    extern __shared__ __align__(128) unsigned char smem[];
+    ZCtl* ctl = reinterpret_cast<ZCtl*>(smem + size_t(A.ns) * A.stage);
+    ZStage* s_info = ctl->info;
+    uint64_t *full = ctl->full, *empty = ctl->empty;
+    volatile int* s_abort = &ctl->abort;
+    const petl_geom& G = A.G;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int NY = G.numY, NZ = G.numZ, NX = G.numX, ns = A.ns;
+    constexpr int EB = int(sizeof(TG));
+    if (tid == 0) {
+        *s_abort = 0;
+        for (int s = 0; s < ns; s++) {
+            mbar_init(&full[s], BULK ? 1 : 33);  // the record's copy, and each lane's pairs
+            mbar_init(&empty[s], A.nw);
+        }
+        fence_barrier_init();
     }
     __syncthreads();
 
-    // ---- the ring: stage j holds slopes 2p and 2p + 1 (p = j mod nsp) of view j / nsp
-    const int nsp = (nlive + 1) / 2;
-    const int nst = nvw * nsp;
-    const uint32_t box_bytes = uint32_t(GCOLS) * uint32_t(A.brb) * uint32_t(sizeof(TG));
-    bool dead = false;
-    // stage j reuses its slot once every warp has released stage j - ns
-    auto issue = [&](int j) {
-        const int slot = j % ns, round = j / ns;
-        if (round > 0 && !mbar_wait(&empty[slot], uint32_t((round - 1) & 1), A.err, A.wait_limit)) return false;
-        if (*s_abort) return false;
-        fence_proxy_async_smem();
-        const int k = j / nsp, pr = j - k * nsp;
-        const int v0 = vbase + k * A.vr.iv0_step;
-        const int np = min(2, nlive - 2 * pr);
-        mbar_arrive_expect_tx(&full[slot], box_bytes * uint32_t(np));
-        for (int h = 0; h < np; h++) {
-            const int2 sl = s_sl[2 * pr + h];
-            tma_load_4d(ringp + size_t(2 * slot + h) * A.sstride, gmap, &full[slot], col0, sl.y, v0, sl.x);
+    if (warp >= A.nw) {
+        producer_registers();
+        if (warp > A.nw) {
+            __syncthreads();
+            return;
         }
-        s_round[slot] = round;
-        return true;
-    };
-    if (tid == 0)
-        for (int j = 0; j < ns - 1 && j < nst; j++) issue(j);
-    // the next stage this warp starts: the first j >= ns - 1 with j % 16 == warp
-    int my_next = warp + GWARPS * ((ns - 1 - warp + GWARPS - 1) / GWARPS);
-    if (my_next < ns - 1) my_next += GWARPS;
-
-    float2 Z[GP][GK];
+        int j = 0;  // stages started
+        bool dead = false;
+        auto claim = [&]() {
+            const int slot = j % ns, round = j / ns;
+            const bool ok = round == 0 || ring_wait(&empty[slot], uint32_t((round - 1) & 1), A.err, s_abort, A.wait_limit);
+            return __all_sync(0xffffffffu, ok && *s_abort == 0) != 0;
+        };
+        int after = 0;  // the tile after the current one (lane 0)
+        for (int tile = blockIdx.x; tile < A.ntile && !dead; tile = __shfl_sync(0xffffffffu, after, 0)) {
+            if (lane == 0) after = int(gridDim.x) + atomicAdd(A.next, 1);
+            int t = tile;
+            const int colblk = t % A.n_colblk;
+            t /= A.n_colblk;
+            const int rowblk = t % A.n_rowblk;
+            t /= A.n_rowblk;
+            const int plblk = t % A.n_plblk, vi = t / A.n_plblk;  // view slot
+            const int mb = NM == 1 ? 0 : vi / A.M.nvm, mv = vi - mb * A.M.nvm;
+            if (mv >= member_pick<NM>(A.M.nv, mb)) continue;  // a member with fewer views than the slots
+            const int v0 = member_pick<NM>(A.M.first, mb) + mv * A.vr.iv0_step;
+            const int p0 = plblk * A.planes, r0 = rowblk * A.rows;
+            // columns that a voxel of the tile's planes reads (and, for the
+            // adjoint, that are visible)
+            const int da = A.T.xt[size_t(v0) * NY + p0].d;
+            const int db = A.T.xt[size_t(v0) * NY + min(p0 + A.planes, NY) - 1].d;
+            int clo = max(-max(da, db) - 1, 0), chi = min(NX - 1 - min(da, db), G.N_u0 - 1);
+            if (ADJ) {
+                const int2 u = A.T.ub0[v0];
+                clo = max(clo, u.x);
+                chi = min(chi, u.y);
+            }
+            clo &= ~(16 / EB - 1);  // a TMA copy starts on a 16-byte boundary
+            const int col0 = clo + colblk * kZCols;
+            if (col0 > chi) continue;
+            const size_t tb = size_t(plblk) * A.n_rowblk + rowblk;
+            const int nlive = A.cnt[tb];
+            const int2* list = A.list + tb * A.nv1;
+            // the slopes' ray scales, a slope per lane and register
+            float S[GV1MAX / 32];
 #pragma unroll
-    for (int u = 0; u < GP; u++)
-#pragma unroll
-        for (int k = 0; k < GK; k++) Z[u][k] = make_float2(0.0f, 0.0f);
-
-    // the z sums of view k go to the scratch (columns outside the view's
-    // visible u0 range zeroed for the adjoint) and restart from zero
-    auto store_view = [&](int k) {
-        const int vi = sbase + k;  // scratch slot
-        const int v0 = vbase + k * A.vr.iv0_step;
-        const int2 u0r = ADJ ? A.T.ub0[v0] : make_int2(0, G.N_u0 - 1);
-        const int c = col0 + 2 * lane;
-        const bool vx = c >= u0r.x && c <= u0r.y, vy = c + 1 >= u0r.x && c + 1 <= u0r.y;
-#pragma unroll
-        for (int u = 0; u < GP; u++) {
-            const int y = p0 + q * GP + u;
-#pragma unroll
-            for (int kk = 0; kk < GK; kk++) {
-                const int z = z0 + kk;
-                if (y < NY && z < NZ && c < G.N_u0) {
-                    float* dst = B + ((size_t(vi) * NY + y) * NZ + z) * A.NUc + c;
-                    const float2 v = make_float2(vx ? Z[u][kk].x : 0.0f, vy ? Z[u][kk].y : 0.0f);
-                    if (c + 1 < G.N_u0)
-                        __stcs(reinterpret_cast<float2*>(dst), v);
-                    else
-                        dst[0] = v.x;
+            for (int i = 0; i < GV1MAX / 32; i++)
+                S[i] = 32 * i + lane < nlive ? A.T.S[size_t(list[32 * i + lane].x) * G.N_v0 + v0] : 0.0f;
+            auto scale = [&](int i) {
+                const float s = i < 32 ? S[0] : i < 64 ? S[1] : i < 96 ? S[2] : S[3];
+                return __shfl_sync(0xffffffffu, s, i & 31);
+            };
+            const int nst = max(1, (nlive + 1) / 2);  // a tile without slopes still writes its zeros
+            for (int i = 0; i < nst; i++) {
+                if (!claim()) {
+                    dead = true;
+                    break;
                 }
-                Z[u][kk] = make_float2(0.0f, 0.0f);
+                const int slot = j % ns, np = max(0, min(2, nlive - 2 * i));
+                unsigned char* st = smem + size_t(slot) * A.stage;
+                const float s0 = scale(2 * i), s1 = scale(min(2 * i + 1, GV1MAX - 1));
+                if (lane == 0) {
+                    s_info[slot] = ZStage{2 * i, np | (i == 0 ? kZFirst : 0) | (i == nst - 1 ? kZLast : 0), p0, vi, r0,
+                                          col0, s0, s1};
+                    fence_proxy_async_smem();
+                    uint32_t bytes = uint32_t(np) * uint32_t(sizeof(GRec));
+                    if (BULK) bytes += uint32_t(np) * uint32_t(A.nrb) * uint32_t(kZCols * EB);
+                    mbar_arrive_expect_tx(&full[slot], bytes);
+                    if (BULK) {
+                        const CUtensorMap* gmap = &gmaps.m[0];
+#pragma unroll
+                        for (int m = 1; m < NM; m++)
+                            if (mb == m) gmap = &gmaps.m[m];
+                        for (int h = 0; h < np; h++) {
+                            const int2 sl = list[2 * i + h];
+                            tma_load_4d(st + size_t(h) * A.sbytes, gmap, &full[slot], col0, sl.y, v0, sl.x);
+                        }
+                    }
+                    if (np)
+                        bulk_load(st + A.stage - 2 * sizeof(GRec), A.rec + tb * A.nv1 + 2 * i,
+                                  uint32_t(np) * uint32_t(sizeof(GRec)), &full[slot]);
+                }
+                if (!BULK) {
+                    const TG* g = static_cast<const TG*>(member_pick<NM>(A.M.in, mb));
+                    const int c = col0 + 2 * lane;
+                    const bool cok = c < G.N_u0;  // N_u0 is even: both columns of the pair
+                    for (int h = 0; h < np; h++) {
+                        const int2 sl = list[2 * i + h];
+                        const TG* gs = g + (size_t(sl.x) * G.N_v0 + v0) * G.N_u1 * G.N_u0;
+                        const uint32_t dst = smem_addr(st + size_t(h) * A.sbytes) + uint32_t(2 * lane * EB);
+                        for (int r = 0; r < A.nrb; r++) {
+                            const int row = sl.y + r;
+                            const bool ok = cok && unsigned(row) < unsigned(G.N_u1);
+                            pair_load<2 * EB>(dst + uint32_t(r * kZCols * EB), ok ? gs + size_t(row) * G.N_u0 + c : gs, ok);
+                        }
+                    }
+                    pair_arrive(&full[slot]);
+                }
+                __syncwarp();
+                j++;
             }
         }
-    };
-
-    int slot = 0;
-    uint32_t phase = 0;
-    int k = 0, pr = 0;  // view and slope pair of stage j
-    for (int j = 0; j < nst; j++) {
-        if (j + ns - 1 == my_next) {
-            if (lane == 0 && !dead && my_next < nst && !issue(my_next)) dead = true;
-            my_next += GWARPS;
+        if (!dead && claim()) {
+            const int slot = j % ns;
+            if (lane == 0) {
+                s_info[slot].flags = kZEnd;
+                mbar_arrive(&full[slot]);
+            }
+            if (!BULK) mbar_arrive(&full[slot]);
+            j++;
+        } else if (lane == 0) {
+            *s_abort = 1;
         }
-        // the hot wait keeps the compile-time bound (a run-time bound here
-        // measured 1 % slower); the forced give-up reaches this kernel through
-        // the slot waits of issue(), and the warps waiting here for a copy
-        // that was then never started leave on the abort flag
-        if (!dead) dead = !mbar_wait_abortable(&full[slot], phase, A.err, s_abort);
-        if (dead) *s_abort = 1;  // before this warp releases the slot
+        __syncthreads();
+        // a wait gave up: drain the copies still in flight
+        if (*s_abort) {
+            pair_drain();
+            if (lane == 0)
+                for (int i = max(0, j - ns); i < j; i++) mbar_wait(&full[i % ns], uint32_t((i / ns) & 1), nullptr);
+        }
+        return;
+    }
+
+    {
+        consumer_registers();
+        const int q = warp % A.pg, gr = warp / A.pg;
+        int slot = 0;
+        uint32_t phase = 0;
+        auto wait = [&]() {
+            return __all_sync(0xffffffffu, ring_wait(&full[slot], phase, A.err, s_abort, A.wait_limit)) != 0;
+        };
+        bool dead = !wait();
+        while (!dead) {  // tiles
+            const ZStage in = s_info[slot];
+            if (in.flags & kZEnd) break;
+            f2x acc[NV][NK];
+#pragma unroll
+            for (int u = 0; u < NV; u++)
+#pragma unroll
+                for (int k = 0; k < NK; k++) acc[u][k] = 0ull;
+            for (;;) {  // stages
+                const int flags = s_info[slot].flags;
+                const unsigned char* st = smem + size_t(slot) * A.stage;
+                const GRec* rec = reinterpret_cast<const GRec*>(st + A.stage - 2 * sizeof(GRec));
+                const float* sc = &s_info[slot].s0;
 #pragma unroll 1
-        for (int h = 0; h < 2 && !dead; h++) {
-            const int li = 2 * pr + h;
-            if (li >= nlive) break;
-            const GEntry en = s_ent[li * GWARPS + warp];
-            if (!(en.code & 0xffffu)) continue;
-            const TG* Gs = ringp + size_t(2 * slot + h) * A.sstride + (en.code >> 20) * GCOLS + 2 * lane;
-            float2 W[GWN];
+                for (int h = flags & 3; h > 0; h--, rec++, sc++, st += A.sbytes) {
+                    const uint32_t code = rec->code[warp];
+                    if (!(code & 0x300u)) continue;
+                    const auto* W = reinterpret_cast<const typename Pair<TG>::type*>(st) +
+                                    int(code >> 16) * (kZCols / 2) + lane;
+                    f2x wa[NV], wb[NV];
 #pragma unroll
-            for (int i = 0; i < GWN; i++) W[i] = Store<TG>::ld2(Gs + i * GCOLS);
-            const float4* W4 = reinterpret_cast<const float4*>(s_wt + (size_t(k) * vcap + li) * GPL + q * GP);
-            const float4 wa = W4[0], wb = W4[1];
-            const uint32_t pid = (en.code >> 16) & 15u;
-            if (pid < 8u) {  // fully visible planes
-                switch (pid) {
-                    case 0: g_taps4<0>(Z, W, wa, wb); break;
-                    case 1: g_taps4<1>(Z, W, wa, wb); break;
-                    case 2: g_taps4<2>(Z, W, wa, wb); break;
-                    case 3: g_taps4<3>(Z, W, wa, wb); break;
-                    case 4: g_taps4<4>(Z, W, wa, wb); break;
-                    case 5: g_taps4<5>(Z, W, wa, wb); break;
-                    default: g_taps4<6>(Z, W, wa, wb); break;
-                }
-            } else if (pid != uint32_t(kPatGen)) {
-                // edge of the visible range: the adjoint zeroes the window
-                // rows outside the view, the reference keeps per-plane rows
-                if (ADJ) {
-#pragma unroll
-                    for (int i = 0; i < GWN; i++)
-                        if (!((en.vm >> i) & 1u)) W[i] = make_float2(0.0f, 0.0f);
-                }
-                switch (pid) {
-                    case 8: g_taps4_ivl<0>(Z, W, wa, wb, en.ivl); break;
-                    case 9: g_taps4_ivl<1>(Z, W, wa, wb, en.ivl); break;
-                    case 10: g_taps4_ivl<2>(Z, W, wa, wb, en.ivl); break;
-                    case 11: g_taps4_ivl<3>(Z, W, wa, wb, en.ivl); break;
-                    case 12: g_taps4_ivl<4>(Z, W, wa, wb, en.ivl); break;
-                    case 13: g_taps4_ivl<5>(Z, W, wa, wb, en.ivl); break;
-                    default: g_taps4_ivl<6>(Z, W, wa, wb, en.ivl); break;
-                }
-            } else {
-                const float w0s[GP] = {wa.x, wa.z, wb.x, wb.z}, w1s[GP] = {wa.y, wa.w, wb.y, wb.w};
-#pragma unroll
-                for (int u = 0; u < GP; u++) {
-                    const uint32_t c = (en.code >> (4 * u)) & 15u;
-                    if (!(c & 3u)) continue;
-                    const int o = int(c >> 2);
-                    if ((c & 3u) == 1u) {
-                        switch (o) {
-                            case 0: g_taps<0, false>(Z[u], W, w0s[u], w1s[u], 0u, 0u); break;
-                            case 1: g_taps<1, false>(Z[u], W, w0s[u], w1s[u], 0u, 0u); break;
-                            default: g_taps<2, false>(Z[u], W, w0s[u], w1s[u], 0u, 0u); break;
+                    for (int u = 0; u < NV; u++) {
+                        const float w = rec->w[q * NV + u], S = *sc;
+                        wa[u] = f2_dup(S * (1.0f - w));
+                        wb[u] = f2_dup(S * w);
+                    }
+                    if ((code & 0x300u) == 0x100u) {
+                        if constexpr (NV == 4) {
+                            switch (code & 0xffu) {
+#define PETL_ZCASE(PC) case PC: z_taps<PC, false>(acc, W, wa, wb); break;
+                                PETL_ZCASE(0x00) PETL_ZCASE(0x40) PETL_ZCASE(0x50) PETL_ZCASE(0x90) PETL_ZCASE(0x54)
+                                PETL_ZCASE(0x94) PETL_ZCASE(0xA4) PETL_ZCASE(0xE4) PETL_ZCASE(0x01) PETL_ZCASE(0x05)
+                                PETL_ZCASE(0x15) PETL_ZCASE(0x06) PETL_ZCASE(0x16) PETL_ZCASE(0x1A) PETL_ZCASE(0x1B)
+                            }
+                        } else {
+                            switch (code & 0xfu) {
+                                PETL_ZCASE(0x0) PETL_ZCASE(0x4) PETL_ZCASE(0x8) PETL_ZCASE(0xC) PETL_ZCASE(0x1)
+                                PETL_ZCASE(0x2) PETL_ZCASE(0x3)
+#undef PETL_ZCASE
+                            }
                         }
                     } else {
-                        // rows at the edge of the visible range: per-row masks
-                        const uint32_t rows = (en.ivl >> (8 * u)) & 0xffu;
-                        const uint32_t vm = ADJ ? en.vm : 0xffffffffu;
-                        const uint32_t om = ADJ ? 0xffffffffu : rows;
-                        switch (o) {
-                            case 0: g_taps<0, true>(Z[u], W, w0s[u], w1s[u], vm, om); break;
-                            case 1: g_taps<1, true>(Z[u], W, w0s[u], w1s[u], vm, om); break;
-                            default: g_taps<2, true>(Z[u], W, w0s[u], w1s[u], vm, om); break;
+                        const unsigned long long m = rec->mask[warp];
+#pragma unroll
+                        for (int u = 0; u < NV; u++) {
+                            const int o = int((code >> (2 * u)) & 3u);
+                            z_taps_edge<ADJ>(acc[u], W + o * (kZCols / 2), wa[u], wb[u],
+                                             uint32_t(m >> (ADJ ? o : 64 / NV * u)));
                         }
                     }
                 }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&empty[slot]);
+                if (++slot == ns) {
+                    slot = 0;
+                    phase ^= 1u;
+                }
+                if (flags & kZLast) break;
+                if (!wait()) {
+                    dead = true;
+                    break;
+                }
             }
+            if (dead) break;
+            // the z sums of the tile
+            const int c = in.col0 + 2 * lane, z0 = in.row0 + gr * NK;
+            f2x* out = ctl->out[warp][0] + lane;
+#pragma unroll 1
+            for (int i = 0; i < NV * NK / kZOut; i++) {
+                out_rows(acc, out, i);
+                const int y = in.a + q * NV + i / (NK / kZOut), zr = z0 + i % (NK / kZOut) * kZOut;
+                if (y >= NY) break;
+                float* dst = B + ((size_t(in.b) * NY + y) * NZ + zr) * A.NUc + c;
+                if (c < G.N_u0)  // N_u0 is even: both columns of the pair
+#pragma unroll 4
+                    for (int k = 0; k < min(kZOut, NZ - zr); k++)
+                        __stcs(reinterpret_cast<float2*>(dst + size_t(k) * A.NUc), f2_unpack(out[k * 32]));
+            }
+            dead = !wait();
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&empty[slot]);
-        if (++slot == ns) {
-            slot = 0;
-            phase ^= 1u;
-        }
-        if (pr == nsp - 1) {
-            if (!dead) store_view(k);
-            pr = 0;
-            k++;
-        } else {
-            pr++;
-        }
+        if (dead) *s_abort = 1;
     }
-    // a tile that no slope reaches still writes its (zero) sums
-    if (nsp == 0)
-        for (int k = 0; k < nvw; k++) store_view(k);
-    if (__syncthreads_or(dead)) {
-        // a wait gave up: drain the copies still in flight
-        if (tid == 0)
-            for (int s = 0; s < ns; s++)
-                if (s_round[s] >= 0) mbar_wait(&full[s], uint32_t(s_round[s] & 1), nullptr);
-    }
+    __syncthreads();
 }
 
 struct XgatherArgs {
@@ -544,7 +470,14 @@ struct XgatherArgs {
     float scale;
     Tables T;
     Members M;       // volumes (out) and views of the chunk
-    int bplanes;     // planes of the scratch: numY, or 1 when its z sums do not depend on the plane
+    int adjoint;     // only the view's visible columns count (the scratch holds no others)
+};
+
+// x shift of a view on a plane and the scratch columns that count
+struct __align__(16) XView {
+    int d;
+    float w;
+    int lo, n;
 };
 
 constexpr int XR = 4;         // volume rows z per k_bwd_xgather thread
@@ -559,14 +492,19 @@ template <int NM>
 __global__ void __launch_bounds__(256) k_bwd_xgather(const float* __restrict__ B, float* __restrict__ part,
                                                      const XgatherArgs A)
 {
-    extern __shared__ Shift s_xs[];  // [views of the member] x shifts of plane y
+    extern __shared__ XView s_xs[];  // [views of the member]
     const petl_geom& G = A.G;
     const int NY = G.numY, NZ = G.numZ, NX = G.numX, NU0 = G.N_u0, NUc = A.NUc;
     const int mb = NM == 1 ? 0 : blockIdx.z / NY, y = blockIdx.z - mb * NY;
     const int x = blockIdx.x * 256 + threadIdx.x, z0 = blockIdx.y * XR;
     const int first = member_pick<NM>(A.M.first, mb), nvb = member_pick<NM>(A.M.nv, mb);
     float* __restrict__ f = static_cast<float*>(member_pick<NM>(A.M.out, mb));
-    for (int vi = threadIdx.x; vi < nvb; vi += 256) s_xs[vi] = A.T.xt[size_t(first + vi * A.step) * NY + y];
+    for (int vi = threadIdx.x; vi < nvb; vi += 256) {
+        const int v0 = first + vi * A.step;
+        const Shift xs = A.T.xt[size_t(v0) * NY + y];
+        const int2 u = A.adjoint ? A.T.ub0[v0] : make_int2(0, NU0 - 1);
+        s_xs[vi] = XView{xs.d, xs.w, u.x, max(0, u.y - u.x + 1)};
+    }
     __syncthreads();
     if (x >= NX) return;
     const int nz = min(XR, NZ - z0);
@@ -575,17 +513,16 @@ __global__ void __launch_bounds__(256) k_bwd_xgather(const float* __restrict__ B
     for (int r = 0; r < XR; r++)
         acc[r] = (!A.first && r < nz) ? part[(size_t(z0 + r) * NY + y) * NX + x] : 0.0f;
     const int rlast = nz - 1;
-    const int yb = A.bplanes == 1 ? 0 : y;  // the scratch plane of y
-    const float* Bm = B + size_t(mb) * A.M.nvm * A.bplanes * NZ * NUc;
+    const float* Bm = B + size_t(mb) * A.M.nvm * NY * NZ * NUc;
 #pragma unroll 4
     for (int vi = 0; vi < nvb; vi++) {
-        const Shift xs = s_xs[vi];
+        const XView xs = s_xs[vi];
         const float wx1 = xs.w, wx0 = 1.0f - xs.w;
         const int j0 = x - xs.d;  // scratch column of tap 0
-        const bool okm = unsigned(j0 - 1) < unsigned(NU0), ok0 = unsigned(j0) < unsigned(NU0);
+        const bool okm = unsigned(j0 - 1 - xs.lo) < unsigned(xs.n), ok0 = unsigned(j0 - xs.lo) < unsigned(xs.n);
         // in-bounds addresses for every tap; the out-of-range ones are selected away
         const int jm = min(max(j0 - 1, 0), NU0 - 1), jz = min(max(j0, 0), NU0 - 1);
-        const float* Bv = Bm + ((size_t(vi) * A.bplanes + yb) * NZ + z0) * NUc;
+        const float* Bv = Bm + ((size_t(vi) * NY + y) * NZ + z0) * NUc;
 #pragma unroll
         for (int r = 0; r < XR; r++) {
             const int rr = min(r, rlast);
@@ -604,82 +541,161 @@ __global__ void __launch_bounds__(256) k_bwd_xgather(const float* __restrict__ B
     }
 }
 
-// z sums of one slope with v1 = 0 (the rebinned planogram of FBP), whose
-// z taps and visible rows are the same on every plane: B[view][z][c] =
-// S (1 - w) g[z - d][c] then + S w g[z - d - 1][c], the operations and
-// masks of k_bwd_zgather for a single slope (rows outside the planogram
-// read zero; the adjoint zeroes rows outside the visible u1 range and
-// columns outside the view's visible u0 range, the reference semantics
-// leave rows z outside the voxel test at zero).  Thread = column c of row z
-// of one view; grid (ceil(N_u0 / 256), numZ, views).
+// One slope with v1 = 0 (the rebinned planogram of FBP): its z taps and
+// visible rows are the same on every plane.  k_bwd_zflat writes the z sums
+// once per view, B[view][c][z] = S (1 - w) g[z - d][c] then + S w g[z - d - 1][c],
+// the operations and masks of k_bwd_zgather for a single slope (rows outside
+// the planogram read zero; the adjoint zeroes rows outside the visible u1
+// range, the reference semantics leave rows z outside the voxel test at
+// zero).  A block transposes 32 columns x 32 rows of one view.  Grid
+// (ceil(N_u0 / 32), ceil(NZc / 32), views), 32 x 8 threads.
 struct FlatArgs {
     petl_geom G;
-    int iv1;    // the slope
-    int first;  // first view
-    int step;   // view step
-    int NUc;    // scratch row pitch
+    int iv1;         // the slope
+    int first;       // first view
+    int step;        // view step
+    int nv;          // views
+    int NZc;         // scratch row pitch (rows z, even)
+    int accumulate;  // add to the volume instead of overwriting it
+    float scale;
     Tables T;
 };
 
 template <bool ADJ>
 __global__ void __launch_bounds__(256) k_bwd_zflat(const float* __restrict__ g, float* __restrict__ B, const FlatArgs A)
 {
+    __shared__ float tile[32][33];
     const petl_geom& G = A.G;
-    const int c = blockIdx.x * 256 + threadIdx.x, z = blockIdx.y, vi = blockIdx.z;
-    if (c >= G.N_u0) return;
+    const int c0 = blockIdx.x * 32, z0 = blockIdx.y * 32, vi = blockIdx.z;
     const int v0 = A.first + vi * A.step;
     const Shift zs = A.T.zt[size_t(A.iv1) * G.numY];  // plane 0: every plane has the same
     const float S = A.T.S[size_t(A.iv1) * G.N_v0 + v0];
     const float w0 = S * (1.0f - zs.w), w1 = S * zs.w;
-    const int2 ub1 = A.T.ub1[A.iv1];
-    auto row = [&](int r) {
-        const bool in = r >= 0 && r < G.N_u1 && (!ADJ || (r >= ub1.x && r <= ub1.y));
-        return in ? g[((size_t(A.iv1) * G.N_v0 + v0) * G.N_u1 + r) * G.N_u0 + c] : 0.0f;
-    };
-    float zsum = 0.0f;
-    bool live;
-    if (ADJ) {
-        live = true;
-    } else {
-        const int2 zv = A.T.zvis[size_t(A.iv1) * G.numY];
-        live = z >= zv.x && z <= zv.y;
+    const int2 ub1 = A.T.ub1[A.iv1], zv = A.T.zvis[size_t(A.iv1) * G.numY];
+    const int c = c0 + threadIdx.x;
+    for (int r = threadIdx.y; r < 32; r += 8) {
+        const int z = z0 + r;
+        auto row = [&](int i) {
+            const bool in = i >= 0 && i < G.N_u1 && c < G.N_u0 && (!ADJ || (i >= ub1.x && i <= ub1.y));
+            return in ? g[((size_t(A.iv1) * G.N_v0 + v0) * G.N_u1 + i) * G.N_u0 + c] : 0.0f;
+        };
+        const bool live = z < G.numZ && (ADJ || (z >= zv.x && z <= zv.y));
+        tile[r][threadIdx.x] = live ? fmaf(w1, row(z - zs.d - 1), fmaf(w0, row(z - zs.d), 0.0f)) : 0.0f;
     }
-    if (live) zsum = fmaf(w1, row(z - zs.d - 1), fmaf(w0, row(z - zs.d), 0.0f));
-    if (ADJ) {
-        const int2 u0r = A.T.ub0[v0];
-        if (c < u0r.x || c > u0r.y) zsum = 0.0f;
+    __syncthreads();
+    const int z = z0 + threadIdx.x;
+    for (int r = threadIdx.y; r < 32; r += 8)
+        if (c0 + r < G.N_u0 && z < A.NZc) B[(size_t(vi) * G.N_u0 + c0 + r) * A.NZc + z] = tile[threadIdx.x][r];
+}
+
+// x taps of the flat z sums into the volume.  A warp takes 64 rows z (two per
+// lane, so every tap is a coalesced eight-byte load whatever the shift) of 8
+// neighbouring x on one plane: 9 loads per view for 16 taps.  The eight warps
+// of a block take neighbouring planes, whose taps meet in L1.  With a thread
+// per x the taps cost two four-byte loads each, and FBP's backprojection at
+// 256x256x128 (129 views) was bound by them (0.70 ms).  The operations of
+// k_bwd_xgather in its order.  Grid (ceil(numX / 8), ceil(numY / 8),
+// ceil(numZ / 64)), 256 threads.
+constexpr int FX = 8;    // x per warp
+constexpr int FVB = 32;  // views whose shifts a block stages at a time
+
+template <bool ADJ>
+__global__ void __launch_bounds__(256) k_bwd_flat_gather(const float* __restrict__ B, float* __restrict__ f,
+                                                        const FlatArgs A)
+{
+    __shared__ XView s_xs[FVB][8];
+    const petl_geom& G = A.G;
+    const int NY = G.numY, NZ = G.numZ, NX = G.numX, NU0 = G.N_u0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int x0 = blockIdx.x * FX, y = blockIdx.y * 8 + warp, z = blockIdx.z * 64 + 2 * lane;
+    const bool zok = z < A.NZc;
+    const f2x* Bz = reinterpret_cast<const f2x*>(B + (zok ? z : 0));
+    const int pitch = A.NZc / 2;
+    f2x acc[FX];
+#pragma unroll
+    for (int k = 0; k < FX; k++) acc[k] = 0ull;
+    for (int vb = 0; vb < A.nv; vb += FVB) {
+        __syncthreads();
+        {
+            const int i = threadIdx.x >> 3, p = threadIdx.x & 7;
+            const int v0 = A.first + (vb + i) * A.step;
+            if (vb + i < A.nv && blockIdx.y * 8 + p < NY) {
+                const Shift xs = A.T.xt[size_t(v0) * NY + blockIdx.y * 8 + p];
+                const int2 u = ADJ ? A.T.ub0[v0] : make_int2(0, NU0 - 1);
+                s_xs[i][p] = XView{xs.d, xs.w, u.x, max(0, u.y - u.x + 1)};
+            }
+        }
+        __syncthreads();
+        if (y >= NY) continue;
+        const int n = min(FVB, A.nv - vb);
+#pragma unroll 2
+        for (int i = 0; i < n; i++) {
+            const XView xs = s_xs[i][warp];
+            const f2x w1 = f2_dup(xs.w), w0 = f2_dup(1.0f - xs.w);
+            const int cb = x0 - xs.d - 1;  // scratch column of tap 1 of x0
+            const f2x* Bv = Bz + size_t(vb + i) * NU0 * pitch;
+            f2x t[FX + 1];
+#pragma unroll
+            for (int k = 0; k <= FX; k++)
+                t[k] = unsigned(cb + k - xs.lo) < unsigned(xs.n) ? __ldg(Bv + size_t(cb + k) * pitch) : 0ull;
+#pragma unroll
+            for (int k = 0; k < FX; k++) acc[k] = f2_add(acc[k], f2_fma(w1, t[k], f2_mul(w0, t[k + 1])));
+        }
     }
-    B[(size_t(vi) * G.numZ + z) * A.NUc + c] = zsum;
+    if (y >= NY) return;
+    const bool quads = (NX & 3) == 0 && (reinterpret_cast<uintptr_t>(f) & 15) == 0;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        if (z + h >= NZ) break;
+        float v[FX];
+#pragma unroll
+        for (int k = 0; k < FX; k++) {
+            const float2 a = f2_unpack(acc[k]);
+            v[k] = h ? a.y : a.x;
+        }
+        float* row = f + (size_t(z + h) * NY + y) * NX + x0;
+#pragma unroll
+        for (int k = 0; k < FX; k += 4) {
+            if (quads && x0 + k + 4 <= NX) {
+                float4* o = reinterpret_cast<float4*>(row + k);
+                if (A.accumulate) {
+                    const float4 p = *o;
+                    *o = make_float4(fmaf(A.scale, v[k], p.x), fmaf(A.scale, v[k + 1], p.y),
+                                     fmaf(A.scale, v[k + 2], p.z), fmaf(A.scale, v[k + 3], p.w));
+                } else {
+                    *o = make_float4(A.scale * v[k], A.scale * v[k + 1], A.scale * v[k + 2], A.scale * v[k + 3]);
+                }
+            } else {
+#pragma unroll
+                for (int i = k; i < k + 4; i++)
+                    if (x0 + i < NX) row[i] = A.accumulate ? fmaf(A.scale, v[i], row[i]) : A.scale * v[i];
+            }
+        }
+    }
 }
 
 int backproject_flat(const petl_geom& G, const float* g, float* f, int mode, int accumulate, float scale,
                      const ViewRange& vr, const Tables& T, cudaStream_t st)
 {
     const int n_v0 = vr.n_v0(G.N_v0);
-    if (n_v0 <= 0 || n_v0 > 4096 || n_v0 > 65535 || G.N_u0 > XMAXN || G.numZ > 65535 || G.numY > 65535)
-        return kNotApplicable;
-    const int NUc = (G.N_u0 + 3) & ~3;
+    if (n_v0 <= 0 || n_v0 > 65535 || G.N_u0 > XMAXN || G.numZ > 65535 || G.numY > 65535) return kNotApplicable;
+    const int NZc = (G.numZ + 1) & ~1;
     float* B = nullptr;
-    if (scratch_alloc(reinterpret_cast<void**>(&B), size_t(n_v0) * G.numZ * NUc * 4, st) != cudaSuccess) {
+    if (scratch_alloc(reinterpret_cast<void**>(&B), size_t(n_v0) * G.N_u0 * NZc * 4, st) != cudaSuccess) {
         cudaGetLastError();
         return kNotApplicable;
     }
-    const FlatArgs FA{G, vr.iv1_begin, vr.iv0_first, vr.iv0_step, NUc, T};
-    const dim3 grid(ceil_div(G.N_u0, 256), unsigned(G.numZ), unsigned(n_v0));
-    if (mode == PETL_BP_ADJOINT)
-        k_bwd_zflat<true><<<grid, 256, 0, st>>>(g, B, FA);
-    else
-        k_bwd_zflat<false><<<grid, 256, 0, st>>>(g, B, FA);
+    const FlatArgs FA{G, vr.iv1_begin, vr.iv0_first, vr.iv0_step, n_v0, NZc, accumulate, scale, T};
+    const dim3 grid(ceil_div(G.N_u0, 32), ceil_div(NZc, 32), unsigned(n_v0));
+    const dim3 ggrid(ceil_div(G.numX, FX), ceil_div(G.numY, 8), ceil_div(G.numZ, 64));
+    if (mode == PETL_BP_ADJOINT) {
+        k_bwd_zflat<true><<<grid, dim3(32, 8), 0, st>>>(g, B, FA);
+        k_bwd_flat_gather<true><<<ggrid, 256, 0, st>>>(B, f, FA);
+    } else {
+        k_bwd_zflat<false><<<grid, dim3(32, 8), 0, st>>>(g, B, FA);
+        k_bwd_flat_gather<false><<<ggrid, 256, 0, st>>>(B, f, FA);
+    }
     note_launch();
-    Members M;
-    M.nb = 1;
-    M.nvm = n_v0;
-    M.first[0] = vr.iv0_first;
-    M.nv[0] = n_v0;
-    M.out[0] = f;
-    const XgatherArgs X{G, vr.iv0_step, NUc, 1, 1, accumulate, scale, T, M, 1};
-    k_bwd_xgather<1><<<dim3(ceil_div(G.numX, 256), ceil_div(G.numZ, XR), unsigned(G.numY)), 256,
-                       size_t(n_v0) * sizeof(Shift), st>>>(B, nullptr, X);
     note_launch();
     const cudaError_t e = cudaGetLastError();
     cudaFreeAsync(B, st);
@@ -717,86 +733,133 @@ int backproject_split_m(const petl_geom& G, const Members& M0, int mode, int acc
     // about ten slopes (the 2-D backprojection of FBP has one) the
     // single-pass kernel is cheaper than that round trip
     if (nv1 < kSplitMinSlopes) return kNotApplicable;
-    // tensor map rows: a multiple of 16 bytes from a 16-byte aligned base
-    if ((G.N_u0 * EB) % 16 != 0) return kNotApplicable;
-    for (int b = 0; b < nb; b++)
-        if ((reinterpret_cast<uintptr_t>(M0.in[b]) & 15) != 0) return kNotApplicable;
+    // staged rows: tiled copies of rows of a multiple of 16 bytes from a
+    // 16-byte aligned base, else lanes copy column pairs (even N_u0)
+    bool bulk = (G.N_u0 * EB) % 16 == 0;
+    if (G.N_u0 & 1) return kNotApplicable;
+    for (int b = 0; b < nb; b++) {
+        const uintptr_t p = reinterpret_cast<uintptr_t>(M0.in[b]);
+        bulk = bulk && (p & 15) == 0;
+        if ((p & (2 * EB - 1)) != 0) return kNotApplicable;
+    }
     if (G.N_u0 > XMAXN || G.numY > 65535 || G.numZ > 65535 * XR) return kNotApplicable;
     if (size_t(G.numY) * nb > 65535) return kNotApplicable;  // k_bwd_xgather grid.z
+    if (std::max(G.numZ, G.N_u1) > GMAXROWS) return kNotApplicable;
     const double step = double(std::max(std::fabs(G.v1_0), std::fabs(G.v1_0 + (G.N_v1 - 1) * G.T_v1))) *
                         double(G.T_x) / double(G.T_z);  // shift change per plane
-    if (shift_spread(GP - 1, step) > GDW) return kNotApplicable;
-    const int brb = GROWS + 1 + shift_spread(GPL - 1, step);
-    if (brb > 254) return kNotApplicable;
+    // four planes share a window of 16 rows where their shifts differ by at
+    // most three rows (shifts below one row per plane), else two planes a
+    // window of 28 rows, as in the forward
+    const int NV = shift_spread(3, step) <= kZSpread ? 4 : 2, NK = NV == 4 ? 12 : 24;
+    if (shift_spread(NV - 1, step) > kZSpread) return kNotApplicable;
     int* err = device_error_ptr();
     if (!err) return kNotApplicable;
 
-    ZgatherArgs A{};
-    A.G = G;
-    A.vr = vr;
-    A.n_colblk = int(ceil_div(G.N_u0, GCOLS));
-    A.n_rowblk = int(ceil_div(G.numZ, GROWS));
-    A.brb = brb;
-    A.sstride = (brb + 2) * GCOLS;  // a multiple of 64 elements: 128-byte aligned slopes
-    A.NUc = (G.N_u0 + 3) & ~3;
-    A.v1cap = nv1;
-    A.T = T;
-    A.err = err;
-    A.wait_limit = wait_limit();
-
     // chunks of views whose scratch fits the budget, balanced in size
-    const size_t per_view = size_t(G.numY) * G.numZ * A.NUc * 4;
+    const int NUc = (G.N_u0 + 3) & ~3;
+    const size_t per_view = size_t(G.numY) * G.numZ * NUc * 4;
     const size_t fit = std::max<size_t>(1, split_scratch_budget() / per_view);
     int nv, nchunks;
     if (nb == 1) {
         nv = int(std::min<size_t>(size_t(nvmax), fit));
-        nv = std::min(nv, 4096);  // k_bwd_xgather stages the chunk's x shifts in shared memory
+        nv = std::min(nv, 3072);  // k_bwd_xgather stages the chunk's x shifts in shared memory
         if (chunk_cap > 0) nv = std::min(nv, chunk_cap);
         nchunks = (nvmax + nv - 1) / nv;
         nv = (nvmax + nchunks - 1) / nchunks;
     } else {
-        if (size_t(nb) * nvmax > fit || nvmax > 4096 || chunk_cap > 0) return kNotApplicable;
+        if (size_t(nb) * nvmax > fit || nvmax > 3072 || chunk_cap > 0) return kNotApplicable;
         nv = nvmax;
         nchunks = 1;
     }
-    A.vg = std::min(GVG, nv);
-    if (size_t(ceil_div(nv, A.vg)) * nb > 65535) return kNotApplicable;  // grid.y
 
-    const size_t fixed = size_t(nv1) * GWARPS * sizeof(GEntry) + size_t(A.vg) * nv1 * GPL * 8 + size_t(nv1) * 8 +
-                         2 * GNSMAX * 8 + 8 + GNSMAX * 4;
-    const size_t stage = size_t(2) * A.sstride * EB;
-    A.ns = int(std::min<size_t>(GNSMAX, (227 * 1024 - std::min<size_t>(fixed, 227 * 1024)) / stage));
+    ZgatherArgs A{};
+    A.G = G;
+    A.vr = vr;
+    A.n_colblk = int(ceil_div(G.N_u0, kZCols));
+    A.NUc = NUc;
+    A.nv1 = nv1;
+    A.T = T;
+    A.err = err;
+    A.wait_limit = wait_limit();
+    // twelve consumer warps, four where twelve would leave SMs without a tile
+    for (A.nw = kZWarps;; A.nw = 4) {
+        A.pg = NV == 4 || A.nw == 4 ? 4 : 6;
+        A.rg = A.nw / A.pg;
+        A.planes = NV * A.pg;
+        A.rows = NK * A.rg;
+        A.n_plblk = int(ceil_div(G.numY, A.planes));
+        A.n_rowblk = int(ceil_div(G.numZ, A.rows));
+        const long long nt = (long long)nv * nb * A.n_plblk * A.n_rowblk * A.n_colblk;
+        if (nt > (1 << 30)) return kNotApplicable;
+        A.ntile = int(nt);
+        if (A.nw == 4 || A.ntile >= sm_count()) break;
+    }
+    if (A.n_rowblk > 65535) return kNotApplicable;  // k_gather_records grid.y
+    A.nrb = A.rows + 1 + shift_spread(A.planes - 1, step);
+    if (A.nrb > 250) return kNotApplicable;  // TMA box rows
+    A.sbytes = (A.nrb + kZSpread) * kZCols * EB;  // a multiple of 128
+    A.stage = (2 * A.sbytes + 2 * int(sizeof(GRec)) + 127) & ~127;
+    A.ns = std::min(kZStages, (227 * 1024 - int(sizeof(ZCtl))) / A.stage);
     if (A.ns < 2) return kNotApplicable;
-    const size_t smem = size_t(A.ns) * stage + fixed;
+    const size_t smem = size_t(A.ns) * A.stage + sizeof(ZCtl);
 
     GMaps<kMaxMembers> maps;
     std::memset(&maps, 0, sizeof(maps));
-    const uint64_t dims[4] = {uint64_t(G.N_u0), uint64_t(G.N_u1), uint64_t(G.N_v0), uint64_t(G.N_v1)};
-    const uint64_t strides[3] = {uint64_t(G.N_u0) * EB, uint64_t(G.N_u0) * G.N_u1 * EB,
-                                 uint64_t(G.N_u0) * G.N_u1 * G.N_v0 * EB};
-    const uint32_t box[4] = {uint32_t(GCOLS), uint32_t(brb), 1u, 1u};
-    for (int b = 0; b < nb; b++)
-        if (!encode_tensor_map(&maps.m[b], M0.in[b], 4, dims, strides, box, EB)) return kNotApplicable;
+    if (bulk) {
+        const uint64_t dims[4] = {uint64_t(G.N_u0), uint64_t(G.N_u1), uint64_t(G.N_v0), uint64_t(G.N_v1)};
+        const uint64_t strides[3] = {uint64_t(G.N_u0) * EB, uint64_t(G.N_u0) * G.N_u1 * EB,
+                                     uint64_t(G.N_u0) * G.N_u1 * G.N_v0 * EB};
+        const uint32_t box[4] = {uint32_t(kZCols), uint32_t(A.nrb), 1u, 1u};
+        for (int b = 0; b < nb; b++)
+            if (!encode_tensor_map(&maps.m[b], M0.in[b], 4, dims, strides, box, EB)) return kNotApplicable;
+    }
 
+    // B, then the table records, the lists and the counts
     float* B = nullptr;
     float* part = nullptr;
     const size_t nvox = size_t(G.numX) * G.numY * G.numZ;
-    if (scratch_alloc(reinterpret_cast<void**>(&B), per_view * nv * nb, st) != cudaSuccess ||
+    const size_t b_bytes = per_view * nv * nb;  // a multiple of 16
+    const size_t ntab = size_t(A.n_plblk) * A.n_rowblk;
+    const size_t t_bytes = ntab * nv1 * (sizeof(GRec) + sizeof(int2)) + (ntab + nchunks) * sizeof(int);
+    if (scratch_alloc(reinterpret_cast<void**>(&B), b_bytes + t_bytes, st) != cudaSuccess ||
         (nchunks > 1 && scratch_alloc(reinterpret_cast<void**>(&part), nvox * 4, st) != cudaSuccess)) {
         cudaGetLastError();  // out of memory is not sticky: the caller takes the single-pass kernel
         if (B) cudaFreeAsync(B, st);
         return kNotApplicable;
     }
+    A.rec = reinterpret_cast<GRec*>(reinterpret_cast<unsigned char*>(B) + b_bytes);
+    A.list = reinterpret_cast<int2*>(A.rec + ntab * nv1);
+    A.cnt = reinterpret_cast<int*>(A.list + ntab * nv1);
+    A.next = A.cnt + ntab;
+    A.nchunks = nchunks;
     const bool adj = mode == PETL_BP_ADJOINT;
-    // kernels compiled for one member where there is one
-    GMaps<1> map1;
-    map1.m[0] = maps.m[0];
-    auto kz1 = adj ? k_bwd_zgather<true, TG, 1> : k_bwd_zgather<false, TG, 1>;
-    auto kzm = adj ? k_bwd_zgather<true, TG, kMaxMembers> : k_bwd_zgather<false, TG, kMaxMembers>;
+    const dim3 rgrid(unsigned(A.n_plblk), unsigned(A.n_rowblk));
+    if (adj)
+        k_gather_records<true><<<rgrid, 256, 0, st>>>(A, NV, NK);
+    else
+        k_gather_records<false><<<rgrid, 256, 0, st>>>(A, NV, NK);
+    note_launch();
+    auto launch = [&](auto bulk_c, auto nv_c, auto nk_c, unsigned grid) {
+        constexpr bool BULK = decltype(bulk_c)::value;
+        constexpr int V = decltype(nv_c)::value, K = decltype(nk_c)::value;
+        const unsigned threads = 32u * unsigned(A.nw + 4);
+        cudaError_t r;
+        if (nb == 1) {  // kernels compiled for one member where there is one
+            GMaps<1> map1;
+            map1.m[0] = maps.m[0];
+            auto kz = adj ? k_bwd_zgather<true, TG, 1, BULK, V, K> : k_bwd_zgather<false, TG, 1, BULK, V, K>;
+            r = cudaFuncSetAttribute(kz, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+            if (r == cudaSuccess) kz<<<grid, threads, smem, st>>>(map1, B, A);
+        } else {
+            auto kz = adj ? k_bwd_zgather<true, TG, kMaxMembers, BULK, V, K>
+                          : k_bwd_zgather<false, TG, kMaxMembers, BULK, V, K>;
+            r = cudaFuncSetAttribute(kz, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+            if (r == cudaSuccess) kz<<<grid, threads, smem, st>>>(maps, B, A);
+        }
+        return r;
+    };
     auto kx = nb == 1 ? k_bwd_xgather<1> : k_bwd_xgather<kMaxMembers>;
-    cudaError_t e = nb == 1 ? cudaFuncSetAttribute(kz1, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))
-                            : cudaFuncSetAttribute(kzm, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    const unsigned ntile = unsigned(A.n_colblk) * unsigned(A.n_rowblk) * ceil_div(G.numY, GPL);
+    cudaError_t e = cudaGetLastError();
     for (int c = 0; c < nchunks && e == cudaSuccess; c++) {
         Members M = M0;
         const int vi0 = c * nv;
@@ -809,15 +872,22 @@ int backproject_split_m(const petl_geom& G, const Members& M0, int mode, int acc
         M.nvm = nvc;
         if (hook && hook->fn) hook->fn(hook->ctx, vi0, nvc);
         A.M = M;
-        A.gpm = int(ceil_div(nvc, A.vg));
-        if (nb == 1)
-            kz1<<<dim3(ntile, unsigned(A.gpm)), GNT, smem, st>>>(map1, B, A);
+        A.nslot = nvc * nb;
+        A.ntile = A.nslot * A.n_plblk * A.n_rowblk * A.n_colblk;
+        const unsigned grid = unsigned(std::min(A.ntile, sm_count()));
+        using std::integral_constant;
+        if (bulk)
+            e = NV == 4 ? launch(std::true_type{}, integral_constant<int, 4>{}, integral_constant<int, 12>{}, grid)
+                        : launch(std::true_type{}, integral_constant<int, 2>{}, integral_constant<int, 24>{}, grid);
         else
-            kzm<<<dim3(ntile, unsigned(A.gpm) * unsigned(nb)), GNT, smem, st>>>(maps, B, A);
+            e = NV == 4 ? launch(std::false_type{}, integral_constant<int, 4>{}, integral_constant<int, 12>{}, grid)
+                        : launch(std::false_type{}, integral_constant<int, 2>{}, integral_constant<int, 24>{}, grid);
+        if (e != cudaSuccess) break;
         note_launch();
-        XgatherArgs X{G, vr.iv0_step, A.NUc, c == 0, c == nchunks - 1, accumulate, scale, T, M, G.numY};
+        A.next++;
+        XgatherArgs X{G, vr.iv0_step, A.NUc, c == 0, c == nchunks - 1, accumulate, scale, T, M, adj};
         kx<<<dim3(ceil_div(G.numX, 256), ceil_div(G.numZ, XR), unsigned(G.numY) * unsigned(nb)), 256,
-                        size_t(nvc) * sizeof(Shift), st>>>(B, part, X);
+                        size_t(nvc) * sizeof(XView), st>>>(B, part, X);
         note_launch();
         e = cudaGetLastError();
     }
