@@ -47,6 +47,7 @@
 #include "projector.cuh"
 #include "storage.cuh"
 #include "tma.cuh"
+#include "ztaps.cuh"
 
 namespace petl {
 
@@ -282,6 +283,333 @@ __global__ void __launch_bounds__(GZT, 1) k_gz(const __grid_constant__ CUtensorM
     }
 }
 
+// ---------------------------------------------------------------------------
+// Unequal voxel height and u1 pitch on an axis-aligned planogram (psi = 0 and
+// 90: PET/X's 1.6 mm bins over 0.5 mm voxels).  The ray parameter of a plane is
+// the same for every column, so the edges of a ray's u1 bin cut the voxel
+// column at the same heights in every column: edge k of a slope lies at
+//   e_k = ((u1_0 + (iu1 - 1/2) T_u1) - t v1 - z_0) / T_z + 1/2,  iu1 = row0 + k
+// in voxels, and bin k sums X over [e_k, e_k+1): the voxel of its lower edge by
+// (1 - frac e_k), the whole voxels, the voxel of its upper edge by
+// frac e_k+1 (all times T_z / T_u1).
+//
+// CTA = one view x 16 slopes (one per warp) x 32 bins x 64 columns (two per
+// lane).  The voxel rows that the tile needs on a plane arrive by a tiled TMA
+// copy (no multicast) into a ring of three planes; lane k of a warp places edge
+// k (in double: the heights reach a hundred voxels, and their fractions are the
+// weights) and the warp reads the edges back as broadcasts.  Planes on which no
+// ray of the tile meets the volume are left out: with panels four times as
+// long as the field of view that is most of them.  Bound by shared-memory
+// loads (T_u1 / T_z + 1 rows per bin).  The general kernel recomputed both
+// footprints' weights per tap and read every tap from global memory: one
+// subset of 8 of PET/X's two planograms into 120x120x120 took it 27.2 ms.
+constexpr int UZS = 16;              // slopes per CTA, one per warp
+constexpr int UZR = 32;              // bins (rows) per CTA
+constexpr int UZC = 64;              // columns per CTA
+constexpr int UZT = 32 * UZS;        // threads per CTA
+constexpr int UZRMAX = 250;          // staged rows per plane at most (TMA box rows <= 256)
+
+struct UzArgs {
+    petl_geom G;
+    ViewRange vr;
+    int vi0;
+    int NPmax;
+    int n_colblk, n_rowblk;
+    int nrows;  // staged rows per plane
+    int ns;     // ring stages (one plane each)
+    int xd;     // driving planes of constant x (psi = 90), else of constant y
+    int* err;
+    unsigned wait_limit;
+};
+
+struct __align__(8) UEdge {
+    int row;  // staged row that holds the edge
+    float f;  // its fraction below the edge
+};
+
+// NI: whole voxels of a bin at most (floor of T_u1 / T_z), or -1 for any number.
+template <int NI>
+__global__ void __launch_bounds__(UZT, 1) k_uz(const __grid_constant__ CUtensorMap xmap, float* __restrict__ g,
+                                               const float* __restrict__ meas, const UzArgs A)
+{
+    extern __shared__ __align__(128) unsigned char usm[];
+    const petl_geom& G = A.G;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int t_ = blockIdx.x;
+    const int colblk = t_ % A.n_colblk;
+    t_ /= A.n_colblk;
+    const int rowblk = t_ % A.n_rowblk;
+    const int v1blk = t_ / A.n_rowblk;
+    const int vi = blockIdx.y;
+    const int iv0 = A.vr.iv0_first + (A.vi0 + vi) * A.vr.iv0_step;
+    const int col0 = colblk * UZC, row0 = rowblk * UZR;
+    const int v1c = A.vr.iv1_begin + v1blk * UZS, v1e = min(v1c + UZS, A.vr.iv1_end);
+    const int iv1 = v1c + warp;  // the warp's slope
+    const int nrows = A.nrows, ns = A.ns, NP = A.xd ? G.numX : G.numY, NA = A.xd ? G.numY : G.numX;
+
+    float* ring = reinterpret_cast<float*>(usm);  // [ns][nrows][64]
+    UEdge* edge = reinterpret_cast<UEdge*>(ring + size_t(ns) * nrows * UZC) + warp * (UZR + 1);
+    uint64_t* full = reinterpret_cast<uint64_t*>(reinterpret_cast<UEdge*>(ring + size_t(ns) * nrows * UZC) +
+                                                 UZS * (UZR + 1));
+    uint64_t* empty = full + GZNS;
+    int* s_wr = reinterpret_cast<int*>(empty + GZNS);  // [GZNS] first staged row of the slot's plane
+    int* s_round = s_wr + GZNS;                        // [GZNS] round of the copy last started in a slot
+    int* s_live = s_round + GZNS;                      // planes [s_live[0], s_live[1])
+    volatile int* s_abort = s_live + 2;
+    if (tid == 0) {
+        for (int k = 0; k < ns; k++) {
+            mbar_init(&full[k], 1);
+            mbar_init(&empty[k], UZS);
+            s_round[k] = -1;
+        }
+        *s_abort = 0;
+        fence_barrier_init();
+    }
+
+    // the ray parameter of plane p and the height of edge k of a slope there
+    const double Tz = double(G.T_z), Tu1 = double(G.T_u1), rho = Tu1 / Tz;
+    const double sign = A.xd ? -double(G.sin_psi) : double(G.cos_psi);  // r_p = +-1
+    const double s0 = A.xd ? double(G.x_0) : double(G.y_0);
+    auto plane_par = [&](int p) { return (s0 + p * double(G.T_x)) * sign; };
+    const double e0 = ((double(G.u1_0) + (row0 - 0.5) * Tu1) - double(G.z_0)) / Tz + 0.5;
+    auto slope = [&](int i) { return double(ffma(float(i), G.T_v1, G.v1_0)) / Tz; };
+    const double va = slope(v1c), vb = slope(v1e - 1);
+    auto first_row = [&](int p) {
+        const double t = plane_par(p);
+        return int(floor(e0 - fmax(t * va, t * vb))) - 1;
+    };
+    // planes whose staged rows meet the volume and on which a column of the
+    // tile does (a voxel of margin)
+    if (warp == 0) {
+        bool rows = false;
+        for (int i = lane; i < (v1e - v1c) * UZR; i += 32)
+            rows |= row0 + i % UZR < G.N_u1 && u1_visible(G, v1c + i / UZR, row0 + i % UZR);
+        bool cols = false;
+        for (int c = col0 + lane; c < min(col0 + UZC, G.N_u0); c += 32) cols |= u0_visible(G, iv0, c);
+        int lo = NP, hi = 0;
+        if (__any_sync(0xffffffffu, rows) && __any_sync(0xffffffffu, cols)) {
+            const double v0 = double(ffma(float(iv0), G.T_v0, G.v0_0));
+            const double a0 = A.xd ? double(G.y_0) : double(G.x_0), Tx = double(G.T_x);
+            const double half = 0.5 * (double(G.T_u0) + Tx) + Tx;
+            // in-plane position of a ray: u0 - t v0 (psi = 0), u0 - t v0 with
+            // y as the in-plane axis (psi = 90)
+            for (int p = lane; p < NP; p += 32) {
+                const double t = plane_par(p);
+                const double ua = double(G.u0_0) + col0 * double(G.T_u0), ub = ua + (UZC - 1) * double(G.T_u0);
+                const double off = -t * v0;
+                const bool in = ub + off + half > a0 - 0.5 * Tx && ua + off - half < a0 + (NA - 0.5) * Tx;
+                const int wr = first_row(p);
+                if (in && wr + nrows > 0 && wr < G.numZ) {
+                    lo = min(lo, p);
+                    hi = p + 1;
+                }
+            }
+        }
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        if (lane == 0) {
+            s_live[0] = min(lo, hi);
+            s_live[1] = hi;
+        }
+    }
+    __syncthreads();
+    const int pa = s_live[0], np = s_live[1] - s_live[0];
+
+    const uint32_t box_bytes = uint32_t(nrows) * UZC * 4u;
+    auto issue = [&](int i) {
+        const int slot = i % ns, round = i / ns;
+        if (round > 0 && !mbar_wait(&empty[slot], uint32_t((round - 1) & 1), A.err, A.wait_limit)) return false;
+        if (*s_abort) return false;
+        fence_proxy_async_smem();
+        const int wr = first_row(pa + i);
+        s_wr[slot] = wr;
+        mbar_arrive_expect_tx(&full[slot], box_bytes);
+        tma_load_3d(ring + size_t(slot) * nrows * UZC, &xmap, &full[slot], col0, wr, vi * A.NPmax + pa + i);
+        s_round[slot] = round;
+        return true;
+    };
+    if (tid == 0)
+        for (int i = 0; i < ns - 1 && i < np; i++) issue(i);
+    // the next plane this warp starts: the first i >= ns - 1 with i % 16 == warp
+    int my_next = warp + UZS * ((ns - 1 - warp + UZS - 1) / UZS);
+    if (my_next < ns - 1) my_next += UZS;
+
+    using shear::f2x;
+    f2x acc[UZR];
+#pragma unroll
+    for (int k = 0; k < UZR; k++) acc[k] = 0ull;
+    const double v1z = slope(min(iv1, A.vr.iv1_end - 1));
+    bool dead = false;
+    int slot = 0;
+    uint32_t phase = 0;
+    for (int i = 0; i < np; i++) {
+        if (i + ns - 1 == my_next) {
+            if (lane == 0 && !dead && my_next < np && !issue(my_next)) dead = true;
+            my_next += UZS;
+        }
+        if (!dead) dead = !mbar_wait(&full[slot], phase, A.err, A.wait_limit);
+        dead = __any_sync(0xffffffffu, dead);
+        if (dead) *s_abort = 1;  // before this warp releases the slot
+        if (!dead && iv1 < v1e) {
+            const double eb = e0 - plane_par(pa + i) * v1z - s_wr[slot];
+            bool bad = false;
+            for (int k = lane; k <= UZR; k += 32) {
+                const double e = fma(double(k), rho, eb), fl = floor(e);
+                const int row = int(fl);
+                bad |= row < 0 || row >= nrows;
+                edge[k] = UEdge{min(max(row, 0), nrows - 1), float(e - fl)};
+            }
+            if (bad) atomicOr(A.err, kErrLayout);  // outside the staged rows: the host bound failed
+            __syncwarp();
+            const f2x* B = reinterpret_cast<const f2x*>(ring + size_t(slot) * nrows * UZC) + lane;
+            UEdge a = edge[0];
+            f2x xa = B[a.row * (UZC / 2)];
+#pragma unroll
+            for (int k = 0; k < UZR; k++) {
+                const UEdge b = edge[k + 1];
+                const int n = b.row - a.row;
+                acc[k] = shear::f2_fma(shear::f2_dup(n > 0 ? 1.0f - a.f : b.f - a.f), xa, acc[k]);
+                if constexpr (NI >= 0) {
+#pragma unroll
+                    for (int j = 1; j <= NI; j++)
+                        if (j < n) acc[k] = shear::f2_add(acc[k], B[(a.row + j) * (UZC / 2)]);
+                } else {
+                    for (int j = 1; j < n; j++) acc[k] = shear::f2_add(acc[k], B[(a.row + j) * (UZC / 2)]);
+                }
+                xa = B[b.row * (UZC / 2)];
+                if (n > 0 && b.f > 0.0f) acc[k] = shear::f2_fma(shear::f2_dup(b.f), xa, acc[k]);
+                a = b;
+            }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[slot]);
+        if (++slot == ns) {
+            slot = 0;
+            phase ^= 1u;
+        }
+    }
+    if (__syncthreads_or(dead)) {
+        // a wait gave up: drain the copies still in flight, write nothing
+        if (tid == 0)
+            for (int k = 0; k < ns; k++)
+                if (s_round[k] >= 0) mbar_wait(&full[k], uint32_t(s_round[k] & 1), nullptr);
+        return;
+    }
+
+    // epilogue: scale, ray masks, optional MLEM ratio
+    const int iu0 = col0 + 2 * lane;
+    if (iv1 >= v1e || iu0 >= G.N_u0) return;
+    const RayGeom rr = ray_geom(G, iv1, iv0, 0, iu0);
+    const float c = float(Tz / Tu1);
+    const bool two = iu0 + 1 < G.N_u0;
+    const bool ok0 = u0_visible(G, iv0, iu0), ok1 = two && u0_visible(G, iv0, iu0 + 1);
+#pragma unroll
+    for (int k = 0; k < UZR; k++) {
+        const int iu1 = row0 + k;
+        if (iu1 >= G.N_u1) break;
+        const bool rv = u1_visible(G, iv1, iu1);
+        const float2 v = shear::f2_unpack(acc[k]);
+        float2 o = make_float2(rv && ok0 ? fmul(fmul(fmul(v.x, c), rr.l_phi), rr.rs) : 0.0f,
+                               rv && ok1 ? fmul(fmul(fmul(v.y, c), rr.l_phi), rr.rs) : 0.0f);
+        const size_t at = ((size_t(iv1) * G.N_v0 + iv0) * G.N_u1 + iu1) * G.N_u0 + iu0;
+        if (meas) o = make_float2(ratio_rule(__ldg(meas + at), o.x), two ? ratio_rule(__ldg(meas + at + 1), o.y) : 0.0f);
+        g[at] = o.x;
+        if (two) g[at + 1] = o.y;
+    }
+}
+
+bool aligned_90(const petl_geom& G) { return std::fabs(G.cos_psi) < 1e-6f && G.sin_psi == 1.0f; }
+
+// The split forward for unequal voxel height and u1 pitch; kNotApplicable (-2)
+// off the axes and where the staged rows would not fit.
+int project_usplit(const petl_geom& G, const float* f, float* g, const ViewRange& vr, const float* meas,
+                   cudaStream_t st)
+{
+    constexpr int kNotApplicable = -2;
+    const int n_v0 = vr.n_v0(G.N_v0), nv1 = vr.iv1_end - vr.iv1_begin;
+    const bool xd = aligned_90(G);
+    if (!xd && !(G.cos_psi == 1.0f && G.sin_psi == 0.0f)) return kNotApplicable;
+    for (int k = 0; k < n_v0; k++)
+        if (host_view(G, vr.iv0_first + k * vr.iv0_step).xd != xd) return kNotApplicable;
+    const int NP = xd ? G.numX : G.numY, NA = xd ? G.numY : G.numX;
+    const double rho = double(G.T_u1) / double(G.T_z);
+    const double first = xd ? double(G.x_0) : double(G.y_0);
+    const double tmax = std::max(std::fabs(first), std::fabs(first + (NP - 1) * double(G.T_x)));
+    const double spread = (UZS - 1) * std::fabs(double(G.T_v1)) * tmax / double(G.T_z);
+    // the rows of 32 bins, the slopes' spread and a row on either side
+    const double need = UZR * rho + spread * (1.0 + 1e-6) + 4.0;
+    if (!(need <= UZRMAX)) return kNotApplicable;
+    const int nrows = int(std::ceil(need));
+    int* err = device_error_ptr();
+    if (!err) return kNotApplicable;
+    const int NUc = (G.N_u0 + 3) & ~3;
+    const size_t per_view = size_t(NP) * G.numZ * NUc * 4;
+    int nv = int(std::max<size_t>(1, std::min<size_t>(size_t(n_v0), gsplit_scratch_budget() / per_view)));
+    nv = std::min(nv, 65535);
+    if (NP > 65535) return kNotApplicable;
+    const int nchunks = (n_v0 + nv - 1) / nv;
+    nv = (n_v0 + nchunks - 1) / nchunks;
+    const size_t stage = size_t(nrows) * UZC * 4;
+    UzArgs Z{};
+    Z.G = G;
+    Z.vr = vr;
+    Z.NPmax = NP;
+    Z.n_colblk = int(ceil_div(G.N_u0, UZC));
+    Z.n_rowblk = int(ceil_div(G.N_u1, UZR));
+    Z.nrows = nrows;
+    Z.ns = int(std::min<size_t>(GZNS, (200 * 1024) / stage));
+    Z.xd = xd;
+    Z.err = err;
+    Z.wait_limit = wait_limit();
+    if (Z.ns < 2) return kNotApplicable;
+    const size_t smem = size_t(Z.ns) * stage + size_t(UZS) * (UZR + 1) * sizeof(UEdge) + GZNS * 16 + GZNS * 8 + 16;
+    float* X = nullptr;
+    float* fT = nullptr;
+    if (scratch_alloc(reinterpret_cast<void**>(&X), per_view * nv, st) != cudaSuccess ||
+        (xd && scratch_alloc(reinterpret_cast<void**>(&fT), size_t(G.numX) * G.numY * G.numZ * 4, st) != cudaSuccess)) {
+        cudaGetLastError();
+        if (X) cudaFreeAsync(X, st);
+        return kNotApplicable;
+    }
+    CUtensorMap map;
+    const uint64_t dims[3] = {uint64_t(NUc), uint64_t(G.numZ), uint64_t(NP) * uint64_t(nv)};
+    const uint64_t strides[2] = {uint64_t(NUc) * 4, uint64_t(NUc) * G.numZ * 4};
+    const uint32_t box[3] = {uint32_t(UZC), uint32_t(nrows), 1u};
+    if (!encode_tensor_map(&map, X, 3, dims, strides, box, 4)) {
+        cudaFreeAsync(X, st);
+        if (fT) cudaFreeAsync(fT, st);
+        return kNotApplicable;
+    }
+    if (xd) {
+        k_transpose_xy<<<dim3(ceil_div(G.numX, 32), ceil_div(G.numY, 32), unsigned(G.numZ)), dim3(32, 8), 0, st>>>(
+            f, fT, G.numX, G.numY);
+        note_launch();
+    }
+    const size_t xsmem = size_t(GXZ) * NA * 4;
+    const int ni = int(std::floor(rho));
+    auto kz = ni == 0 ? k_uz<0> : ni == 1 ? k_uz<1> : ni == 2 ? k_uz<2> : ni == 3 ? k_uz<3> : k_uz<-1>;
+    cudaError_t e = cudaFuncSetAttribute(k_gx, cudaFuncAttributeMaxDynamicSharedMemorySize, int(xsmem));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kz, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    for (int c = 0; c < nchunks && e == cudaSuccess; c++) {
+        const int vi0 = c * nv, nvc = std::min(nv, n_v0 - vi0);
+        const GxArgs XA{G, vr, vi0, NP, NUc};
+        k_gx<<<dim3(ceil_div(G.numZ, GXZ), unsigned(NP), unsigned(nvc)), 256, xsmem, st>>>(f, fT, X, XA);
+        note_launch();
+        Z.vi0 = vi0;
+        kz<<<dim3(unsigned(Z.n_colblk) * unsigned(Z.n_rowblk) * ceil_div(nv1, UZS), unsigned(nvc)), UZT, smem, st>>>(
+            map, g, meas, Z);
+        note_launch();
+        e = cudaGetLastError();
+    }
+    cudaFreeAsync(X, st);
+    if (fT) cudaFreeAsync(fT, st);
+    if (e != cudaSuccess) {
+        set_error(std::string("project_usplit: ") + cudaGetErrorString(e));
+        return int(e);
+    }
+    return 0;
+}
+
 }  // namespace
 
 
@@ -312,7 +640,8 @@ int project_gsplit(const petl_geom& G, const float* f, float* g, const ViewRange
     const int n_v0 = vr.n_v0(G.N_v0);
     const int nv1 = vr.iv1_end - vr.iv1_begin;
     if (n_v0 <= 0 || nv1 <= 0) return 0;
-    if (G.T_z != G.T_u1 || G.N_u0 > 4096 || G.numX > 4096 || G.numY > 4096) return kNotApplicable;
+    if (G.N_u0 > 4096 || G.numX > 4096 || G.numY > 4096) return kNotApplicable;
+    if (G.T_z != G.T_u1) return project_usplit(G, f, g, vr, meas, st);
     // staged rows per plane: the CTA's rows + the range of floor(-c0) over a
     // tile's 32 columns and its slopes + margins.  -c0 = (u1_0 - z_0 + t v1)
     // / T_u1 with t = (coordinate of the plane - u0 pscale) * inv: bounded

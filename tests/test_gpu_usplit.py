@@ -1,0 +1,58 @@
+"""The split forward for unequal voxel height and u1 pitch on an axis-aligned
+planogram against the FP64 oracle and the general kernels: bins taller and
+lower than voxels (0 to 3 whole voxels in a bin, the unrolled forms, and
+more), psi = 0 and 90, ragged and off-centre volumes, rays that miss the
+volume on most planes, a volume wider than the panels, view subsets, slope
+ranges and the MLEM ratio."""
+import numpy as np
+import pytest
+
+import oracle as O
+from conftest import rel_l2
+from helpers import ellipsoids
+
+pytestmark = pytest.mark.gpu
+
+CASES = {
+    # psi, D, L, H, T, v_m0, v_m1 ; volume (x, y, z, width, height, offsets) ; path (3 split, 0 general)
+    "petx0": ((0.0, 101.0, 120.0, 60.0, 1.6, 0.99, 0.55), (40, 36, 30, 0.5, 0.5), 3),
+    "petx90": ((90.0, 120.0, 80.0, 60.0, 1.6, 0.7, 0.45), (36, 41, 33, 0.5, 0.5, 2.0, -1.0, 3.0), 3),
+    "low_bins": ((0.0, 100.0, 50.0, 30.0, 1.0, 0.5, 0.25), (30, 40, 12, 2.0, 2.7), 3),
+    "one_whole": ((90.0, 100.0, 75.0, 27.0, 1.5, 0.45, 0.2), (52, 60, 18, 1.5, 1.1, 3.0, -4.5, 1.5), 3),
+    "two_whole": ((0.0, 100.0, 40.0, 44.0, 2.0, 0.4, 0.2), (50, 20, 61, 0.9, 0.75), 3),
+    "four_whole": ((0.0, 100.0, 40.0, 44.0, 2.0, 0.4, 0.2), (30, 20, 90, 1.0, 0.45), 3),
+    "too_many_rows": ((0.0, 100.0, 40.0, 44.0, 4.0, 0.4, 0.2), (30, 20, 90, 1.0, 0.45), 0),
+}
+
+
+@pytest.mark.parametrize("name", list(CASES))
+def test_unequal_pitch_forward(cuda, name):
+    import torch
+    from petl_b200 import Geometry, lib, ops
+    args, vol, path = CASES[name]
+    G, Go = Geometry(*args, volume=vol), O.make_geom(*args, vol)
+    rng = np.random.default_rng(2)
+    f = ellipsoids(G.vol_shape, (vol[3], vol[4]), rng, 6) + 0.1 * rng.random(G.vol_shape).astype(np.float32)
+    ft = torch.from_numpy(f).to(cuda)
+    a = ops.project(G, ft)
+    assert lib().petl_last_projector_path() == path
+    assert rel_l2(a.cpu().numpy(), O.project(Go, f)[0]) < 1e-5
+    meas = torch.rand(G.shape, device=cuda)
+    sub, v1 = (1, 3), (2, G.shape[0] - 1)
+    out = []
+    for d in (0, 1):
+        try:
+            lib().petl_set_dispatch(d)
+            out.append([ops.project(G, ft, torch.full(G.shape, -7.0, device=cuda), subset=sub, v1_range=v1),
+                        ops.project_ratio(G, ft, meas, torch.full(G.shape, -7.0, device=cuda), subset=sub, v1_range=v1)])
+        finally:
+            lib().petl_set_dispatch(0)
+    torch.cuda.synchronize()
+    assert lib().petl_device_error_flag() == 0
+    for x, y in zip(*out):
+        assert torch.equal(x == -7.0, y == -7.0)
+    assert torch.equal(out[0][0] == 0, out[1][0] == 0)  # rays that meet no voxel stay exactly zero
+    assert rel_l2(out[0][0].cpu().numpy(), out[1][0].cpu().numpy()) < 1e-5
+    # the ratio where the ray meets more than the rim of a voxel
+    ok = out[1][0] > 0.05 * out[1][0].max()
+    assert rel_l2(out[0][1][ok].cpu().numpy(), out[1][1][ok].cpu().numpy()) < 1e-5
