@@ -53,7 +53,11 @@ namespace petl {
 
 namespace {
 
-constexpr int GXZ = 8;        // volume rows per k_gx block
+// Volume rows per k_gx block: a column's taps are evaluated once per block, and
+// with 8 rows their evaluation bounded the pass (psi = 30, 256x256x128: 3.4 ms
+// for 4.3 GB of scratch); 32 rows of axes up to 512 voxels (64 KB of shared
+// memory), 8 of longer ones.
+constexpr int GXZ = 32, GXZ_LONG = 8, GXZ_AXIS = 512;
 constexpr int GZS = 16;       // slopes per k_gz CTA (2 per warp), main shape
 constexpr int GZR = 64;       // rows per k_gz CTA (32 per warp), main shape
 constexpr int GZS_T = 8;      // slopes per CTA of the tail shape (a last slope block of at most 8)
@@ -87,26 +91,41 @@ struct GzArgs {
     unsigned wait_limit;  // bound of the waits on staged data (wait_limit(): kWaitLimit or 0)
 };
 
+// First and last of n bins that a warp-wide test holds for, (1 << 30, -1) if none.
+template <class F>
+__device__ __forceinline__ int2 visible_range(int n, int lane, F test)
+{
+    int lo = 1 << 30, hi = -1;
+    for (int i = lane; i < n; i += 32)
+        if (test(i)) {
+            lo = min(lo, i);
+            hi = i;
+        }
+    return make_int2(__reduce_min_sync(0xffffffffu, lo), __reduce_max_sync(0xffffffffu, hi));
+}
+
 __device__ __forceinline__ bool view_xdriven(const petl_geom& G, int iv0)
 {
     return ray_geom(G, 0, iv0, 0, 0).xdriven;
 }
 
-// X[vi][p][z][u0] for 8 rows z of plane p of one view.  Grid (ceil(NZ / 8),
-// NPmax, views of the chunk); dynamic shared memory 8 rows of the longest
-// in-plane axis.
+// X[vi][p][z][u0] for ZB rows z of plane p of one view; columns whose rays are
+// all masked are left out.  The taps of a column are evaluated once for all
+// rows of the block.  Grid (ceil(NZ / ZB), NPmax, views of the chunk); dynamic
+// shared memory ZB rows of the longest in-plane axis.
+template <int ZB>
 __global__ void __launch_bounds__(256) k_gx(const float* __restrict__ f, const float* __restrict__ fT,
                                            float* __restrict__ X, const GxArgs A)
 {
     extern __shared__ float rowbuf[];
     const petl_geom& G = A.G;
-    const int z0 = blockIdx.x * GXZ, p = blockIdx.y, vi = blockIdx.z;
+    const int z0 = blockIdx.x * ZB, p = blockIdx.y, vi = blockIdx.z;
     const int iv0 = A.vr.iv0_first + (A.vi0 + vi) * A.vr.iv0_step;
     const bool xd = view_xdriven(G, iv0);
     const int NP = xd ? G.numX : G.numY, NA = xd ? G.numY : G.numX;
     if (p >= NP) return;
     const float* __restrict__ src = xd ? fT : f;  // [z][p][a]
-    const int nz = min(GXZ, G.numZ - z0);
+    const int nz = min(ZB, G.numZ - z0);
     for (int e = threadIdx.x; e < nz * NA; e += blockDim.x) {
         const int r = e / NA, a = e - r * NA;
         rowbuf[r * NA + a] = src[(size_t(z0 + r) * NP + p) * NA + a];
@@ -114,18 +133,21 @@ __global__ void __launch_bounds__(256) k_gx(const float* __restrict__ f, const f
     __syncthreads();
     float* Xv = X + (size_t(vi) * A.NPmax + p) * G.numZ * A.NUc;
     for (int iu0 = threadIdx.x; iu0 < G.N_u0; iu0 += blockDim.x) {
+        if (!u0_visible(G, iv0, iu0)) continue;
         const RayGeom r = ray_geom(G, 0, iv0, 0, iu0);
         const PlaneTaps pt = xd ? plane_taps_x(G, r, p) : plane_taps_y(G, r, p);
-        float acc[GXZ];
+        float acc[ZB];
 #pragma unroll
-        for (int k = 0; k < GXZ; k++) acc[k] = 0.0f;
+        for (int k = 0; k < ZB; k++) acc[k] = 0.0f;
         for (int a = pt.a_min; a <= pt.a_max; a++) {
             const float w0 = xd ? tap_w0_x(G, r, pt.t, a, iu0) : tap_w0_y(G, r, pt.t, a, iu0);
             if (!(w0 > 0.0f)) continue;
 #pragma unroll
-            for (int k = 0; k < GXZ; k++) acc[k] = fmaf(w0, rowbuf[k * NA + a], acc[k]);
+            for (int k = 0; k < ZB; k++) acc[k] = fmaf(w0, rowbuf[k * NA + a], acc[k]);
         }
-        for (int k = 0; k < nz; k++) Xv[size_t(z0 + k) * A.NUc + iu0] = acc[k];
+#pragma unroll
+        for (int k = 0; k < ZB; k++)
+            if (k < nz) Xv[size_t(z0 + k) * A.NUc + iu0] = acc[k];
     }
 }
 
@@ -150,10 +172,23 @@ __global__ void __launch_bounds__(GZT, 1) k_gz(const __grid_constant__ CUtensorM
     const int v1blk = t_ / A.n_rowblk;
     const int vi = blockIdx.y;
     const int iv0 = A.vr.iv0_first + (A.vi0 + vi) * A.vr.iv0_step;
-    const int col0 = colblk * GZC, iu0 = col0 + lane;
-    const int row0c = rowblk * RZ, row0 = row0c + rg * GRW;
     const int v1c = A.vr.iv1_begin + v1blk * SZ;           // first slope of the CTA
     const int v1c_last = min(v1c + SZ, A.vr.iv1_end) - 1;  // last slope of the CTA
+    // tiles start at the first visible row of the CTA's slopes and the first
+    // visible column of the view; the tiles at the edge write the zeros of
+    // the masked rays around them
+    const int2 cvis = visible_range(G.N_u0, lane, [&](int c) { return u0_visible(G, iv0, c); });
+    int2 rvis = make_int2(1 << 30, -1);
+    for (int v = v1c; v <= v1c_last; v++) {
+        const int2 x = visible_range(G.N_u1, lane, [&](int u) { return u1_visible(G, v, u); });
+        rvis = make_int2(min(rvis.x, x.x), max(rvis.y, x.y));
+    }
+    const bool any = cvis.x <= cvis.y && rvis.x <= rvis.y;
+    const int clo = any ? cvis.x & ~3 : 0, rlo = any ? rvis.x : 0;
+    const int ncol = any ? (cvis.y - clo) / GZC + 1 : 1, nrow = any ? (rvis.y - rlo) / RZ + 1 : 1;
+    if (colblk >= ncol || rowblk >= nrow) return;
+    const int col0 = clo + colblk * GZC, iu0 = col0 + lane;
+    const int row0c = rlo + rowblk * RZ, row0 = row0c + rg * GRW;
     const int v1w = v1c + q * GJS;                          // first slope of the warp
     const int nrows = A.nrows, ns = A.ns;
     const float Tu1_inv = __frcp_rn(G.T_u1);
@@ -171,6 +206,7 @@ __global__ void __launch_bounds__(GZT, 1) k_gz(const __grid_constant__ CUtensorM
     int* s_wr = reinterpret_cast<int*>(empty + GZNS);  // [GZNS] first staged row of the slot's plane
     int* s_round = s_wr + GZNS;                        // [GZNS] round of the copy last started in a slot
     volatile int* s_abort = s_round + GZNS;
+    int* s_live = const_cast<int*>(s_abort) + 1;       // planes [s_live[0], s_live[1])
     if (tid == 0) {
         for (int k = 0; k < ns; k++) {
             mbar_init(&full[k], 1);
@@ -180,7 +216,6 @@ __global__ void __launch_bounds__(GZT, 1) k_gz(const __grid_constant__ CUtensorM
         *s_abort = 0;
         fence_barrier_init();
     }
-    __syncthreads();
 
     // first staged row of plane p: the smallest shift at the tile's corners
     // (monotone in t and in v1), less one row of margin
@@ -193,9 +228,44 @@ __global__ void __launch_bounds__(GZT, 1) k_gz(const __grid_constant__ CUtensorM
         const float m = fminf(fminf(fmaf(-ta, v1lo, K), fmaf(-ta, v1hi, K)), fminf(fmaf(-tb, v1lo, K), fmaf(-tb, v1hi, K)));
         return row0c + int(floorf(m)) - 1;
     };
+    // planes on which a ray of the tile meets the volume (the tile's rays lie
+    // between its first and last column's, and its staged rows; a voxel of
+    // margin)
+    if (warp == 0) {
+        const RayGeom ra = ray_geom(G, 0, iv0, 0, col0);
+        const RayGeom rb = ray_geom(G, 0, iv0, 0, min(col0 + GZC - 1, G.N_u0 - 1));
+        const int NA = r.xdriven ? G.numY : G.numX;
+        const float a0 = r.xdriven ? G.y_0 : G.x_0, half = ra.width + 1.5f * G.T_x;
+        int lo = NP, hi = 0;
+        if (any)
+            for (int p = lane; p < NP; p += 32) {
+                const float ta = plane_t(G, ra, p), tb = plane_t(G, rb, p);
+                const float pa = r.xdriven ? ffma(ta, ra.ry, ra.py) : ffma(ta, ra.rx, ra.px);
+                const float pb = r.xdriven ? ffma(tb, rb.ry, rb.py) : ffma(tb, rb.rx, rb.px);
+                const int wr = first_row(p);
+                if (fmaxf(pa, pb) + half > a0 - 0.5f * G.T_x && fminf(pa, pb) - half < a0 + (NA - 0.5f) * G.T_x &&
+                    wr + nrows > 0 && wr < G.numZ) {
+                    lo = min(lo, p);
+                    hi = p + 1;
+                }
+            }
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        if (lane == 0) {
+            s_live[0] = min(lo, hi);
+            s_live[1] = hi;
+        }
+    }
+    __syncthreads();
+    const int pl0 = s_live[0], npl = s_live[1] - s_live[0];
+    // slopes and rows of this warp with a visible ray
+    bool have = false;
+    for (int v = v1w; v < min(v1w + GJS, v1c_last + 1); v++)
+        have |= __any_sync(0xffffffffu, row0 + lane < G.N_u1 && lane < GRW && u1_visible(G, v, row0 + lane));
+
     const uint32_t box_bytes = uint32_t(nrows) * GZC * 4u;
-    auto issue = [&](int p) {
-        const int slot = p % ns, round = p / ns;
+    auto issue = [&](int i) {
+        const int p = pl0 + i, slot = i % ns, round = i / ns;
         if (round > 0 && !mbar_wait(&empty[slot], uint32_t((round - 1) & 1), A.err, A.wait_limit)) return false;
         if (*s_abort) return false;
         fence_proxy_async_smem();
@@ -207,8 +277,8 @@ __global__ void __launch_bounds__(GZT, 1) k_gz(const __grid_constant__ CUtensorM
         return true;
     };
     if (tid == 0)
-        for (int p = 0; p < ns - 1 && p < NP; p++) issue(p);
-    // the next plane this warp starts: the first p >= ns - 1 with p % 16 == warp
+        for (int i = 0; i < ns - 1 && i < npl; i++) issue(i);
+    // the next plane this warp starts: the first i >= ns - 1 with i % 16 == warp
     constexpr int NW = GZT / 32;
     int my_next = warp + NW * ((ns - 1 - warp + NW - 1) / NW);
     if (my_next < ns - 1) my_next += NW;
@@ -222,15 +292,15 @@ __global__ void __launch_bounds__(GZT, 1) k_gz(const __grid_constant__ CUtensorM
     bool dead = false;
     int slot = 0;
     uint32_t phase = 0;
-    for (int p = 0; p < NP; p++) {
-        if (p + ns - 1 == my_next) {
-            if (lane == 0 && !dead && my_next < NP && !issue(my_next)) dead = true;
+    for (int i = 0; i < npl; i++) {
+        if (i + ns - 1 == my_next) {
+            if (lane == 0 && !dead && my_next < npl && !issue(my_next)) dead = true;
             my_next += NW;
         }
         if (!dead) dead = !mbar_wait(&full[slot], phase, A.err, A.wait_limit);
         if (dead) *s_abort = 1;  // before this warp releases the slot
-        if (!dead) {
-            const float tt = plane_t(G, r, p);
+        if (!dead && have) {
+            const float tt = plane_t(G, r, pl0 + i);
             const float* B = ring + size_t(slot) * nrows * GZC + lane;
             const int wr = s_wr[slot];
 #pragma unroll
@@ -266,20 +336,34 @@ __global__ void __launch_bounds__(GZT, 1) k_gz(const __grid_constant__ CUtensorM
     }
 
     // epilogue: scale, ray masks, optional MLEM ratio
-    if (iu0 >= G.N_u0) return;
+    const bool ok0 = iu0 < G.N_u0 && u0_visible(G, iv0, iu0);
+    const int cz0 = colblk == 0 ? 0 : col0, cz1 = colblk == ncol - 1 ? G.N_u0 : min(col0 + GZC, G.N_u0);
+    const int row1 = min(row0 + GRW, G.N_u1);
+    const int rz0 = rowblk == 0 && rg == 0 ? 0 : row0;
+    const int rz1 = rowblk == nrow - 1 && rg == GZT / 32 / NQ - 1 ? G.N_u1 : row1;
 #pragma unroll
     for (int j = 0; j < GJS; j++) {
         const int iv1 = v1w + j;
-        if (iv1 >= A.vr.iv1_end) continue;
+        if (iv1 > v1c_last) continue;
+        const RayGeom rr = ray_geom(G, iv1, iv0, 0, min(iu0, G.N_u0 - 1));
+        const size_t o0 = (size_t(iv1) * G.N_v0 + iv0) * G.N_u1 * G.N_u0;
+        if (iu0 < G.N_u0) {
 #pragma unroll
-        for (int k = 0; k < GRW; k++) {
-            const int iu1 = row0 + k;
-            if (iu1 >= G.N_u1) continue;
-            const RayGeom rr = ray_geom(G, iv1, iv0, iu1, iu0);
-            const float val = ray_visible(G, iv1, iv0, iu1, iu0) ? fmul(fmul(acc[j][k], rr.l_phi), rr.rs) : 0.0f;
-            const size_t o = ((size_t(iv1) * G.N_v0 + iv0) * G.N_u1 + iu1) * G.N_u0 + iu0;
-            g[o] = meas ? ratio_rule(__ldg(&meas[o]), val) : val;
+            for (int k = 0; k < GRW; k++) {
+                if (row0 + k >= G.N_u1) break;
+                const float val = ok0 && u1_visible(G, iv1, row0 + k) ? fmul(fmul(acc[j][k], rr.l_phi), rr.rs) : 0.0f;
+                const size_t o = o0 + size_t(row0 + k) * G.N_u0 + iu0;
+                g[o] = meas ? ratio_rule(__ldg(&meas[o]), val) : val;
+            }
         }
+        if (cz0 < col0 || cz1 > col0 + GZC || rz0 < row0 || rz1 > row1)
+#pragma unroll 1
+            for (int u = rz0; u < rz1; u++) {
+                const bool inside = u >= row0 && u < row1;
+#pragma unroll 1
+                for (int c = cz0 + lane; c < cz1; c += 32)
+                    if (!inside || c < col0 || c >= col0 + GZC) g[o0 + size_t(u) * G.N_u0 + c] = 0.0f;
+            }
     }
 }
 
@@ -585,15 +669,17 @@ int project_usplit(const petl_geom& G, const float* f, float* g, const ViewRange
             f, fT, G.numX, G.numY);
         note_launch();
     }
-    const size_t xsmem = size_t(GXZ) * NA * 4;
+    const int xzb = NA <= GXZ_AXIS ? GXZ : GXZ_LONG;
+    auto kx = xzb == GXZ ? k_gx<GXZ> : k_gx<GXZ_LONG>;
+    const size_t xsmem = size_t(xzb) * NA * 4;
     const int ni = int(std::floor(rho));
     auto kz = ni == 0 ? k_uz<0> : ni == 1 ? k_uz<1> : ni == 2 ? k_uz<2> : ni == 3 ? k_uz<3> : k_uz<-1>;
-    cudaError_t e = cudaFuncSetAttribute(k_gx, cudaFuncAttributeMaxDynamicSharedMemorySize, int(xsmem));
+    cudaError_t e = cudaFuncSetAttribute(kx, cudaFuncAttributeMaxDynamicSharedMemorySize, int(xsmem));
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kz, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     for (int c = 0; c < nchunks && e == cudaSuccess; c++) {
         const int vi0 = c * nv, nvc = std::min(nv, n_v0 - vi0);
         const GxArgs XA{G, vr, vi0, NP, NUc};
-        k_gx<<<dim3(ceil_div(G.numZ, GXZ), unsigned(NP), unsigned(nvc)), 256, xsmem, st>>>(f, fT, X, XA);
+        kx<<<dim3(ceil_div(G.numZ, xzb), unsigned(NP), unsigned(nvc)), 256, xsmem, st>>>(f, fT, X, XA);
         note_launch();
         Z.vi0 = vi0;
         kz<<<dim3(unsigned(Z.n_colblk) * unsigned(Z.n_rowblk) * ceil_div(nv1, UZS), unsigned(nvc)), UZT, smem, st>>>(
@@ -696,8 +782,10 @@ int project_gsplit(const petl_geom& G, const float* f, float* g, const ViewRange
         note_launch();
     }
     const int NAmax = any_xd ? std::max(G.numX, G.numY) : G.numX;
-    const size_t xsmem = size_t(GXZ) * NAmax * 4;
-    e = cudaFuncSetAttribute(k_gx, cudaFuncAttributeMaxDynamicSharedMemorySize, int(xsmem));
+    const int xzb = NAmax <= GXZ_AXIS ? GXZ : GXZ_LONG;
+    auto kx = xzb == GXZ ? k_gx<GXZ> : k_gx<GXZ_LONG>;
+    const size_t xsmem = size_t(xzb) * NAmax * 4;
+    e = cudaFuncSetAttribute(kx, cudaFuncAttributeMaxDynamicSharedMemorySize, int(xsmem));
     // one z launch shape: its argument block, tensor map (boxes of 32
     // columns x its staged rows; TMA, no multicast; rows outside read zero)
     // and shared memory
@@ -711,7 +799,7 @@ int project_gsplit(const petl_geom& G, const float* f, float* g, const ViewRange
         const size_t stage = size_t(staged) * GZC * 4;
         const int ns = int(std::min<size_t>(GZNS, (200 * 1024) / stage));
         if (ns < 2) return cudaErrorInvalidValue;
-        L.smem = size_t(ns) * stage + GZNS * 16 + GZNS * 8 + 16;
+        L.smem = size_t(ns) * stage + GZNS * 16 + GZNS * 8 + 16;  // ring, barriers, slot words, abort and live planes
         L.Z = GzArgs{};
         L.Z.G = G;
         L.Z.vr = vr;
@@ -741,7 +829,7 @@ int project_gsplit(const petl_geom& G, const float* f, float* g, const ViewRange
     for (int c = 0; c < nchunks && e == cudaSuccess; c++) {
         const int vi0 = c * nv, nvc = std::min(nv, n_v0 - vi0);
         const GxArgs XA{G, vr, vi0, NPmax, NUc};
-        k_gx<<<dim3(ceil_div(G.numZ, GXZ), unsigned(NPmax), unsigned(nvc)), 256, xsmem, st>>>(f, fT, X, XA);
+        kx<<<dim3(ceil_div(G.numZ, xzb), unsigned(NPmax), unsigned(nvc)), 256, xsmem, st>>>(f, fT, X, XA);
         note_launch();
         if (nv1_main > 0) {
             zm.Z.vi0 = vi0;
