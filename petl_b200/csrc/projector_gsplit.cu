@@ -74,6 +74,7 @@ struct GxArgs {
     petl_geom G;
     ViewRange vr;
     int vi0;    // first view of the chunk (index in vr)
+    int nvc;    // views of the chunk
     int NPmax;  // planes per view slot of the scratch
     int NUc;    // scratch row pitch
 };
@@ -109,45 +110,57 @@ __device__ __forceinline__ bool view_xdriven(const petl_geom& G, int iv0)
     return ray_geom(G, 0, iv0, 0, 0).xdriven;
 }
 
-// X[vi][p][z][u0] for ZB rows z of plane p of one view; columns whose rays are
-// all masked are left out.  The taps of a column are evaluated once for all
-// rows of the block.  Grid (ceil(NZ / ZB), NPmax, views of the chunk); dynamic
-// shared memory ZB rows of the longest in-plane axis.
+// X[vi][p][z][u0] for ZB rows z of plane p, for the views of the chunk that are
+// driven along one axis (grid.z even: y, odd: x; above two, every n-th of
+// them).  The rows are staged once for all views: a block per view read the
+// volume anew for each (4.3 GB at 256x256x128 and 129 views, as much as the
+// scratch it wrote) and waited for it.  A column's taps are evaluated once for
+// all rows of the block; columns whose rays are all masked are left out.  Grid
+// (ceil(NZ / ZB), NPmax, x_parts()); dynamic shared memory ZB rows of the
+// longest in-plane axis.
 template <int ZB>
 __global__ void __launch_bounds__(256) k_gx(const float* __restrict__ f, const float* __restrict__ fT,
                                            float* __restrict__ X, const GxArgs A)
 {
     extern __shared__ float rowbuf[];
     const petl_geom& G = A.G;
-    const int z0 = blockIdx.x * ZB, p = blockIdx.y, vi = blockIdx.z;
-    const int iv0 = A.vr.iv0_first + (A.vi0 + vi) * A.vr.iv0_step;
-    const bool xd = view_xdriven(G, iv0);
+    const int z0 = blockIdx.x * ZB, p = blockIdx.y;
+    const bool xd = blockIdx.z & 1;  // this block's views: driven along x or along y
+    const int part = blockIdx.z >> 1, nparts = (gridDim.z + 1) >> 1;
     const int NP = xd ? G.numX : G.numY, NA = xd ? G.numY : G.numX;
     if (p >= NP) return;
     const float* __restrict__ src = xd ? fT : f;  // [z][p][a]
     const int nz = min(ZB, G.numZ - z0);
-    for (int e = threadIdx.x; e < nz * NA; e += blockDim.x) {
-        const int r = e / NA, a = e - r * NA;
-        rowbuf[r * NA + a] = src[(size_t(z0 + r) * NP + p) * NA + a];
-    }
-    __syncthreads();
-    float* Xv = X + (size_t(vi) * A.NPmax + p) * G.numZ * A.NUc;
-    for (int iu0 = threadIdx.x; iu0 < G.N_u0; iu0 += blockDim.x) {
-        if (!u0_visible(G, iv0, iu0)) continue;
-        const RayGeom r = ray_geom(G, 0, iv0, 0, iu0);
-        const PlaneTaps pt = xd ? plane_taps_x(G, r, p) : plane_taps_y(G, r, p);
-        float acc[ZB];
-#pragma unroll
-        for (int k = 0; k < ZB; k++) acc[k] = 0.0f;
-        for (int a = pt.a_min; a <= pt.a_max; a++) {
-            const float w0 = xd ? tap_w0_x(G, r, pt.t, a, iu0) : tap_w0_y(G, r, pt.t, a, iu0);
-            if (!(w0 > 0.0f)) continue;
-#pragma unroll
-            for (int k = 0; k < ZB; k++) acc[k] = fmaf(w0, rowbuf[k * NA + a], acc[k]);
+    bool staged = false;
+    for (int vi = part; vi < A.nvc; vi += nparts) {
+        const int iv0 = A.vr.iv0_first + (A.vi0 + vi) * A.vr.iv0_step;
+        if (view_xdriven(G, iv0) != xd) continue;
+        if (!staged) {
+            for (int e = threadIdx.x; e < nz * NA; e += blockDim.x) {
+                const int r = e / NA, a = e - r * NA;
+                rowbuf[r * NA + a] = src[(size_t(z0 + r) * NP + p) * NA + a];
+            }
+            __syncthreads();
+            staged = true;
         }
+        float* Xv = X + (size_t(vi) * A.NPmax + p) * G.numZ * A.NUc;
+        for (int iu0 = threadIdx.x; iu0 < G.N_u0; iu0 += blockDim.x) {
+            if (!u0_visible(G, iv0, iu0)) continue;
+            const RayGeom r = ray_geom(G, 0, iv0, 0, iu0);
+            const PlaneTaps pt = xd ? plane_taps_x(G, r, p) : plane_taps_y(G, r, p);
+            float acc[ZB];
 #pragma unroll
-        for (int k = 0; k < ZB; k++)
-            if (k < nz) Xv[size_t(z0 + k) * A.NUc + iu0] = acc[k];
+            for (int k = 0; k < ZB; k++) acc[k] = 0.0f;
+            for (int a = pt.a_min; a <= pt.a_max; a++) {
+                const float w0 = xd ? tap_w0_x(G, r, pt.t, a, iu0) : tap_w0_y(G, r, pt.t, a, iu0);
+                if (!(w0 > 0.0f)) continue;
+#pragma unroll
+                for (int k = 0; k < ZB; k++) acc[k] = fmaf(w0, rowbuf[k * NA + a], acc[k]);
+            }
+#pragma unroll
+            for (int k = 0; k < ZB; k++)
+                if (k < nz) Xv[size_t(z0 + k) * A.NUc + iu0] = acc[k];
+        }
     }
 }
 
@@ -523,6 +536,8 @@ __global__ void __launch_bounds__(UZT, 1) k_uz(const __grid_constant__ CUtensorM
 #pragma unroll
     for (int k = 0; k < UZR; k++) acc[k] = 0ull;
     const double v1z = slope(min(iv1, A.vr.iv1_end - 1));
+    // a bin of the warp's slope is visible
+    const bool have = iv1 < v1e && __any_sync(0xffffffffu, row0 + lane < G.N_u1 && u1_visible(G, iv1, row0 + lane));
     bool dead = false;
     int slot = 0;
     uint32_t phase = 0;
@@ -534,8 +549,9 @@ __global__ void __launch_bounds__(UZT, 1) k_uz(const __grid_constant__ CUtensorM
         if (!dead) dead = !mbar_wait(&full[slot], phase, A.err, A.wait_limit);
         dead = __any_sync(0xffffffffu, dead);
         if (dead) *s_abort = 1;  // before this warp releases the slot
-        if (!dead && iv1 < v1e) {
-            const double eb = e0 - plane_par(pa + i) * v1z - s_wr[slot];
+        const double ez = e0 - plane_par(pa + i) * v1z;  // edge 0
+        if (!dead && have && ez < G.numZ && ez + UZR * rho > 0.0) {
+            const double eb = ez - s_wr[slot];
             bool bad = false;
             for (int k = lane; k <= UZR; k += 32) {
                 const double e = fma(double(k), rho, eb), fl = floor(e);
@@ -600,6 +616,14 @@ __global__ void __launch_bounds__(UZT, 1) k_uz(const __grid_constant__ CUtensorM
         g[at] = o.x;
         if (two) g[at + 1] = o.y;
     }
+}
+
+// grid.z of k_gx: both driving axes, and the views split over more blocks
+// where rows and planes alone give an SM less than about eight blocks.
+unsigned x_parts(unsigned blocks, int nviews)
+{
+    const unsigned want = ceil_div(8ll * sm_count(), blocks);
+    return 2u * std::max(1u, std::min(want, unsigned(nviews)));
 }
 
 bool aligned_90(const petl_geom& G) { return std::fabs(G.cos_psi) < 1e-6f && G.sin_psi == 1.0f; }
@@ -678,8 +702,9 @@ int project_usplit(const petl_geom& G, const float* f, float* g, const ViewRange
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kz, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     for (int c = 0; c < nchunks && e == cudaSuccess; c++) {
         const int vi0 = c * nv, nvc = std::min(nv, n_v0 - vi0);
-        const GxArgs XA{G, vr, vi0, NP, NUc};
-        kx<<<dim3(ceil_div(G.numZ, xzb), unsigned(NP), unsigned(nvc)), 256, xsmem, st>>>(f, fT, X, XA);
+        const GxArgs XA{G, vr, vi0, nvc, NP, NUc};
+        kx<<<dim3(ceil_div(G.numZ, xzb), unsigned(NP), x_parts(ceil_div(G.numZ, xzb) * unsigned(NP), nvc)), 256, xsmem,
+             st>>>(f, fT, X, XA);
         note_launch();
         Z.vi0 = vi0;
         kz<<<dim3(unsigned(Z.n_colblk) * unsigned(Z.n_rowblk) * ceil_div(nv1, UZS), unsigned(nvc)), UZT, smem, st>>>(
@@ -828,8 +853,9 @@ int project_gsplit(const petl_geom& G, const float* f, float* g, const ViewRange
         e = cudaFuncSetAttribute(k_gz<GZS_T / GJS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(zt.smem));
     for (int c = 0; c < nchunks && e == cudaSuccess; c++) {
         const int vi0 = c * nv, nvc = std::min(nv, n_v0 - vi0);
-        const GxArgs XA{G, vr, vi0, NPmax, NUc};
-        kx<<<dim3(ceil_div(G.numZ, xzb), unsigned(NPmax), unsigned(nvc)), 256, xsmem, st>>>(f, fT, X, XA);
+        const GxArgs XA{G, vr, vi0, nvc, NPmax, NUc};
+        kx<<<dim3(ceil_div(G.numZ, xzb), unsigned(NPmax), x_parts(ceil_div(G.numZ, xzb) * unsigned(NPmax), nvc)), 256,
+             xsmem, st>>>(f, fT, X, XA);
         note_launch();
         if (nv1_main > 0) {
             zm.Z.vi0 = vi0;
