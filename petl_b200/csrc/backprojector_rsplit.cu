@@ -148,11 +148,31 @@ __global__ void __launch_bounds__(RT2, 4) k_rbp_xy(const float* __restrict__ g, 
         live[v] = ix[v] < G.numX && iy[v] < G.numY;
         voxel_tx(G, min(ix[v], G.numX - 1), min(iy[v], G.numY - 1), t[v], xdt[v]);
     }
-    const int r0 = blockIdx.y * RRB;
     const int jv1 = blockIdx.z;
     const int iv1 = A.vr.iv1_begin + A.jv1_0 + jv1;
     const int lgW = A.lgW, W = 1 << lgW;
     const float v1 = fmaf(float(iv1), G.T_v1, G.v1_0);
+    // The u1 rows that k_rbp_z reads for voxels of this tile: u1 = z + v1 t over
+    // the volume's heights and the tile's corners, cut to the voxel visibility
+    // test's range, with a bin, half a voxel and a row of margin; other rows of P are left unwritten.
+    // PET/X's panels are two and a half times as high as its field of view:
+    // 1.17 -> 0.82 ms for a subset of 8 of both planograms.
+    float tmin = 3.0e38f, tmax = -3.0e38f;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        float tc, xc;
+        voxel_tx(G, c & 1 ? xl : x0, c & 2 ? yl : y0, tc, xc);
+        tmin = fminf(tmin, tc);
+        tmax = fmaxf(tmax, tc);
+    }
+    const float zt = fmaf(float(G.numZ - 1), G.T_z, G.z_0), ulim = G.H - G.R * fabsf(v1) + 0.5f * G.T_u1;
+    const float ulo = fmaxf(G.z_0 + fminf(v1 * tmin, v1 * tmax), -ulim);
+    const float uhi = fminf(zt + fmaxf(v1 * tmin, v1 * tmax), ulim);
+    const float pad = 0.5f * G.T_z / G.T_u1 + 2.0f;
+    const int rlo = max(0, int(floorf((ulo - G.u1_0) / G.T_u1 - pad)));
+    const int rhi = min(G.N_u1 - 1, int(ceilf((uhi - G.u1_0) / G.T_u1 + pad)));
+    const int r0 = rlo + blockIdx.y * RRB;
+    if (ulo > uhi + G.T_u1 || r0 > rhi) return;
     float* ring = rsm;  // [RSTG][W][RRP]
     // per view of the call: first staged column (the smallest first bin over
     // the tile's corners, the extent being affine in x and y, less one of
