@@ -237,7 +237,7 @@ k_bwd_zgather(const __grid_constant__ GMaps<NM> gmaps, float* __restrict__ B, co
     if (tid == 0) {
         *s_abort = 0;
         for (int s = 0; s < ns; s++) {
-            mbar_init(&full[s], BULK ? 1 : 33);  // the record's copy, and each lane's pairs
+            mbar_init(&full[s], BULK ? 1 : 1 + 128);  // or the stage's words, and each lane's copies
             mbar_init(&empty[s], A.nw);
         }
         fence_barrier_init();
@@ -245,8 +245,12 @@ k_bwd_zgather(const __grid_constant__ GMaps<NM> gmaps, float* __restrict__ B, co
     __syncthreads();
 
     if (warp >= A.nw) {
+        // the first of these warps is the producer; column pairs keep all four
+        // busy, each with every fourth row (one warp took 2.3 ms for what the
+        // consumers sum in 0.8: 31 slopes, 69 views, 150x141x75, 162 columns)
         producer_registers();
-        if (warp > A.nw) {
+        const int pw = warp - A.nw;
+        if (BULK && pw > 0) {
             __syncthreads();
             return;
         }
@@ -257,9 +261,24 @@ k_bwd_zgather(const __grid_constant__ GMaps<NM> gmaps, float* __restrict__ B, co
             const bool ok = round == 0 || ring_wait(&empty[slot], uint32_t((round - 1) & 1), A.err, s_abort, A.wait_limit);
             return __all_sync(0xffffffffu, ok && *s_abort == 0) != 0;
         };
-        int after = 0;  // the tile after the current one (lane 0)
-        for (int tile = blockIdx.x; tile < A.ntile && !dead; tile = __shfl_sync(0xffffffffu, after, 0)) {
-            if (lane == 0) after = int(gridDim.x) + atomicAdd(A.next, 1);
+        int after = 0;  // the tile after the current one (first lane)
+        int turn = 0;
+        // the next tile, or -1 once a wait gave up.  Several producer warps
+        // meet here after every tile, a warp that gave up included (each gets
+        // here in bounded time), and leave together.
+        auto next_tile = [&]() {
+            if (BULK) return dead ? -1 : __shfl_sync(0xffffffffu, after, 0);
+            if (dead) *s_abort = 1;
+            turn ^= 1;
+            if (pw == 0 && lane == 0) ctl->tile[turn] = after;
+            if (producers_or(dead)) {
+                dead = true;
+                return -1;
+            }
+            return ctl->tile[turn];
+        };
+        for (int tile = blockIdx.x; unsigned(tile) < unsigned(A.ntile); tile = next_tile()) {
+            if (pw == 0 && lane == 0) after = int(gridDim.x) + atomicAdd(A.next, 1);
             int t = tile;
             const int colblk = t % A.n_colblk;
             t /= A.n_colblk;
@@ -299,19 +318,19 @@ k_bwd_zgather(const __grid_constant__ GMaps<NM> gmaps, float* __restrict__ B, co
             for (int i = 0; i < nst; i++) {
                 if (!claim()) {
                     dead = true;
+                    if (!BULK) *s_abort = 1;  // the other producer warps stop as well
                     break;
                 }
                 const int slot = j % ns, np = max(0, min(2, nlive - 2 * i));
                 unsigned char* st = smem + size_t(slot) * A.stage;
                 const float s0 = scale(2 * i), s1 = scale(min(2 * i + 1, GV1MAX - 1));
-                if (lane == 0) {
+                if (lane == 0 && pw == 0) {
                     s_info[slot] = ZStage{2 * i, np | (i == 0 ? kZFirst : 0) | (i == nst - 1 ? kZLast : 0), p0, vi, r0,
                                           col0, s0, s1};
-                    fence_proxy_async_smem();
-                    uint32_t bytes = uint32_t(np) * uint32_t(sizeof(GRec));
-                    if (BULK) bytes += uint32_t(np) * uint32_t(A.nrb) * uint32_t(kZCols * EB);
-                    mbar_arrive_expect_tx(&full[slot], bytes);
                     if (BULK) {
+                        fence_proxy_async_smem();
+                        mbar_arrive_expect_tx(&full[slot], uint32_t(np) * (uint32_t(sizeof(GRec)) +
+                                                                           uint32_t(A.nrb) * uint32_t(kZCols * EB)));
                         const CUtensorMap* gmap = &gmaps.m[0];
 #pragma unroll
                         for (int m = 1; m < NM; m++)
@@ -320,23 +339,31 @@ k_bwd_zgather(const __grid_constant__ GMaps<NM> gmaps, float* __restrict__ B, co
                             const int2 sl = list[2 * i + h];
                             tma_load_4d(st + size_t(h) * A.sbytes, gmap, &full[slot], col0, sl.y, v0, sl.x);
                         }
+                        if (np)
+                            bulk_load(st + A.stage - 2 * sizeof(GRec), A.rec + tb * A.nv1 + 2 * i,
+                                      uint32_t(np) * uint32_t(sizeof(GRec)), &full[slot]);
+                    } else {
+                        mbar_arrive(&full[slot]);
                     }
-                    if (np)
-                        bulk_load(st + A.stage - 2 * sizeof(GRec), A.rec + tb * A.nv1 + 2 * i,
-                                  uint32_t(np) * uint32_t(sizeof(GRec)), &full[slot]);
                 }
                 if (!BULK) {
                     const TG* g = static_cast<const TG*>(member_pick<NM>(A.M.in, mb));
                     const int c = col0 + 2 * lane;
                     const bool cok = c < G.N_u0;  // N_u0 is even: both columns of the pair
+                    static_assert(sizeof(GRec) % 16 == 0 && 2 * sizeof(GRec) <= 32 * 16, "a lane per 16 bytes");
+                    if (pw == 0 && lane < np * int(sizeof(GRec) / 16))
+                        pair_load<16>(smem_addr(st + A.stage - 2 * sizeof(GRec)) + 16u * lane,
+                                      reinterpret_cast<const unsigned char*>(A.rec + tb * A.nv1 + 2 * i) + 16 * lane, true);
                     for (int h = 0; h < np; h++) {
                         const int2 sl = list[2 * i + h];
-                        const TG* gs = g + (size_t(sl.x) * G.N_v0 + v0) * G.N_u1 * G.N_u0;
-                        const uint32_t dst = smem_addr(st + size_t(h) * A.sbytes) + uint32_t(2 * lane * EB);
-                        for (int r = 0; r < A.nrb; r++) {
-                            const int row = sl.y + r;
-                            const bool ok = cok && unsigned(row) < unsigned(G.N_u1);
-                            pair_load<2 * EB>(dst + uint32_t(r * kZCols * EB), ok ? gs + size_t(row) * G.N_u0 + c : gs, ok);
+                        const TG* src = g + ((size_t(sl.x) * G.N_v0 + v0) * G.N_u1 + sl.y + pw) * G.N_u0 + c;
+                        uint32_t dst = smem_addr(st + size_t(h) * A.sbytes) + uint32_t((pw * kZCols + 2 * lane) * EB);
+#pragma unroll 4
+                        for (int r = pw; r < A.nrb; r += 4) {
+                            const bool ok = cok && unsigned(sl.y + r) < unsigned(G.N_u1);
+                            pair_load<2 * EB>(dst, ok ? src : g, ok);
+                            src += 4 * G.N_u0;
+                            dst += uint32_t(4 * kZCols * EB);
                         }
                     }
                     pair_arrive(&full[slot]);
@@ -347,7 +374,7 @@ k_bwd_zgather(const __grid_constant__ GMaps<NM> gmaps, float* __restrict__ B, co
         }
         if (!dead && claim()) {
             const int slot = j % ns;
-            if (lane == 0) {
+            if (lane == 0 && pw == 0) {
                 s_info[slot].flags = kZEnd;
                 mbar_arrive(&full[slot]);
             }
@@ -359,8 +386,9 @@ k_bwd_zgather(const __grid_constant__ GMaps<NM> gmaps, float* __restrict__ B, co
         __syncthreads();
         // a wait gave up: drain the copies still in flight
         if (*s_abort) {
-            pair_drain();
-            if (lane == 0)
+            if (!BULK)
+                pair_drain();
+            else if (lane == 0)
                 for (int i = max(0, j - ns); i < j; i++) mbar_wait(&full[i % ns], uint32_t((i / ns) & 1), nullptr);
         }
         return;

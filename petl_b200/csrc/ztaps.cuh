@@ -146,6 +146,22 @@ constexpr int kZThreads = 32 * (kZWarps + 4);
 __device__ __forceinline__ void consumer_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 160;"); }
 __device__ __forceinline__ void producer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 32;"); }
 
+// Whether any of the four producer warps (128 threads) passes true; all of
+// them call it the same number of times.
+__device__ __forceinline__ bool producers_or(bool v)
+{
+    uint32_t any;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "bar.red.or.pred q, 1, 128, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(any)
+        : "r"(uint32_t(v))
+        : "memory");
+    return any != 0;
+}
+
 // What the producer tells the consumers about a stage.
 struct __align__(16) ZStage {
     int y;      // first plane (forward) or position in the slope list (backward)
@@ -170,6 +186,7 @@ struct ZCtl {
     // per tile, and its instruction fetches took a fifth of the forward's time
     f2x out[kZWarps][4][32];
     int abort;  // a warp gave up a wait: start no further copies
+    int tile[2];  // the producer warps' next tile, by turns
 };
 
 // Rows 4 * (i % (NK / 4)) .. + 3 of accumulator block i / (NK / 4) to the
