@@ -26,7 +26,17 @@ __global__ void __launch_bounds__(256) k_reduce_partial(Term term, long long n, 
 {
     double s = 0.0;
     const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) s += term(i);
+    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    // four terms at a time, added in the order of the plain loop, so that
+    // their loads are in flight together
+    for (; i + 3 * stride < n; i += 4 * stride) {
+        double t[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) t[k] = term(i + k * stride);
+#pragma unroll
+        for (int k = 0; k < 4; k++) s += t[k];
+    }
+    for (; i < n; i += stride) s += term(i);
     s = block_sum<256>(s);
     if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }

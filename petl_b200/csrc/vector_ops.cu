@@ -95,7 +95,12 @@ struct LoglikTerm {
     __device__ double operator()(long long i) const
     {
         const float p = pf[i];
-        return p > 0.0f ? double(g[i]) * log(double(p)) - double(p) : 0.0;
+        const float x = g[i];
+        if (!(p > 0.0f)) return 0.0;
+        // a bin without counts (most bins of a low-count scan) needs no log;
+        // 0 * log(p) is 0 for every finite p
+        if (x == 0.0f && p <= 3.402823466e38f) return -double(p);
+        return double(x) * log(double(p)) - double(p);
     }
 };
 
