@@ -25,7 +25,7 @@
 // at v1 = 0 (the rebinned planogram of FBP) takes k_bwd_zflat: its z sums
 // do not depend on the plane.
 //
-// 256x256x128, planogram (65, 129, 128, 256): 8.7 ms for the z taps and 0.9
+// 256x256x128, planogram (65, 129, 128, 256): 7.9 ms for the z taps and 0.9
 // for the x pass (before: 12.5 and 0.9, with one 16-warp CTA per tile, tables
 // built by every CTA and scalar FMAs).  FBP's single slope: 0.42 ms (0.72 with
 // a thread per x).
@@ -498,7 +498,6 @@ struct XgatherArgs {
     float scale;
     Tables T;
     Members M;       // volumes (out) and views of the chunk
-    int adjoint;     // only the view's visible columns count (the scratch holds no others)
 };
 
 // x shift of a view on a plane and the scratch columns that count
@@ -516,11 +515,13 @@ constexpr int XMAXN = 1024;   // longest scratch / volume row
 // view of that member straight from global memory (neighbouring threads
 // share them through L1).  Grid (ceil(numX / 256), ceil(numZ / 4), numY x
 // members).
-template <int NM>
+template <bool ADJ, int NM>
 __global__ void __launch_bounds__(256) k_bwd_xgather(const float* __restrict__ B, float* __restrict__ part,
                                                      const XgatherArgs A)
 {
-    extern __shared__ XView s_xs[];  // [views of the member]
+    extern __shared__ __align__(16) unsigned char s_views[];
+    Shift* s_xs = reinterpret_cast<Shift*>(s_views);                     // [views of the member] x shifts of plane y
+    int2* s_vis = reinterpret_cast<int2*>(s_views) + A.M.nvm;             // and (adjoint) visible columns
     const petl_geom& G = A.G;
     const int NY = G.numY, NZ = G.numZ, NX = G.numX, NU0 = G.N_u0, NUc = A.NUc;
     const int mb = NM == 1 ? 0 : blockIdx.z / NY, y = blockIdx.z - mb * NY;
@@ -529,9 +530,8 @@ __global__ void __launch_bounds__(256) k_bwd_xgather(const float* __restrict__ B
     float* __restrict__ f = static_cast<float*>(member_pick<NM>(A.M.out, mb));
     for (int vi = threadIdx.x; vi < nvb; vi += 256) {
         const int v0 = first + vi * A.step;
-        const Shift xs = A.T.xt[size_t(v0) * NY + y];
-        const int2 u = A.adjoint ? A.T.ub0[v0] : make_int2(0, NU0 - 1);
-        s_xs[vi] = XView{xs.d, xs.w, u.x, max(0, u.y - u.x + 1)};
+        s_xs[vi] = A.T.xt[size_t(v0) * NY + y];
+        if (ADJ) s_vis[vi] = A.T.ub0[v0];
     }
     __syncthreads();
     if (x >= NX) return;
@@ -544,10 +544,12 @@ __global__ void __launch_bounds__(256) k_bwd_xgather(const float* __restrict__ B
     const float* Bm = B + size_t(mb) * A.M.nvm * NY * NZ * NUc;
 #pragma unroll 4
     for (int vi = 0; vi < nvb; vi++) {
-        const XView xs = s_xs[vi];
+        const Shift xs = s_xs[vi];
         const float wx1 = xs.w, wx0 = 1.0f - xs.w;
         const int j0 = x - xs.d;  // scratch column of tap 0
-        const bool okm = unsigned(j0 - 1 - xs.lo) < unsigned(xs.n), ok0 = unsigned(j0 - xs.lo) < unsigned(xs.n);
+        // the adjoint counts the view's visible columns only (the scratch holds no others)
+        const int2 u = ADJ ? s_vis[vi] : make_int2(0, NU0 - 1);
+        const bool okm = j0 - 1 >= u.x && j0 - 1 <= u.y, ok0 = j0 >= u.x && j0 <= u.y;
         // in-bounds addresses for every tap; the out-of-range ones are selected away
         const int jm = min(max(j0 - 1, 0), NU0 - 1), jz = min(max(j0, 0), NU0 - 1);
         const float* Bv = Bm + ((size_t(vi) * NY + y) * NZ + z0) * NUc;
@@ -886,7 +888,8 @@ int backproject_split_m(const petl_geom& G, const Members& M0, int mode, int acc
         }
         return r;
     };
-    auto kx = nb == 1 ? k_bwd_xgather<1> : k_bwd_xgather<kMaxMembers>;
+    auto kx = adj ? (nb == 1 ? k_bwd_xgather<true, 1> : k_bwd_xgather<true, kMaxMembers>)
+                  : (nb == 1 ? k_bwd_xgather<false, 1> : k_bwd_xgather<false, kMaxMembers>);
     cudaError_t e = cudaGetLastError();
     for (int c = 0; c < nchunks && e == cudaSuccess; c++) {
         Members M = M0;
@@ -913,9 +916,9 @@ int backproject_split_m(const petl_geom& G, const Members& M0, int mode, int acc
         if (e != cudaSuccess) break;
         note_launch();
         A.next++;
-        XgatherArgs X{G, vr.iv0_step, A.NUc, c == 0, c == nchunks - 1, accumulate, scale, T, M, adj};
+        XgatherArgs X{G, vr.iv0_step, A.NUc, c == 0, c == nchunks - 1, accumulate, scale, T, M};
         kx<<<dim3(ceil_div(G.numX, 256), ceil_div(G.numZ, XR), unsigned(G.numY) * unsigned(nb)), 256,
-                        size_t(nvc) * sizeof(XView), st>>>(B, part, X);
+                        size_t(nvc) * (adj ? 2 : 1) * sizeof(Shift), st>>>(B, part, X);
         note_launch();
         e = cudaGetLastError();
     }

@@ -18,14 +18,14 @@
 //   slope to slope, so they form one of 15 monotone patterns: one dispatch per
 //   plane selects a fully unrolled form.
 //
-// 256x256x128, planogram (65, 129, 128, 256): 7.7 ms for the z taps and 0.7
+// 256x256x128, planogram (65, 129, 128, 256): 7.5 ms for the z taps and 0.7
 // for the x pass (before: 10.0 and 0.9, with one 16-warp CTA per tile, tables
 // built by every CTA, scalar FMAs on 8 rows per warp and tiles that started at
 // bin 0).  What the steps gave on the z taps: twelve warps x 12 rows against
 // eight x 16 9 %, tiles handed out by a counter against a fixed stride 18 % (the
 // stride of 148 met the period of the column blocks, whose last is often
-// empty), a rolled epilogue 10 % and its loads in batches another 25 % where
-// the MLEM ratio is computed.
+// empty), a rolled epilogue 10 %, twelve rows at a time against four 4 %, and its
+// loads in batches another 25 % where the MLEM ratio is computed.
 //
 // Both kernels do the float operations of project_tma in the same order (x
 // taps fmaf(w1, b, w0 * a); per ray, the z taps of the live planes in
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(256) k_xshift(float* __restrict__ X, const Xsh
 // Bound by FP32 issue: a plane costs a warp 96 packed FMAs (192 cycles of its
 // scheduler, which holds three such warps) and 16 eight-byte window loads (32
 // cycles of the SM's shared memory, of which twelve warps take 384 of the 576
-// cycles the FMAs take).  Measured 850 cycles per plane: the dispatch, the
+// cycles the FMAs take).  Measured 830 cycles per plane: the dispatch, the
 // window's first loads and the ring's waits are not fully covered.  4 slopes x
 // 16 rows in eight warps need fewer loads per FMA but ran at 800 cycles for
 // 512 of FMAs; 8 rows and 16 warps are bound by the loads.
@@ -464,31 +464,36 @@ k_fwd_zsum(const __grid_constant__ ZMaps maps, const __grid_constant__ ZsumArgs 
                 const float S = A.T.S[size_t(v1) * G.N_v0 + iv0];
                 const int2 u1r = A.T.ub1[v1];
                 const size_t o0 = (size_t(v1) * G.N_v0 + iv0) * G.N_u1 * G.N_u0;
-                if (pairs && colA + 1 < G.N_u0) {
-                    float2 m[kZOut];
-                    if (meas)
-#pragma unroll
-                        for (int k = 0; k < kZOut; k++)
-                            if (r0 + k < G.N_u1) m[k] = Store<TG>::ld2(meas + o0 + size_t(r0 + k) * G.N_u0 + colA);
-#pragma unroll
-                    for (int k = 0; k < kZOut; k++) {
-                        if (r0 + k >= G.N_u1) break;
-                        const bool rv = r0 + k >= u1r.x && r0 + k <= u1r.y;
-                        const float2 a = f2_unpack(out[k * 32]);
-                        float2 val = make_float2(rv && ok0 ? a.x * S : 0.0f, rv && ok1 ? a.y * S : 0.0f);
-                        if (meas) val = make_float2(ratio_rule(m[k].x, val.x), ratio_rule(m[k].y, val.y));
-                        Store<TG>::st2(g + o0 + size_t(r0 + k) * G.N_u0 + colA, val);
-                    }
-                } else {  // odd rows, or the row's last column
 #pragma unroll 1
-                    for (int k = 0; k < min(kZOut, G.N_u1 - r0); k++) {
-                        const bool rv = r0 + k >= u1r.x && r0 + k <= u1r.y;
-                        const size_t o = o0 + size_t(r0 + k) * G.N_u0 + colA;
-                        const float2 a = f2_unpack(out[k * 32]);
-                        const float2 val = make_float2(rv && ok0 ? a.x * S : 0.0f, rv && ok1 ? a.y * S : 0.0f);
-                        if (colA < G.N_u0) g[o] = Store<TG>::st(meas ? ratio_rule(Store<TG>::ld(meas[o]), val.x) : val.x);
-                        if (colA + 1 < G.N_u0)
-                            g[o + 1] = Store<TG>::st(meas ? ratio_rule(Store<TG>::ld(meas[o + 1]), val.y) : val.y);
+                for (int kk = 0; kk < kZOut; kk += 4) {
+                    if (pairs && colA + 1 < G.N_u0) {
+                        float2 m[4];
+                        if (meas)
+#pragma unroll
+                            for (int k = 0; k < 4; k++)
+                                if (r0 + kk + k < G.N_u1)
+                                    m[k] = Store<TG>::ld2(meas + o0 + size_t(r0 + kk + k) * G.N_u0 + colA);
+#pragma unroll
+                        for (int k = 0; k < 4; k++) {
+                            const int iu1 = r0 + kk + k;
+                            if (iu1 >= G.N_u1) break;
+                            const bool rv = iu1 >= u1r.x && iu1 <= u1r.y;
+                            const float2 a = f2_unpack(out[(kk + k) * 32]);
+                            float2 val = make_float2(rv && ok0 ? a.x * S : 0.0f, rv && ok1 ? a.y * S : 0.0f);
+                            if (meas) val = make_float2(ratio_rule(m[k].x, val.x), ratio_rule(m[k].y, val.y));
+                            Store<TG>::st2(g + o0 + size_t(iu1) * G.N_u0 + colA, val);
+                        }
+                    } else {  // odd rows, or the row's last column
+#pragma unroll 1
+                        for (int k = kk; k < min(kk + 4, G.N_u1 - r0); k++) {
+                            const bool rv = r0 + k >= u1r.x && r0 + k <= u1r.y;
+                            const size_t o = o0 + size_t(r0 + k) * G.N_u0 + colA;
+                            const float2 a = f2_unpack(out[k * 32]);
+                            const float2 val = make_float2(rv && ok0 ? a.x * S : 0.0f, rv && ok1 ? a.y * S : 0.0f);
+                            if (colA < G.N_u0) g[o] = Store<TG>::st(meas ? ratio_rule(Store<TG>::ld(meas[o]), val.x) : val.x);
+                            if (colA + 1 < G.N_u0)
+                                g[o + 1] = Store<TG>::st(meas ? ratio_rule(Store<TG>::ld(meas[o + 1]), val.y) : val.y);
+                        }
                     }
                 }
             }

@@ -176,34 +176,34 @@ constexpr int kZEnd = 16;    // no more tiles
 constexpr int kZRow0 = 32, kZRowN = 64, kZCol0 = 128, kZColN = 256;  // tile at an edge of the output
 constexpr int kZTail = 512;  // tile of the tail launch shape
 
+constexpr int kZOut = 12;
+
 // Ring control block, after the stages in shared memory.
 struct ZCtl {
     ZStage info[kZStages];
     uint64_t full[kZStages], empty[kZStages];
-    // a warp's epilogue passes its accumulators through here, four rows at a
+    // a warp's epilogue passes its accumulators through here, twelve rows at a
     // time, so that the code that scales, masks and stores them is one rolled
     // loop: unrolled over all accumulators it was tens of KB of straight code
     // per tile, and its instruction fetches took a fifth of the forward's time
-    f2x out[kZWarps][4][32];
+    f2x out[kZWarps][kZOut][32];
     int abort;  // a warp gave up a wait: start no further copies
     int tile[2];  // the producer warps' next tile, by turns
 };
 
-// Rows 4 * (i % (NK / 4)) .. + 3 of accumulator block i / (NK / 4) to the
+// Rows 12 * (i % (NK / 12)) .. + 11 of accumulator block i / (NK / 12) to the
 // warp's lane slots.
-constexpr int kZOut = 4;
 template <int N, int NK>
 __device__ __forceinline__ void out_rows(const f2x (&acc)[N][NK], f2x* out, int i)
 {
-    static_assert(N * NK == 12 * kZOut, "twelve groups of four rows");
+    static_assert(N * NK == 4 * kZOut, "four groups of twelve rows");
     switch (i) {
 #define PETL_ZOUT(I)                                                                       \
     case I:                                                                                \
         _Pragma("unroll") for (int k = 0; k < kZOut; k++) out[k * 32] =                    \
             acc[I / (NK / kZOut)][I % (NK / kZOut) * kZOut + k];                           \
         break;
-        PETL_ZOUT(0) PETL_ZOUT(1) PETL_ZOUT(2) PETL_ZOUT(3) PETL_ZOUT(4) PETL_ZOUT(5) PETL_ZOUT(6) PETL_ZOUT(7)
-        PETL_ZOUT(8) PETL_ZOUT(9) PETL_ZOUT(10) PETL_ZOUT(11)
+        PETL_ZOUT(0) PETL_ZOUT(1) PETL_ZOUT(2) PETL_ZOUT(3)
 #undef PETL_ZOUT
     }
 }
