@@ -417,7 +417,7 @@ k_bwd_zgather(const __grid_constant__ GMaps<NM> gmaps, float* __restrict__ B, co
                 const GRec* rec = reinterpret_cast<const GRec*>(st + A.stage - 2 * sizeof(GRec));
                 const float* sc = &s_info[slot].s0;
 #pragma unroll 1
-                for (int h = flags & 3; h > 0; h--, rec++, sc++, st += A.sbytes) {
+                for (int h = flags & kZCount; h > 0; h--, rec++, sc++, st += A.sbytes) {
                     const uint32_t code = rec->code[warp];
                     if (!(code & 0x300u)) continue;
                     const auto* W = reinterpret_cast<const typename Pair<TG>::type*>(st) +

@@ -85,7 +85,7 @@ struct ZKind {
     int n_rowblk;      // row blocks at most (the visible rows of a block need fewer)
     int nrb;           // staged rows per plane (rows + shift spread of the block + 1)
     int pstride;       // floats per staged plane (nrb + kZSpread rows of 64)
-    int pps;           // planes per stage: two, or one of the tail's tall planes
+    int pps;           // planes per stage
     int blk0;          // index of the first block in the tables
     int ntile;
 };
@@ -96,8 +96,9 @@ struct ZsumArgs {
     int nw;         // consumer warps
     int nslot;      // view slots of all members
     int n_colblk;   // column blocks at most
-    int ns;         // ring stages, two planes each
-    int stage;      // bytes per stage (planes, then two records)
+    int ns;         // ring stages
+    int stage;      // bytes per stage (planes, then their records)
+    int rec_off;    // the records' offset in a stage
     ZKind k[2];     // full blocks, and the tail of at most half a block
     ZRec* rec;      // [block][plane]
     int* dz;        // [block][plane] smallest shift of the block
@@ -343,7 +344,7 @@ k_fwd_zsum(const __grid_constant__ ZMaps maps, const __grid_constant__ ZsumArgs 
                         tma_load_4d(st + size_t(h) * K.pstride * 4, &maps.m[kind], &full[slot], col0, row0 + dz[y + h],
                                     y + h, vi);
                     if (np)
-                        bulk_load(st + A.stage - 2 * sizeof(ZRec), A.rec + size_t(K.blk0 + blk) * NY + y,
+                        bulk_load(st + A.rec_off, A.rec + size_t(K.blk0 + blk) * NY + y,
                                   uint32_t(np) * uint32_t(sizeof(ZRec)), &full[slot]);
                     j++;
                 }
@@ -396,38 +397,57 @@ k_fwd_zsum(const __grid_constant__ ZMaps maps, const __grid_constant__ ZsumArgs 
                 const int flags = s_info[slot].flags;
                 if (have) {
                     const unsigned char* st = smem + size_t(slot) * A.stage;
-                    const ZRec* rec = reinterpret_cast<const ZRec*>(st + A.stage - 2 * sizeof(ZRec));
-#pragma unroll 1
-                    for (int h = flags & 3; h > 0; h--, rec++, st += pbytes) {
-                        const uint32_t code = rec->code[gv];
-                        f2x wa[NV], wb[NV];
+                    const ZRec* rec = reinterpret_cast<const ZRec*>(st + A.rec_off);
+                    const f2x* W;
+                    f2x wa[NV], wb[NV];
+                    uint32_t code;
+                    int left = flags & kZCount;  // planes of the stage still to sum
+                    auto load = [&]() {
+                        code = rec->code[gv];
+                        W = reinterpret_cast<const f2x*>(st) + (int((code >> 8) & 0xffu) + gr * NK) * (kZCols / 2) + lane;
 #pragma unroll
                         for (int j = 0; j < NV; j++) {
                             const float w = rec->w[gv * NV + j];
                             wa[j] = f2_dup(1.0f - w);
                             wb[j] = f2_dup(w);
                         }
-                        const int iz0 = row0 + int(int16_t(code >> 16));  // volume row of window row 0
-                        if (iz0 + WN - 1 < 0 || iz0 >= NZ) continue;
-                        const f2x* W = reinterpret_cast<const f2x*>(st) +
-                                       (int((code >> 8) & 0xffu) + gr * NK) * (kZCols / 2) + lane;
-                        // the offsets of consecutive slopes are monotone and
-                        // (four slopes) at most one row apart: one dispatch
-                        // per plane over the patterns that occur
+                    };
+                    // on to the next plane; whether it has the same pattern
+                    auto next = [&](uint32_t pattern) {
+                        rec++;
+                        st += pbytes;
+                        if (--left <= 0) return false;
+                        load();
+                        return (code & 0xffu) == pattern;
+                    };
+                    if (left > 0) load();
+                    // the offsets of consecutive slopes are monotone and (four
+                    // slopes) at most one row apart: one dispatch over the
+                    // patterns that occur for each run of planes with the same
+                    // one (a jump to another pattern's code costs a quarter of
+                    // the time a plane's taps take)
+                    while (left > 0) {
+#define PETL_ZCASE(PC)                        \
+    case PC:                                  \
+        do                                    \
+            z_taps<PC, true>(acc, W, wa, wb); \
+        while (next(PC));                     \
+        break;
                         if constexpr (NV == 4) {
                             switch (code & 0xffu) {
-#define PETL_ZCASE(PC) case PC: z_taps<PC, true>(acc, W, wa, wb); break;
                                 PETL_ZCASE(0x00) PETL_ZCASE(0x40) PETL_ZCASE(0x50) PETL_ZCASE(0x90) PETL_ZCASE(0x54)
                                 PETL_ZCASE(0x94) PETL_ZCASE(0xA4) PETL_ZCASE(0xE4) PETL_ZCASE(0x01) PETL_ZCASE(0x05)
                                 PETL_ZCASE(0x15) PETL_ZCASE(0x06) PETL_ZCASE(0x16) PETL_ZCASE(0x1A) PETL_ZCASE(0x1B)
+                                default: next(0x100u);  // no such pattern: a layout error, reported
                             }
                         } else {
-                            switch (code & 0xfu) {
+                            switch (code & 0xffu) {
                                 PETL_ZCASE(0x0) PETL_ZCASE(0x4) PETL_ZCASE(0x8) PETL_ZCASE(0xC) PETL_ZCASE(0x1)
                                 PETL_ZCASE(0x2) PETL_ZCASE(0x3)
-#undef PETL_ZCASE
+                                default: next(0x100u);
                             }
                         }
+#undef PETL_ZCASE
                     }
                 }
                 __syncwarp();
@@ -571,7 +591,6 @@ bool zsum_plan(const petl_geom& G, const ViewRange& vr, double step, int nslot, 
             K.n_rowblk = int(ceil_div(G.N_u1, K.rows));
             K.nrb = K.rows + shift_spread(P.nv * K.sg - 1, step) + 1;
             K.pstride = (K.nrb + kZSpread) * kZCols;
-            K.pps = i ? 1 : 2;
             K.blk0 = i ? A.k[0].nblk : 0;
             if (K.nrb > 256 - kZSpread) return false;  // TMA box rows; the window row fits 8 bits
             const long long nt = (long long)nslot * K.nblk * K.n_rowblk * A.n_colblk;
@@ -581,12 +600,18 @@ bool zsum_plan(const petl_geom& G, const ViewRange& vr, double step, int nslot, 
         }
         if (A.nw == 4 || tiles >= sm_count()) break;
     }
-    A.stage = 0;
-    for (const ZKind& K : A.k)
-        if (K.nblk > 0) A.stage = std::max(A.stage, K.pstride * K.pps * 4);
-    A.stage += 2 * int(sizeof(ZRec));
-    A.stage = (A.stage + 127) & ~127;
-    A.ns = std::min(kZStages, (227 * 1024 - int(sizeof(ZCtl))) / A.stage);
+    // four planes per stage (longer runs of one pattern, fewer waits) where
+    // three stages fit, else two; the tail's tall planes one or two at a time
+    for (int pps = 4;; pps = 2) {
+        A.k[0].pps = pps;
+        A.k[1].pps = std::max(1, std::min(pps, A.k[0].nblk ? pps * A.k[0].pstride / A.k[1].pstride : 2));
+        A.rec_off = 0;
+        for (const ZKind& K : A.k)
+            if (K.nblk > 0) A.rec_off = std::max(A.rec_off, K.pstride * K.pps * 4);
+        A.stage = (A.rec_off + pps * int(sizeof(ZRec)) + 127) & ~127;
+        A.ns = std::min(kZStages, (227 * 1024 - int(sizeof(ZCtl))) / A.stage);
+        if (A.ns >= 3 || pps == 2) break;
+    }
     if (A.ns < 2) return false;
     P.smem = size_t(A.ns) * A.stage + sizeof(ZCtl);
     const size_t nrec = size_t(A.k[0].nblk + A.k[1].nblk) * G.numY;

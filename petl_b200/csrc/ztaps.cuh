@@ -165,14 +165,15 @@ __device__ __forceinline__ bool producers_or(bool v)
 // What the producer tells the consumers about a stage.
 struct __align__(16) ZStage {
     int y;      // first plane (forward) or position in the slope list (backward)
-    int flags;  // staged planes / slopes (0..2) | kFirst | kLast | kEnd | kExt*
+    int flags;  // staged planes / slopes | kZFirst | kZLast | ...
     int a, b;   // tile: first slope / plane, view slot
     int row0, col0;
     float s0, s1;  // backward: ray scale of the staged slopes
 };
-constexpr int kZFirst = 4;   // first stage of a tile
-constexpr int kZLast = 8;    // last stage of a tile
-constexpr int kZEnd = 16;    // no more tiles
+constexpr int kZCount = 7;   // planes / slopes of the stage
+constexpr int kZFirst = 8;   // first stage of a tile
+constexpr int kZLast = 16;   // last stage of a tile
+constexpr int kZEnd = 1024;  // no more tiles
 constexpr int kZRow0 = 32, kZRowN = 64, kZCol0 = 128, kZColN = 256;  // tile at an edge of the output
 constexpr int kZTail = 512;  // tile of the tail launch shape
 
