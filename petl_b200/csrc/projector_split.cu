@@ -16,15 +16,16 @@
 //   into a ring with full/empty mbarriers, across tile borders.  The tap
 //   offsets of a warp's four consecutive slopes move by at most one row from
 //   slope to slope, so they form one of 15 monotone patterns: one dispatch per
-//   plane selects a fully unrolled form.
+//   run of planes with the same one selects a fully unrolled form.
 //
-// 256x256x128, planogram (65, 129, 128, 256): 7.5 ms for the z taps and 0.7
+// 256x256x128, planogram (65, 129, 128, 256): 7.0 ms for the z taps and 0.7
 // for the x pass (before: 10.0 and 0.9, with one 16-warp CTA per tile, tables
 // built by every CTA, scalar FMAs on 8 rows per warp and tiles that started at
 // bin 0).  What the steps gave on the z taps: twelve warps x 12 rows against
 // eight x 16 9 %, tiles handed out by a counter against a fixed stride 18 % (the
 // stride of 148 met the period of the column blocks, whose last is often
-// empty), a rolled epilogue 10 %, twelve rows at a time against four 4 %, and its
+// empty), a rolled epilogue 10 %, twelve rows at a time against four 4 %, runs of
+// planes with one pattern 7 %, and the epilogue's
 // loads in batches another 25 % where the MLEM ratio is computed.
 //
 // Both kernels do the float operations of project_tma in the same order (x
@@ -227,7 +228,7 @@ __global__ void __launch_bounds__(256) k_xshift(float* __restrict__ X, const Xsh
 // of the block and the first visible column of the view (masked rays are
 // written as zeros by the tiles at the edge, not computed); a warp sums NV
 // slopes x NK rows x 2 columns per lane over the planes.  The producer walks
-// the tiles and stages their planes two at a time, rows by a tiled TMA copy
+// the tiles and stages their planes two or four at a time, rows by a tiled TMA copy
 // (no multicast) and the planes' table records by a bulk copy, ahead of the
 // consumers across tile borders, so set-up and epilogue of a warp overlap the
 // sums of the others.
