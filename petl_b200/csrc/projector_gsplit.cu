@@ -115,10 +115,13 @@ __device__ __forceinline__ bool view_xdriven(const petl_geom& G, int iv0)
 // them).  The rows are staged once for all views: a block per view read the
 // volume anew for each (4.3 GB at 256x256x128 and 129 views, as much as the
 // scratch it wrote) and waited for it.  A column's taps are evaluated once for
-// all rows of the block; columns whose rays are all masked are left out.  Grid
+// all rows of the block; columns whose rays are all masked are left out.  AXIS
+// (psi = 0 and 90, unequal pitch): the taps in double, for bins hundreds of
+// voxels from the origin leave a float's fraction five digits, and a sharp image
+// shows it.  Grid
 // (ceil(NZ / ZB), NPmax, x_parts()); dynamic shared memory ZB rows of the
 // longest in-plane axis.
-template <int ZB>
+template <int ZB, bool AXIS>
 __global__ void __launch_bounds__(256) k_gx(const float* __restrict__ f, const float* __restrict__ fT,
                                            float* __restrict__ X, const GxArgs A)
 {
@@ -146,13 +149,32 @@ __global__ void __launch_bounds__(256) k_gx(const float* __restrict__ f, const f
         float* Xv = X + (size_t(vi) * A.NPmax + p) * G.numZ * A.NUc;
         for (int iu0 = threadIdx.x; iu0 < G.N_u0; iu0 += blockDim.x) {
             if (!u0_visible(G, iv0, iu0)) continue;
-            const RayGeom r = ray_geom(G, 0, iv0, 0, iu0);
-            const PlaneTaps pt = xd ? plane_taps_x(G, r, p) : plane_taps_y(G, r, p);
             float acc[ZB];
 #pragma unroll
             for (int k = 0; k < ZB; k++) acc[k] = 0.0f;
+            RayGeom r;
+            PlaneTaps pt;
+            double ua = 0.0, a0 = 0.0;  // AXIS: in-plane position of the ray, of voxel 0
+            const double Tx = double(G.T_x), Tu = double(G.T_u0), fw = 0.5 * Tx / Tu;
+            if (AXIS) {
+                const double t = ((xd ? double(G.x_0) : double(G.y_0)) + p * Tx) * (xd ? -1.0 : 1.0);
+                a0 = xd ? double(G.y_0) : double(G.x_0);
+                ua = (double(G.u0_0) + iu0 * Tu) - t * (double(G.v0_0) + iv0 * double(G.T_v0));
+                const double half = 0.5 * (Tu + Tx);
+                pt.a_min = max(0, int(ceil((ua - half - a0) / Tx)));
+                pt.a_max = min(NA - 1, int(floor((ua + half - a0) / Tx)));
+            } else {
+                r = ray_geom(G, 0, iv0, 0, iu0);
+                pt = xd ? plane_taps_x(G, r, p) : plane_taps_y(G, r, p);
+            }
             for (int a = pt.a_min; a <= pt.a_max; a++) {
-                const float w0 = xd ? tap_w0_x(G, r, pt.t, a, iu0) : tap_w0_y(G, r, pt.t, a, iu0);
+                float w0;
+                if (AXIS) {
+                    const double c = (a0 + a * Tx - ua) / Tu;  // voxel centre in bins from the ray
+                    w0 = float(fmin(0.5, c + fw) - fmax(-0.5, c - fw));
+                } else {
+                    w0 = xd ? tap_w0_x(G, r, pt.t, a, iu0) : tap_w0_y(G, r, pt.t, a, iu0);
+                }
                 if (!(w0 > 0.0f)) continue;
 #pragma unroll
                 for (int k = 0; k < ZB; k++) acc[k] = fmaf(w0, rowbuf[k * NA + a], acc[k]);
@@ -469,7 +491,7 @@ __global__ void __launch_bounds__(UZT, 1) k_uz(const __grid_constant__ CUtensorM
     const double s0 = A.xd ? double(G.x_0) : double(G.y_0);
     auto plane_par = [&](int p) { return (s0 + p * double(G.T_x)) * sign; };
     const double e0 = ((double(G.u1_0) + (row0 - 0.5) * Tu1) - double(G.z_0)) / Tz + 0.5;
-    auto slope = [&](int i) { return double(ffma(float(i), G.T_v1, G.v1_0)) / Tz; };
+    auto slope = [&](int i) { return (double(G.v1_0) + i * double(G.T_v1)) / Tz; };
     const double va = slope(v1c), vb = slope(v1e - 1);
     auto first_row = [&](int p) {
         const double t = plane_par(p);
@@ -694,7 +716,7 @@ int project_usplit(const petl_geom& G, const float* f, float* g, const ViewRange
         note_launch();
     }
     const int xzb = NA <= GXZ_AXIS ? GXZ : GXZ_LONG;
-    auto kx = xzb == GXZ ? k_gx<GXZ> : k_gx<GXZ_LONG>;
+    auto kx = xzb == GXZ ? k_gx<GXZ, true> : k_gx<GXZ_LONG, true>;
     const size_t xsmem = size_t(xzb) * NA * 4;
     const int ni = int(std::floor(rho));
     auto kz = ni == 0 ? k_uz<0> : ni == 1 ? k_uz<1> : ni == 2 ? k_uz<2> : ni == 3 ? k_uz<3> : k_uz<-1>;
@@ -808,7 +830,7 @@ int project_gsplit(const petl_geom& G, const float* f, float* g, const ViewRange
     }
     const int NAmax = any_xd ? std::max(G.numX, G.numY) : G.numX;
     const int xzb = NAmax <= GXZ_AXIS ? GXZ : GXZ_LONG;
-    auto kx = xzb == GXZ ? k_gx<GXZ> : k_gx<GXZ_LONG>;
+    auto kx = xzb == GXZ ? k_gx<GXZ, false> : k_gx<GXZ_LONG, false>;
     const size_t xsmem = size_t(xzb) * NAmax * 4;
     e = cudaFuncSetAttribute(kx, cudaFuncAttributeMaxDynamicSharedMemorySize, int(xsmem));
     // one z launch shape: its argument block, tensor map (boxes of 32
