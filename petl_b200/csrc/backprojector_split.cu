@@ -174,6 +174,8 @@ __global__ void __launch_bounds__(256) k_gather_records(const ZgatherArgs A, int
             const Shift zs = A.T.zt[size_t(v1) * NY + y];
             const int o = dmx - zs.d;
             bad |= o > kZSpread;
+            // four planes: neighbours a row apart at most, else no unrolled form has the pattern
+            if (NV == 4 && u > 0) bad |= abs(zs.d - A.T.zt[size_t(v1) * NY + min(yq - 1, NY - 1)].d) > 1;
             offs |= uint32_t(min(o, kZSpread)) << (2 * u);
             if (w < A.pg) R->w[q * NV + u] = zs.w;
             if (yq >= NY) continue;
@@ -775,12 +777,11 @@ int backproject_split_m(const petl_geom& G, const Members& M0, int mode, int acc
     if (G.N_u0 > XMAXN || G.numY > 65535 || G.numZ > 65535 * XR) return kNotApplicable;
     if (size_t(G.numY) * nb > 65535) return kNotApplicable;  // k_bwd_xgather grid.z
     if (std::max(G.numZ, G.N_u1) > GMAXROWS) return kNotApplicable;
-    const double step = double(std::max(std::fabs(G.v1_0), std::fabs(G.v1_0 + (G.N_v1 - 1) * G.T_v1))) *
-                        double(G.T_x) / double(G.T_z);  // shift change per plane
-    // four planes share a window of 16 rows where their shifts differ by at
-    // most three rows (shifts below one row per plane), else two planes a
-    // window of 28 rows, as in the forward
-    const int NV = shift_spread(3, step) <= kZSpread ? 4 : 2, NK = NV == 4 ? 12 : 24;
+    const ShiftStep step = plane_step(G);
+    // four planes share a window of 16 rows where their shifts move by less
+    // than a row per plane, else two planes a window of 28 rows, as in the
+    // forward
+    const int NV = four_per_window(step) ? 4 : 2, NK = NV == 4 ? 12 : 24;
     if (shift_spread(NV - 1, step) > kZSpread) return kNotApplicable;
     int* err = device_error_ptr();
     if (!err) return kNotApplicable;

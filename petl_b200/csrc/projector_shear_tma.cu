@@ -871,7 +871,7 @@ int project_tma_t(const petl_geom& G, const TF* f, TG* g, const ViewRange& vr, c
     // volume rows a multiple of 16 bytes (TMA strides), 16-byte aligned base
     if ((G.numX * EB) % 16 != 0 || (reinterpret_cast<uintptr_t>(f) & 15) != 0 || G.numY > 4096)
         return kNotApplicable;
-    const double step = double(G.T_v1) * plane_ymax(G) / double(G.T_z);  // shift change per slope
+    const ShiftStep step = slope_step(G);
     if (shift_spread(FV - 1, step) > FDMAX) return kNotApplicable;
     const int nrb = FROWS + shift_spread(FSL - 1, step) + 1;
     if (nrb > 256) return kNotApplicable;
@@ -930,8 +930,7 @@ int backproject_tma_t(const petl_geom& G, const TG* g, TF* f, int mode, int accu
     const int pg = std::max(NU0, G.numX) <= 256 ? 2 : 1;
     const int np = BPT * pg;
     if (vr.iv1_end - vr.iv1_begin > BV1CAP) return kNotApplicable;
-    const double step = double(std::max(std::fabs(G.v1_0), std::fabs(G.v1_0 + (G.N_v1 - 1) * G.T_v1))) *
-                        double(G.T_x) / double(G.T_z);  // shift change per plane
+    const ShiftStep step = plane_step(G);
     if (shift_spread(BPT - 1, step) > BDW) return kNotApplicable;
     const int brb = BWN + shift_spread(np - 1, step);
     if (brb > 254) return kNotApplicable;

@@ -153,6 +153,8 @@ __device__ void z_records(const XshiftArgs& A, int y)
             for (int j = j0; j < j1; j++) {
                 const Shift zs = A.T.zt[size_t(j) * NY + y];
                 if (zs.d - base > kZSpread) bad = true;
+                // four slopes: neighbours a row apart at most, else no unrolled form has the pattern
+                if (nv == 4 && j > j0 && abs(zs.d - A.T.zt[size_t(j - 1) * NY + y].d) > 1) bad = true;
                 code |= uint32_t(min(zs.d - base, kZSpread)) << (2 * (j - j0));
                 R->w[q * nv + j - j0] = zs.w;
             }
@@ -439,7 +441,7 @@ k_fwd_zsum(const __grid_constant__ ZMaps maps, const __grid_constant__ ZsumArgs 
                                 PETL_ZCASE(0x00) PETL_ZCASE(0x40) PETL_ZCASE(0x50) PETL_ZCASE(0x90) PETL_ZCASE(0x54)
                                 PETL_ZCASE(0x94) PETL_ZCASE(0xA4) PETL_ZCASE(0xE4) PETL_ZCASE(0x01) PETL_ZCASE(0x05)
                                 PETL_ZCASE(0x15) PETL_ZCASE(0x06) PETL_ZCASE(0x16) PETL_ZCASE(0x1A) PETL_ZCASE(0x1B)
-                                default: next(0x100u);  // no such pattern: a layout error, reported
+                                default: next(0x100u);  // no such pattern: z_records reported a layout error
                             }
                         } else {
                             switch (code & 0xffu) {
@@ -550,7 +552,7 @@ struct ZPlan {
     size_t table_bytes;
 };
 
-bool zsum_plan(const petl_geom& G, const ViewRange& vr, double step, int nslot, ZPlan& P)
+bool zsum_plan(const petl_geom& G, const ViewRange& vr, const ShiftStep& step, int nslot, ZPlan& P)
 {
     ZsumArgs& A = P.A;
     A = ZsumArgs{};
@@ -559,13 +561,13 @@ bool zsum_plan(const petl_geom& G, const ViewRange& vr, double step, int nslot, 
     A.nslot = nslot;
     A.n_colblk = int(ceil_div(G.N_u0, kZCols));
     A.wait_limit = wait_limit();
-    // four slopes share a window of 16 rows where their shifts differ by at
-    // most three rows (steps below one row per slope); steeper slopes (a volume
+    // four slopes share a window of 16 rows where their shifts move by less
+    // than a row per slope; steeper slopes (a volume
     // that reaches beyond the panels) take two per warp and a window of 28
     // rows, whose loads then bound them; steps of three rows and more are left
     // to the first-generation kernel.  192x192x96 at 1.1 to 1.4 rows per
     // slope: 3.3 ms for 67 views here, 6.0 on the first-generation kernel
-    P.nv = shift_spread(3, step) <= kZSpread ? 4 : 2;
+    P.nv = four_per_window(step) ? 4 : 2;
     P.nk = P.nv == 4 ? 12 : 24;
     if (shift_spread(P.nv - 1, step) > kZSpread) return false;
     const int nv1 = vr.iv1_end - vr.iv1_begin;
@@ -669,8 +671,7 @@ int project_split_m(const petl_geom& G, const Members& M0, const ViewRange& vr, 
     // about ten slopes the single-pass kernel is cheaper than that round trip
     if (nv1 < kSplitMinSlopes) return kNotApplicable;
     if (std::max(G.numZ, G.N_u1) > ZMAXROWS) return kNotApplicable;
-    const double step = double(G.T_v1) * plane_ymax(G) / double(G.T_z);  // shift change per slope
-    if (!(step * std::max(G.N_v1, 1) < ZMAXROWS)) return kNotApplicable;
+    const ShiftStep step = slope_step(G);
     int* err = device_error_ptr();
     if (!err) return kNotApplicable;
 

@@ -71,16 +71,52 @@ struct TableBuf {
 
 int make_tables(const petl_geom& G, TableBuf& tb, cudaStream_t st);
 
-// Largest |y| of the volume's plane centres.
+// Largest |y| of the volume's plane centres, largest |v1| of the slopes.
 inline double plane_ymax(const petl_geom& G)
 {
     return std::fmax(std::fabs(double(G.y_0)), std::fabs(double(G.y_0) + (G.numY - 1) * double(G.T_x)));
 }
+inline double slope_vmax(const petl_geom& G)
+{
+    return std::fmax(std::fabs(double(G.v1_0)), std::fabs(double(G.v1_0) + (G.N_v1 - 1) * double(G.T_v1)));
+}
+
+// How far the tabulated z shifts move, in rows: per slope (on the outermost
+// plane) or per plane (of the steepest slope) in exact arithmetic, and what
+// the tables add to a difference of two shifts: y v1 / T_z is formed from
+// floats, each 2^-24 of itself off at most (together 2.4e-6 .. 1.2e-5 rows where the
+// largest shift is 20 .. 100 rows), the rest in double.
+struct ShiftStep {
+    double step, slack;
+};
+inline double shift_slack(const petl_geom& G)
+{
+    return plane_ymax(G) * slope_vmax(G) / double(G.T_z) * (1.0 / (1 << 23)) + 1e-9;
+}
+inline ShiftStep slope_step(const petl_geom& G)
+{
+    return {std::fabs(double(G.T_v1)) * plane_ymax(G) / double(G.T_z), shift_slack(G)};
+}
+inline ShiftStep plane_step(const petl_geom& G)
+{
+    return {slope_vmax(G) * double(G.T_x) / double(G.T_z), shift_slack(G)};
+}
 
 // Upper bound on the difference of the integer z shifts of slopes (or planes)
-// n steps apart: the exact shifts differ by at most n * step, their floors by
-// at most floor(n * step) + 1 (with a relative margin for the float inputs).
-inline int shift_spread(int n, double step) { return int(std::floor(double(n) * step * (1.0 + 1e-6))) + 1; }
+// n steps apart: the tabulated shifts differ by at most n * step + slack (with
+// a relative margin for the rounding that they share), their floors by at most
+// the floor of that + 1.
+inline int shift_spread(int n, const ShiftStep& s)
+{
+    const double x = double(n) * s.step * (1.0 + 1e-6) + s.slack;
+    return x < double(1 << 29) ? int(std::floor(x)) + 1 : 1 << 29;
+}
+
+// Whether four neighbouring slopes (planes) fit one window of the split z
+// kernels: shifts of neighbours at most one row apart, so that the four
+// window offsets form one of the 15 patterns the kernels unroll, and of all
+// four at most three.
+inline bool four_per_window(const ShiftStep& s) { return shift_spread(1, s) <= 1 && shift_spread(3, s) <= 3; }
 
 // Bytes of FP32 scratch one split projection call may hold (its chunk of
 // views): PETL_SPLIT_SCRATCH_MB, else 5 GiB, at most an eighth of the

@@ -71,3 +71,47 @@ def test_flat_backprojection_shapes(cuda, nx, nz, acc):
         lib().petl_set_dispatch(0)
     for a, b in zip(out[0], out[3]):
         assert torch.equal(a, b)
+
+
+# Shift steps a rounding error below one row: the exact steps differ by less
+# than a row, the tabulated shifts (v1 and y are floats) by two in places.
+NEAR_ONE_ROW = {
+    # slopes 8..11 on plane 0: -116, -116, -115, -113
+    "slopes": ((0.0, 214.36044311523438, 18.4, 180.48056, 0.92, 0.02, 0.7152043),
+               (24, 234, 114, 0.92, 0.92, 0.0, 0.0, 0.00013313642136), None),
+    # planes 20..23 of slope 0: -296, -295, -295, -293
+    "planes": ((0.0, 167.48048400878906, 15.8, 385.2051086425781, 0.79, 0.02, 1.0),
+               (24, 208, 60, 0.79, 0.79, 0.0, 0.0, -0.3948222875649961), (0, 64)),
+}
+
+
+@pytest.mark.parametrize("name", list(NEAR_ONE_ROW))
+def test_shift_steps_near_one_row(cuda, name):
+    """Every plane and slope counts where neighbouring shifts differ by two
+    rows although their step is below one: bit equality with dispatch 3 for
+    the forward; the backward there takes the first-generation kernel, whose
+    sums of at most 64 x 5 terms in another order differ by rounding."""
+    import torch
+    from petl_b200 import Geometry, lib, ops
+    args, vol, rng = NEAR_ONE_ROW[name]
+    G = Geometry(*args, volume=vol)
+    gen = torch.Generator(device=cuda).manual_seed(11)
+    f = torch.rand(G.vol_shape, device=cuda, generator=gen)
+    g = torch.rand(G.shape, device=cuda, generator=gen)
+    L = lib()
+    out = {}
+    try:
+        for d in (0, 3):
+            assert L.petl_set_dispatch(d) == 0
+            n = L.petl_launch_count()
+            x = ops.project(G, f, torch.zeros(G.shape, device=cuda), v1_range=rng)
+            n1 = L.petl_launch_count()
+            out[d] = (n1 - n, x, [ops.backproject(G, g, v1_range=rng, mode=m) for m in ("reference", "adjoint")])
+    finally:
+        L.petl_set_dispatch(0)
+    torch.cuda.synchronize()
+    assert L.petl_device_error_flag() == 0
+    assert out[0][0] == out[3][0] + 1  # the split forward ran: two passes
+    assert torch.equal(out[0][1], out[3][1])
+    for a, b in zip(out[0][2], out[3][2]):
+        assert float((a - b).norm() / b.norm()) < 1e-6

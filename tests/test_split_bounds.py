@@ -14,7 +14,11 @@ backprojector's voxel extents, src/projectors.cu:318-345):
   inside;
 * the z passes (k_gz, k_gzT) stage per plane or slope the rows their tile
   needs from a host bound on the spread of the per-column shifts: over a
-  sweep of further geometries the actual spread stays within it."""
+  sweep of further geometries the actual spread stays within it;
+* the split kernels on the axes (k_fwd_zsum, k_bwd_zgather) sum four slopes
+  (planes) per warp only where the tabulated shifts of neighbours differ by
+  at most a row, and stage rows for a bound on the spread of n + 1 of them:
+  both hold for steps of shifts up to a rounding error below a whole row."""
 import math
 
 import numpy as np
@@ -191,3 +195,62 @@ def test_z_pass_staged_rows_hold_the_shift_spread(i):
                 fl = np.floor(nc)
                 spread = fl.max(axis=(0, 1)) - fl.min(axis=(0, 1))
                 assert float(spread.max()) <= math.ceil(bound_adj) + 1
+
+
+def _shifts(F):
+    """The z shifts as the tables hold them (v1 and y rounded to float once,
+    the rest in double): [slope][plane]."""
+    f32, f64 = np.float32, np.float64
+    v1 = f32(np.arange(F["N_v1"]) * f64(F["T_v1"]) + f64(F["v1_0"])).astype(f64)
+    y = f32(np.arange(F["numY"]) * f64(F["T_x"]) + f64(F["y_0"])).astype(f64)
+    m = -((f64(F["z_0"]) + y[None, :] * v1[:, None]) - f64(F["u1_0"])) / f64(F["T_u1"])
+    return np.floor(m).astype(np.int64)
+
+
+def _shift_rule(F):
+    """The host's bounds: slack, and per slope (axis 0) and plane (axis 1) the
+    step, whether four share a window, and the spread of n steps."""
+    ymax = max(abs(F["y_0"]), abs(F["y_0"] + (F["numY"] - 1) * F["T_x"]))
+    vmax = max(abs(F["v1_0"]), abs(F["v1_0"] + (F["N_v1"] - 1) * F["T_v1"]))
+    slack = ymax * vmax / F["T_z"] / (1 << 23) + 1e-9
+    out = []
+    for step in (F["T_v1"] * ymax / F["T_z"], vmax * F["T_x"] / F["T_z"]):
+        spread = lambda n, s=step: math.floor(n * s * (1 + 1e-6) + slack) + 1  # noqa: E731
+        out.append((step, spread(1) <= 1 and spread(3) <= 3, spread))
+    return out
+
+
+def test_four_per_window_only_where_neighbours_differ_by_a_row():
+    from petl_b200 import Geometry
+    rng = np.random.default_rng(3)
+    near = [1.0, 1.0 / 3.0, 0.2, 2.0 / 3.0, 2.0, 3.0]  # steps whose multiples are whole rows
+    four = two = close = 0
+    for it in range(600):
+        T = round(float(rng.uniform(0.5, 1.9)), 2)
+        axis = it % 2
+        step = near[it % len(near)] * (1 - 10.0 ** rng.uniform(-7.0, -4.5))
+        if axis == 0:  # step per slope = ymax / R
+            ny = int(rng.integers(40, 236))
+            R = 0.5 * (ny - 1) * T / step
+            v = float(rng.uniform(0.4, 1.0))
+        else:          # step per plane = the steepest slope, a whole number of bins over R
+            ny = int(rng.integers(20, 120)) * 2
+            k = int(rng.integers(20, 118))
+            R, v = k * T / step, step * (1 + 1e-6)
+        vol = (8, ny, 16, T, T, 0.0, 0.0, float(rng.uniform(-1.0, 1.0)) * T)
+        P = Geometry(0.0, 2.0 * R, 8.0 * T, 2.0 * R * (v + 0.3), T, 0.02, v, volume=vol).g
+        F = {k_: getattr(P, k_) for k_, _ in P._fields_}
+        d = _shifts(F)
+        for ax, (st, is_four, spread) in enumerate(_shift_rule(F)):
+            j = int(np.abs(np.diff(d, axis=ax)).max())
+            if is_four:
+                assert j <= 1, (T, ny, R, st)
+                four += 1
+            else:
+                two += 1
+            close += not is_four and st < 1
+            for n in (1, 3, 11, 15):
+                if d.shape[ax] > n:
+                    a = np.swapaxes(d, 0, ax)
+                    assert int(np.abs(a[n:] - a[:-n]).max()) <= spread(n), (T, ny, R, st, n)
+    assert four > 300 and two > 300 and close > 50
