@@ -70,6 +70,7 @@ struct FwdTmaArgs {
     int nf;        // raw-row buffers in the copy ring
     int fstride;   // bytes per raw buffer
     int xstride;   // floats per interpolated buffer
+    int pairs;     // the planograms take column-pair accesses (pair_access)
     Tables T;
     int* err;
     unsigned wait_limit;  // bound of the waits on staged data (wait_limit(): kWaitLimit or 0)
@@ -316,7 +317,6 @@ k_fwd_tma(const __grid_constant__ CUtensorMap fmap, TG* __restrict__ g, const TG
 
     // epilogue: scale, ray masks, optional MLEM ratio
     const int colA = col0 + 2 * lane;
-    const bool pairs = (G.N_u0 & 1) == 0;  // float2 accesses stay 8-byte aligned
 #pragma unroll
     for (int j = 0; j < FV; j++) {
         const int v1 = v1a + jw + j;
@@ -332,7 +332,7 @@ k_fwd_tma(const __grid_constant__ CUtensorMap fmap, TG* __restrict__ g, const TG
             const bool v0ok = rv && colA >= ub0.x && colA <= ub0.y;
             const bool v1ok = rv && colA + 1 >= ub0.x && colA + 1 <= ub0.y;
             float2 val = make_float2(v0ok ? acc[j][k].x * S : 0.0f, v1ok ? acc[j][k].y * S : 0.0f);
-            if (pairs && colA + 1 < G.N_u0) {
+            if (A.pairs && colA + 1 < G.N_u0) {
                 if (meas) {
                     const float2 m = Store<TG>::ld2(meas + o);
                     val = make_float2(ratio_rule(m.x, val.x), ratio_rule(m.y, val.y));
@@ -887,6 +887,7 @@ int project_tma_t(const petl_geom& G, const TF* f, TG* g, const ViewRange& vr, c
     A.G = G;
     A.vr = vr;
     A.n_colblk = int(ceil_div(G.N_u0, FCOLS));
+    A.pairs = pair_access<TG>(G, g, meas);
     A.nrb = nrb;
     A.fstride = (nrb * FBOXW * EB + 127) & ~127;
     A.xstride = (nrb + FDMAX) * FCOLS;

@@ -100,6 +100,7 @@ struct ZsumArgs {
     int ns;         // ring stages
     int stage;      // bytes per stage (planes, then their records)
     int rec_off;    // the records' offset in a stage
+    int pairs;      // the planograms take column-pair accesses (pair_access)
     ZKind k[2];     // full blocks, and the tail of at most half a block
     ZRec* rec;      // [block][plane]
     int* dz;        // [block][plane] smallest shift of the block
@@ -476,7 +477,6 @@ k_fwd_zsum(const __grid_constant__ ZMaps maps, const __grid_constant__ ZsumArgs 
             const int2 ub0 = A.T.ub0[iv0];
             const int colA = in.col0 + 2 * lane;
             const int row1 = min(row0 + NK, G.N_u1);
-            const bool pairs = (G.N_u0 & 1) == 0;  // float2 accesses stay 8-byte aligned
             const bool ok0 = colA >= ub0.x && colA <= ub0.y, ok1 = colA + 1 >= ub0.x && colA + 1 <= ub0.y;
             f2x* out = ctl->out[warp][0] + lane;
 #pragma unroll 1
@@ -489,7 +489,7 @@ k_fwd_zsum(const __grid_constant__ ZMaps maps, const __grid_constant__ ZsumArgs 
                 const size_t o0 = (size_t(v1) * G.N_v0 + iv0) * G.N_u1 * G.N_u0;
 #pragma unroll 1
                 for (int kk = 0; kk < kZOut; kk += 4) {
-                    if (pairs && colA + 1 < G.N_u0) {
+                    if (A.pairs && colA + 1 < G.N_u0) {
                         float2 m[4];
                         if (meas)
 #pragma unroll
@@ -506,7 +506,7 @@ k_fwd_zsum(const __grid_constant__ ZMaps maps, const __grid_constant__ ZsumArgs 
                             if (meas) val = make_float2(ratio_rule(m[k].x, val.x), ratio_rule(m[k].y, val.y));
                             Store<TG>::st2(g + o0 + size_t(iu1) * G.N_u0 + colA, val);
                         }
-                    } else {  // odd rows, or the row's last column
+                    } else {  // no pairs, or the row's last column
 #pragma unroll 1
                         for (int k = kk; k < min(kk + 4, G.N_u1 - r0); k++) {
                             const bool rv = r0 + k >= u1r.x && r0 + k <= u1r.y;
@@ -704,6 +704,9 @@ int project_split_m(const petl_geom& G, const Members& M0, const ViewRange& vr, 
     ZsumArgs& A = P.A;
     A.T = T;
     A.err = err;
+    A.pairs = 1;
+    for (int b = 0; b < nb; b++)
+        if (!pair_access<TG>(G, M0.out[b], M0.meas[b])) A.pairs = 0;
     A.rec = reinterpret_cast<ZRec*>(reinterpret_cast<unsigned char*>(X) + x_bytes);
     A.dz = reinterpret_cast<int*>(A.rec + size_t(A.k[0].nblk + A.k[1].nblk) * G.numY);
     A.next = A.dz + size_t(A.k[0].nblk + A.k[1].nblk) * G.numY;

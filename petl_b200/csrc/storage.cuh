@@ -7,6 +7,7 @@
 
 #include <cstdint>
 
+#include "common.cuh"
 #include "tma.cuh"
 
 namespace petl {
@@ -39,6 +40,17 @@ struct Store<__nv_bfloat16> {
         *reinterpret_cast<__nv_bfloat162*>(p) = __float22bfloat162_rn(v);
     }
 };
+
+// Host: whether a planogram's column pairs are naturally aligned: rows of an
+// even number of columns from a base aligned to a pair, for the planogram that
+// a forward kernel writes and the measured one that it reads (or null).  A
+// contiguous tensor may start at any element of its allocation.
+template <class T>
+inline bool pair_access(const petl_geom& G, const void* out, const void* meas)
+{
+    const uintptr_t p = reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(meas);
+    return G.N_u0 % 2 == 0 && p % (2 * sizeof(T)) == 0;
+}
 
 // Two scalar FMAs on a column pair (the single-pass kernels).
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
