@@ -588,14 +588,23 @@ bool zsum_plan(const petl_geom& G, const ViewRange& vr, const ShiftStep& step, i
             K.v1_first = i ? v1_split : vr.iv1_begin;
             K.v1_end = i ? vr.iv1_end : v1_split;
             K.sg = i ? std::max(tail_sg, 1) : sg;
-            K.rg = std::min(A.nw / K.sg, int(ceil_div(G.N_u1, P.nk)));
-            K.rows = P.nk * K.rg;
             K.nblk = int(ceil_div(K.v1_end - K.v1_first, P.nv * K.sg));
+            // staged rows: the tile's, the spread of the block's shifts and
+            // the second tap's.  They fit a TMA box and, with the window's
+            // margin, the 8 bits of a window row: a tail of one group of two
+            // slopes on a tall panel takes fewer warps (192x192x128, 256 rows,
+            // 79 views, 1.2 rows per slope: 72 slopes 5.9 ms and 74 slopes 6.4
+            // here, 18.8 and 19.0 on the first-generation kernel)
+            const int extra = shift_spread(P.nv * K.sg - 1, step) + 1;
+            K.rg = std::min(A.nw / K.sg, int(ceil_div(G.N_u1, P.nk)));
+            K.rg = std::min(K.rg, (256 - kZSpread - extra) / P.nk);
+            if (K.rg < 1 && K.nblk == 0) K.rg = 1;  // no such blocks
+            if (K.rg < 1) return false;
+            K.rows = P.nk * K.rg;
             K.n_rowblk = int(ceil_div(G.N_u1, K.rows));
-            K.nrb = K.rows + shift_spread(P.nv * K.sg - 1, step) + 1;
+            K.nrb = K.rows + extra;
             K.pstride = (K.nrb + kZSpread) * kZCols;
             K.blk0 = i ? A.k[0].nblk : 0;
-            if (K.nrb > 256 - kZSpread) return false;  // TMA box rows; the window row fits 8 bits
             const long long nt = (long long)nslot * K.nblk * K.n_rowblk * A.n_colblk;
             if (nt > (1 << 30)) return false;
             K.ntile = int(nt);

@@ -115,3 +115,32 @@ def test_shift_steps_near_one_row(cuda, name):
     assert torch.equal(out[0][1], out[3][1])
     for a, b in zip(out[0][2], out[3][2]):
         assert float((a - b).norm() / b.norm()) < 1e-6
+
+
+@pytest.mark.parametrize("slopes", [72, 74])
+@pytest.mark.parametrize("rows", [250, 320])
+def test_steep_slopes_on_tall_panels(cuda, slopes, rows):
+    """1.2 rows per slope on planograms of more than 240 rows, without a tail
+    of slopes (72) and with one of a single group (74): the split forward
+    takes both, equal to the single-pass or first-generation form."""
+    import torch
+    from petl_b200 import Geometry, lib, ops
+    # R = 24.6 bins, volume of 60 planes: step = 29.5 / 24.6
+    G = Geometry(0.0, 49.2, 20.0, float(rows), 1.0, 0.2, 1.52, volume=(24, 60, 40, 1.0))
+    assert G.shape[0] >= slopes and G.shape[2] == rows
+    gen = torch.Generator(device=cuda).manual_seed(5)
+    f = torch.rand(G.vol_shape, device=cuda, generator=gen)
+    L = lib()
+    out, launches = {}, {}
+    try:
+        for d in (0, 3):
+            assert L.petl_set_dispatch(d) == 0
+            n = L.petl_launch_count()
+            out[d] = ops.project(G, f, torch.full(G.shape, 7.0, device=cuda), v1_range=(0, slopes))
+            launches[d] = L.petl_launch_count() - n
+    finally:
+        L.petl_set_dispatch(0)
+    torch.cuda.synchronize()
+    assert L.petl_device_error_flag() == 0
+    assert launches[0] == launches[3] + 1  # the split forward ran: two passes
+    assert torch.equal(out[0], out[3])
