@@ -184,6 +184,13 @@ int backproject_range(const petl_geom& G, const float* g, float* f, int mode, in
             note_path(3);
             return rc;
         }
+        if (mode == PETL_BP_ADJOINT) {
+            const int ru = backproject_usplit_adjoint(G, g, f, accumulate, scale, vr, st);
+            if (ru != -2) {
+                note_path(0);  // one gather over the rays, as the general kernel
+                return ru;
+            }
+        }
     }
     note_path(0);
     return launch_backproject_general(G, g, f, mode, accumulate, scale, vr, st);

@@ -6,8 +6,10 @@
 // (95-101 / 150-156) and the box-overlap footprint weights (110-119 /
 // 165-174).  Two deliberate differences: the in-plane coordinate of a tap is
 // formed directly from its index instead of by running addition, and every
-// weight is evaluated with rounding-pinned intrinsics, so the forward
-// projector and its gather-form adjoint compute bit-identical weights.
+// weight is evaluated with rounding-pinned intrinsics, so the general forward
+// projector and its gather-form adjoint compute bit-identical weights.  (On the
+// axes with unequal voxel height and u1 pitch both take their weights from
+// positions in double instead: k_gx, k_uz and k_backproject_uz.)
 #pragma once
 #include "common.cuh"
 
@@ -176,6 +178,10 @@ int project_gsplit(const petl_geom& G, const float* f, float* g, const ViewRange
 // Its exact transpose (backprojector_gsplit.cu, adjoint mode); -2 when the
 // layout rules fail (the caller then runs launch_backproject_general).
 int backproject_gsplit_adjoint(const petl_geom& G, const float* g, float* f, int accumulate, float scale,
+                               const ViewRange& vr, cudaStream_t st);
+// The exact transpose of project_gsplit on the axes with unequal voxel height
+// and u1 pitch (projector_gsplit.cu), with its weights; -2 elsewhere.
+int backproject_usplit_adjoint(const petl_geom& G, const float* g, float* f, int accumulate, float scale,
                                const ViewRange& vr, cudaStream_t st);
 // Backprojection with the reference's semantics for any psi, split into an
 // in-plane pass per (v1, u1) slice and a z pass (backprojector_rsplit.cu);

@@ -56,3 +56,61 @@ def test_unequal_pitch_forward(cuda, name):
     # the ratio where the ray meets more than the rim of a voxel
     ok = out[1][0] > 0.05 * out[1][0].max()
     assert rel_l2(out[0][1][ok].cpu().numpy(), out[1][1][ok].cpu().numpy()) < 1e-5
+
+
+@pytest.mark.parametrize("name", list(CASES))
+def test_unequal_pitch_adjoint_has_the_forward_weights(cuda, name):
+    """Single weights of P and of P^T: the column P e_j of a voxel against the
+    rows P^T e_i of bins along it.  Either side rounds a weight a handful of
+    times (its u0 and u1 part and three factors): 4e-7 of the largest weight.
+    Weights from positions in float differ by up to 1e-5 here."""
+    import torch
+    from petl_b200 import Geometry, lib, ops
+    args, vol, path = CASES[name]
+    G = Geometry(*args, volume=vol)
+    gen = torch.Generator().manual_seed(4)
+    nz, ny, nx = G.vol_shape
+    worst = 0.0
+    for k in range(4):
+        # corners and the middle of the volume
+        j = ((nz // 2, ny // 2, nx // 2), (1, 2, nx - 2), (nz - 2, ny - 1, 3), (nz // 3, 0, nx // 2))[k]
+        f = torch.zeros(G.vol_shape, device=cuda)
+        f[j] = 1.0
+        col = ops.project(G, f)
+        bins = torch.nonzero(col.reshape(-1) > 0.02 * col.max()).reshape(-1).cpu()
+        if len(bins) == 0:
+            continue
+        for i in bins[torch.randint(len(bins), (8,), generator=gen)].tolist():
+            g = torch.zeros(G.shape, device=cuda)
+            g.view(-1)[i] = 1.0
+            row = ops.backproject(G, g, mode="adjoint")
+            worst = max(worst, abs(float(row[j]) - float(col.view(-1)[i])) / float(col.max()))
+    assert lib().petl_device_error_flag() == 0
+    assert worst < 4e-7, worst
+
+
+@pytest.mark.parametrize("name", list(CASES))
+@pytest.mark.parametrize("sub,v1", [(None, None), ((1, 3), (2, -1))])
+def test_unequal_pitch_adjoint_against_oracle(cuda, name, sub, v1):
+    """Voxels of P^T g, with accumulation and scale, against 64 bits: voxel j is
+    <P e_j, g>, with P e_j from the oracle."""
+    import torch
+    from petl_b200 import Geometry, lib, ops
+    args, vol, path = CASES[name]
+    G, Go = Geometry(*args, volume=vol), O.make_geom(*args, vol)
+    rng = np.random.default_rng(6)
+    g = rng.random(G.shape).astype(np.float32)
+    r1 = None if v1 is None else (v1[0], G.shape[0] + v1[1])
+    keep = np.zeros(G.shape, bool)
+    keep[slice(*r1) if r1 else slice(None), slice(sub[0], None, sub[1]) if sub else slice(None)] = True
+    gk = np.where(keep, g, 0.0).astype(np.float64)
+    f0 = torch.ones(G.vol_shape, device=cuda)
+    got = ops.backproject(G, torch.from_numpy(g).to(cuda), f0, mode="adjoint", subset=sub, v1_range=r1,
+                          accumulate=True, scale=0.5).cpu().numpy()
+    assert lib().petl_last_projector_path() == 0 and lib().petl_device_error_flag() == 0
+    nz, ny, nx = G.vol_shape
+    for j in ((nz // 2, ny // 2, nx // 2), (0, 0, 0), (nz - 1, ny - 1, nx - 1), (1, ny // 3, nx - 2), (nz - 2, 1, 2)):
+        e = np.zeros(G.vol_shape, np.float32)
+        e[j] = 1.0
+        want = 1.0 + 0.5 * float((np.asarray(O.project(Go, e)[0], np.float64) * gk).sum())
+        assert abs(float(got[j]) - want) < 1e-5 * want, (j, got[j], want)
