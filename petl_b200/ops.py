@@ -58,9 +58,9 @@ def project(geom, f, g=None, subset=None, v1_range=None):
     which case ``g`` is a list."""
     geoms = as_list(geom)
     if g is None:
-        # a projection of every view and slope writes every bin
-        new = torch.empty if subset is None and v1_range is None else torch.zeros
-        g = [new(G.shape, device=f.device, dtype=torch.float32) for G in geoms]
+        # zeros, although a projection of every view and slope writes every
+        # bin: kernels whose waits give up return without writing
+        g = [torch.zeros(G.shape, device=f.device, dtype=torch.float32) for G in geoms]
     gl = as_list(g)
     first, step = subset if subset is not None else (0, 1)
     for G, gi in zip(geoms, gl):
@@ -216,8 +216,7 @@ def backproject(geom, g, f=None, mode="reference", accumulate=False, scale=1.0, 
 def project_bf16(geom, f, g=None, subset=None, v1_range=None):
     """g = P f with f and g in bfloat16 (one geometry)."""
     if g is None:
-        new = torch.empty if subset is None and v1_range is None else torch.zeros
-        g = new(geom.shape, device=f.device, dtype=torch.bfloat16)
+        g = torch.zeros(geom.shape, device=f.device, dtype=torch.bfloat16)
     first, step = subset if subset is not None else (0, 1)
     b, e = v1_range if v1_range is not None else (0, geom.shape[0])
     check(lib().petl_project_bf16_dev(geom.ptr, _dev16(f, "f"), _dev16(g, "g"), b, e, first, step, _stream()),
