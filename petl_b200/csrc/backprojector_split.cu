@@ -620,26 +620,31 @@ __global__ void __launch_bounds__(256) k_bwd_zflat(const float* __restrict__ g, 
         if (c0 + r < G.N_u0 && z < A.NZc) B[(size_t(vi) * G.N_u0 + c0 + r) * A.NZc + z] = tile[threadIdx.x][r];
 }
 
-// x taps of the flat z sums into the volume.  A warp takes 64 rows z (two per
-// lane, so every tap is a coalesced eight-byte load whatever the shift) of 8
-// neighbouring x on one plane: 9 loads per view for 16 taps.  The eight warps
-// of a block take neighbouring planes, whose taps meet in L1.  With a thread
-// per x the taps cost two four-byte loads each, and FBP's backprojection at
-// 256x256x128 (129 views) was bound by them (0.70 ms).  The operations of
-// k_bwd_xgather in its order.  Grid (ceil(numX / 8), ceil(numY / 8),
-// ceil(numZ / 64)), 256 threads.
-constexpr int FX = 8;    // x per warp
-constexpr int FVB = 32;  // views whose shifts a block stages at a time
-
-template <bool ADJ>
-__global__ void __launch_bounds__(256) k_bwd_flat_gather(const float* __restrict__ B, float* __restrict__ f,
+// x taps of the flat z sums into the volume.  LZ lanes take 2 LZ rows z (two
+// per lane, so every tap is a coalesced eight-byte load whatever the shift) of
+// FX neighbouring x on one plane: FX + 1 loads per view for 2 FX taps.  The
+// block's FW warps take neighbouring planes, whose taps meet in L1, FVB views'
+// shifts staged at a time.  With a thread per x the taps cost two four-byte
+// loads each, and FBP's backprojection at 256x256x128 (129 views) was bound by
+// them (0.70 ms).  The operations of k_bwd_xgather in its order.  Grid
+// (ceil(numX / FX), ceil(numY / FPL), ceil(numZ / (2 LZ))), 32 FW threads.
+//
+// Large volumes: 8 x, 8 planes, 64 rows.  Where such blocks number fewer than
+// the SMs the kernel waits on a view's loads after the other's: 2 x, 8 planes
+// of half a warp each, 32 rows, four views' loads in flight (whole
+// backprojection of 65 views, large shape / this one / a thread per x:
+// 48x48x24 46 / 32 / 41 us, 63x63x28 48 / 32 / 41, 80x80x40 49 / 39 / 43,
+// 96x96x32 47 / 35 / 43; 96x96x96, 288 blocks of the large shape, 56 / 58 / 79).
+template <bool ADJ, int FX, int FW, int LZ, int FVB, int UNROLL>
+__global__ void __launch_bounds__(32 * FW) k_bwd_flat_gather(const float* __restrict__ B, float* __restrict__ f,
                                                         const FlatArgs A)
 {
-    __shared__ XView s_xs[FVB][8];
+    constexpr int FPL = FW * 32 / LZ;  // planes per block
+    __shared__ XView s_xs[FVB][FPL];
     const petl_geom& G = A.G;
     const int NY = G.numY, NZ = G.numZ, NX = G.numX, NU0 = G.N_u0;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int x0 = blockIdx.x * FX, y = blockIdx.y * 8 + warp, z = blockIdx.z * 64 + 2 * lane;
+    const int lane = threadIdx.x % LZ, pl = threadIdx.x / LZ;
+    const int x0 = blockIdx.x * FX, y = blockIdx.y * FPL + pl, z = blockIdx.z * (2 * LZ) + 2 * lane;
     const bool zok = z < A.NZc;
     const f2x* Bz = reinterpret_cast<const f2x*>(B + (zok ? z : 0));
     const int pitch = A.NZc / 2;
@@ -648,11 +653,12 @@ __global__ void __launch_bounds__(256) k_bwd_flat_gather(const float* __restrict
     for (int k = 0; k < FX; k++) acc[k] = 0ull;
     for (int vb = 0; vb < A.nv; vb += FVB) {
         __syncthreads();
-        {
-            const int i = threadIdx.x >> 3, p = threadIdx.x & 7;
+#pragma unroll 4
+        for (int r = 0; r < FVB * FPL / (32 * FW); r++) {  // by four: by eight and one by one ran 7 us slower
+            const int e = r * (32 * FW) + threadIdx.x, i = e / FPL, p = e % FPL;
             const int v0 = A.first + (vb + i) * A.step;
-            if (vb + i < A.nv && blockIdx.y * 8 + p < NY) {
-                const Shift xs = A.T.xt[size_t(v0) * NY + blockIdx.y * 8 + p];
+            if (vb + i < A.nv && blockIdx.y * FPL + p < NY) {
+                const Shift xs = A.T.xt[size_t(v0) * NY + blockIdx.y * FPL + p];
                 const int2 u = ADJ ? A.T.ub0[v0] : make_int2(0, NU0 - 1);
                 s_xs[i][p] = XView{xs.d, xs.w, u.x, max(0, u.y - u.x + 1)};
             }
@@ -660,9 +666,9 @@ __global__ void __launch_bounds__(256) k_bwd_flat_gather(const float* __restrict
         __syncthreads();
         if (y >= NY) continue;
         const int n = min(FVB, A.nv - vb);
-#pragma unroll 2
+#pragma unroll UNROLL
         for (int i = 0; i < n; i++) {
-            const XView xs = s_xs[i][warp];
+            const XView xs = s_xs[i][pl];
             const f2x w1 = f2_dup(xs.w), w0 = f2_dup(1.0f - xs.w);
             const int cb = x0 - xs.d - 1;  // scratch column of tap 1 of x0
             const f2x* Bv = Bz + size_t(vb + i) * NU0 * pitch;
@@ -679,7 +685,7 @@ __global__ void __launch_bounds__(256) k_bwd_flat_gather(const float* __restrict
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         if (z + h >= NZ) break;
-        float v[FX];
+        float v[FX < 4 ? 4 : FX];
 #pragma unroll
         for (int k = 0; k < FX; k++) {
             const float2 a = f2_unpack(acc[k]);
@@ -688,7 +694,7 @@ __global__ void __launch_bounds__(256) k_bwd_flat_gather(const float* __restrict
         float* row = f + (size_t(z + h) * NY + y) * NX + x0;
 #pragma unroll
         for (int k = 0; k < FX; k += 4) {
-            if (quads && x0 + k + 4 <= NX) {
+            if (FX % 4 == 0 && quads && x0 + k + 4 <= NX) {
                 float4* o = reinterpret_cast<float4*>(row + k);
                 if (A.accumulate) {
                     const float4 p = *o;
@@ -699,7 +705,7 @@ __global__ void __launch_bounds__(256) k_bwd_flat_gather(const float* __restrict
                 }
             } else {
 #pragma unroll
-                for (int i = k; i < k + 4; i++)
+                for (int i = k; i < (k + 4 < FX ? k + 4 : FX); i++)
                     if (x0 + i < NX) row[i] = A.accumulate ? fmaf(A.scale, v[i], row[i]) : A.scale * v[i];
             }
         }
@@ -719,14 +725,15 @@ int backproject_flat(const petl_geom& G, const float* g, float* f, int mode, int
     }
     const FlatArgs FA{G, vr.iv1_begin, vr.iv0_first, vr.iv0_step, n_v0, NZc, accumulate, scale, T};
     const dim3 grid(ceil_div(G.N_u0, 32), ceil_div(NZc, 32), unsigned(n_v0));
-    const dim3 ggrid(ceil_div(G.numX, FX), ceil_div(G.numY, 8), ceil_div(G.numZ, 64));
-    if (mode == PETL_BP_ADJOINT) {
-        k_bwd_zflat<true><<<grid, dim3(32, 8), 0, st>>>(g, B, FA);
-        k_bwd_flat_gather<true><<<ggrid, 256, 0, st>>>(B, f, FA);
-    } else {
-        k_bwd_zflat<false><<<grid, dim3(32, 8), 0, st>>>(g, B, FA);
-        k_bwd_flat_gather<false><<<ggrid, 256, 0, st>>>(B, f, FA);
-    }
+    const bool adj = mode == PETL_BP_ADJOINT;
+    const bool small = (long long)ceil_div(G.numX, 8) * ceil_div(G.numY, 8) * ceil_div(G.numZ, 64) < sm_count();
+    const dim3 ggrid = small ? dim3(ceil_div(G.numX, 2), ceil_div(G.numY, 8), ceil_div(G.numZ, 32))
+                             : dim3(ceil_div(G.numX, 8), ceil_div(G.numY, 8), ceil_div(G.numZ, 64));
+    auto kz = adj ? k_bwd_zflat<true> : k_bwd_zflat<false>;
+    auto kg = adj ? (small ? k_bwd_flat_gather<true, 2, 4, 16, 128, 4> : k_bwd_flat_gather<true, 8, 8, 32, 32, 2>)
+                  : (small ? k_bwd_flat_gather<false, 2, 4, 16, 128, 4> : k_bwd_flat_gather<false, 8, 8, 32, 32, 2>);
+    kz<<<grid, dim3(32, 8), 0, st>>>(g, B, FA);
+    kg<<<ggrid, small ? 128 : 256, 0, st>>>(B, f, FA);
     note_launch();
     note_launch();
     const cudaError_t e = cudaGetLastError();

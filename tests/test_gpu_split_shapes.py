@@ -52,10 +52,11 @@ def test_split_shapes_equal_single_pass(cuda, name, sub, v1):
             assert torch.equal(a, b), i
 
 
-@pytest.mark.parametrize("nx,nz,acc", [(64, 32, False), (61, 33, True), (50, 70, False)])
+@pytest.mark.parametrize("nx,nz,acc", [(64, 32, False), (61, 33, True), (50, 70, False), (132, 70, True), (131, 65, False)])
 def test_flat_backprojection_shapes(cuda, nx, nz, acc):
-    """One slope at v1 = 0: ragged x (blocks of 8), z (pairs and blocks of
-    64), accumulation, both modes; bit equality with the single-pass kernel."""
+    """One slope at v1 = 0: ragged x (blocks of 2 and of 8), z (pairs and
+    blocks of 32 and of 64), accumulation, both modes, volumes on either side of
+    the rule for small ones; bit equality with the single-pass kernel."""
     import torch
     from petl_b200 import Geometry, lib, ops
     G = Geometry(0.0, 128.0, 64.0, 1.5 * nz, 1.5, 0.5, 0.25, volume=(nx, 57, nz, 1.5, 1.5, 3.0, 0.0, 0.0)).rebinned()
