@@ -56,7 +56,6 @@ namespace {
 
 constexpr int GPLMAX = 16;          // planes per block at most (a table record holds 16 weights)
 constexpr int GV1MAX = 128;         // slopes per call at most
-constexpr int GMAXROWS = 15000;     // rows of volume and planogram at most
 
 // Table record of one (plane block, row block, slope), staged with the slope:
 // the second tap's weight of each plane; per warp a code word (window offsets,
@@ -783,7 +782,6 @@ int backproject_split_m(const petl_geom& G, const Members& M0, int mode, int acc
     }
     if (G.N_u0 > XMAXN || G.numY > 65535 || G.numZ > 65535 * XR) return kNotApplicable;
     if (size_t(G.numY) * nb > 65535) return kNotApplicable;  // k_bwd_xgather grid.z
-    if (std::max(G.numZ, G.N_u1) > GMAXROWS) return kNotApplicable;
     const ShiftStep step = plane_step(G);
     // four planes share a window of 16 rows where their shifts move by less
     // than a row per plane, else two planes a window of 28 rows, as in the

@@ -64,14 +64,12 @@ namespace shear {
 namespace {
 
 constexpr int ZSLOPES = 16;           // slopes per block at most (a table record holds 16 weights)
-constexpr int ZMAXROWS = 15000;       // rows of volume and planogram at most (16-bit row shifts)
 constexpr int XZB = 8;                // volume rows z per k_xshift block
 constexpr int XMAXNX = 1024;          // longest volume row k_xshift stages
 
 // Table record of one (slope block, plane), staged with the plane: the second
 // tap's weight of each slope, and per slope group (warp) the tap offsets (2
-// bits per slope), the window's first staged row << 8 and the shift of that
-// row << 16.
+// bits per slope) and the window's first staged row << 8.
 struct __align__(16) ZRec {
     float w[ZSLOPES];
     uint32_t code[kZWarps];
@@ -150,7 +148,6 @@ __device__ void z_records(const XshiftArgs& A, int y)
             for (int j = j0; j < j1; j++) base = min(base, A.T.zt[size_t(j) * NY + y].d);
             int xoff = base - dmin;
             bool bad = xoff < 0 || max(da, db) - dmin + K.rows + 1 > K.nrb;
-            code = (uint32_t(uint16_t(int16_t(base))) << 16);
             for (int j = j0; j < j1; j++) {
                 const Shift zs = A.T.zt[size_t(j) * NY + y];
                 if (zs.d - base > kZSpread) bad = true;
@@ -679,7 +676,6 @@ int project_split_m(const petl_geom& G, const Members& M0, const ViewRange& vr, 
     // the x pass writes a volume per view whatever the slope count: below
     // about ten slopes the single-pass kernel is cheaper than that round trip
     if (nv1 < kSplitMinSlopes) return kNotApplicable;
-    if (std::max(G.numZ, G.N_u1) > ZMAXROWS) return kNotApplicable;
     const ShiftStep step = slope_step(G);
     int* err = device_error_ptr();
     if (!err) return kNotApplicable;

@@ -145,3 +145,34 @@ def test_steep_slopes_on_tall_panels(cuda, slopes, rows):
     assert L.petl_device_error_flag() == 0
     assert launches[0] == launches[3] + 1  # the split forward ran: two passes
     assert torch.equal(out[0], out[3])
+
+
+def test_more_rows_than_fifteen_thousand(cuda):
+    """Long thin volumes and panels keep the split kernels (row indexes are
+    plain integers throughout)."""
+    import torch
+    from petl_b200 import Geometry, lib, ops
+    rows = 16400
+    G = Geometry(0.0, 40.0, 4.0, float(rows), 1.0, 0.1, 0.26, volume=(8, 10, rows, 1.0))
+    assert G.shape[2] == rows and G.shape[0] >= 10
+    gen = torch.Generator(device=cuda).manual_seed(9)
+    f = torch.rand(G.vol_shape, device=cuda, generator=gen)
+    g = torch.rand(G.shape, device=cuda, generator=gen)
+    L = lib()
+    out = {}
+    try:
+        for d in (0, 3):
+            assert L.petl_set_dispatch(d) == 0
+            n = [L.petl_launch_count()]
+            x = ops.project(G, f)
+            n.append(L.petl_launch_count())
+            y = ops.backproject(G, g)
+            n.append(L.petl_launch_count())
+            out[d] = (x, y, n[1] - n[0], n[2] - n[1])
+    finally:
+        L.petl_set_dispatch(0)
+    torch.cuda.synchronize()
+    assert L.petl_device_error_flag() == 0
+    assert out[0][2] == out[3][2] + 1 and out[0][3] == out[3][3] + 2  # the split kernels ran
+    assert torch.equal(out[0][0], out[3][0])
+    assert float((out[0][1] - out[3][1]).norm() / out[3][1].norm()) < 1e-6
