@@ -92,3 +92,21 @@ def test_bf16_refuses_non_shear_geometry(cuda):
     f16 = torch.ones(G.vol_shape, device=cuda, dtype=torch.bfloat16)
     with pytest.raises(PetlError, match="axis-aligned"):
         ops.project_bf16(G, f16)
+
+
+def test_bf16_rows_of_any_even_length(cuda):
+    """Planogram rows that are no multiple of 8 elements (staged by column
+    pairs) and slopes steeper than a row: the FP32 kernels on the same values,
+    whose operations and order are the same, rounded once."""
+    import torch
+    from petl_b200 import Geometry, ops
+    for args, vol in (((0.0, 250.0, 48.0, 48.0, 1.5, 0.5, 0.25), (64, 64, 32, 1.5)),  # 114 columns
+                      ((0.0, 60.0, 64.0, 120.0, 2.0, 0.6, 1.6), (36, 58, 40, 2.0))):  # 50 columns, 1.9 rows per slope
+        G = Geometry(*args, volume=vol)
+        assert G.shape[3] % 8 != 0
+        gen = torch.Generator(device=cuda).manual_seed(2)
+        f = torch.rand(G.vol_shape, device=cuda, generator=gen).bfloat16()
+        g = torch.rand(G.shape, device=cuda, generator=gen).bfloat16()
+        assert torch.equal(ops.project_bf16(G, f), ops.project(G, f.float()).bfloat16())
+        for m in ("reference", "adjoint"):
+            assert torch.equal(ops.backproject_bf16(G, g, mode=m), ops.backproject(G, g.float(), mode=m))

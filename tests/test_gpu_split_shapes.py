@@ -1,6 +1,9 @@
 """The split z kernels' launch shapes against the single-pass and
 first-generation shear kernels (dispatch 3), which do the same float
-operations in the same order: bit equality is the bound.  The cases sit where
+operations in the same order: bit equality is the bound.  The launch counts
+show that the split kernels ran (an x pass beside the z pass, and a record
+kernel in the backward, that the others do not have); which launch shape each
+case takes is in tests/test_split_bounds.py.  The cases sit where
 a shape or a rule changes: slopes steeper than one row per plane or slope
 (two per warp), planogram rows that are no multiple of 16 bytes (staged by
 column pairs), few tiles (four consumer warps), slope tails of one group,
@@ -14,8 +17,10 @@ CASES = {
     # psi, D, L, H, T, v_m0, v_m1 ; volume
     "tail1_u0mod2": ((0.0, 250.0, 48.0, 48.0, 1.5, 0.5, 0.25), (64, 64, 32, 1.5)),          # (33, 83, 32, 114)
     "steep_slopes": ((0.0, 100.0, 72.0, 72.0, 1.5, 0.5, 0.25), (96, 96, 48, 1.5)),          # 1.4 rows per slope
-    "steep_planes": ((0.0, 60.0, 60.0, 90.0, 2.0, 0.6, 1.0), (40, 36, 45, 2.0)),            # v1 up to 1 row per plane
-    "tall_voxels": ((0.0, 120.0, 60.0, 60.0, 2.0, 0.6, 0.5), (60, 130, 30, 2.0)),           # steep, 65-column rows
+    "steep_planes": ((0.0, 60.0, 60.0, 90.0, 2.0, 0.6, 1.0), (40, 36, 45, 2.0)),            # 0.93 rows per plane
+    "steeper_planes": ((0.0, 60.0, 60.0, 120.0, 2.0, 0.6, 1.6), (40, 60, 100, 2.0)),        # 1.6 rows per plane
+    "steepest_planes": ((0.0, 60.0, 64.0, 190.0, 2.0, 0.6, 2.5), (36, 58, 98, 2.0)),         # 2.5, 50-column rows
+    "tall_voxels": ((0.0, 120.0, 60.0, 60.0, 2.0, 0.6, 0.5), (60, 130, 30, 2.0)),           # steep, 66-column rows
     "rag90": ((90.0, 115.0, 71.0, 65.0, 1.5, 0.45, 0.2), (75, 71, 38, 1.5, 1.5, 3.0, -4.5, 1.5)),
     "wide": ((0.0, 300.0, 128.0, 32.0, 1.0, 0.5, 0.25), (130, 40, 20, 1.0)),                # 278 columns, volume narrower
     "one_row_block": ((0.0, 128.0, 64.0, 13.0, 1.0, 0.3, 0.1), (30, 34, 11, 1.0, 1.0, 6.0, 0.0, 0.0)),
@@ -33,20 +38,29 @@ def test_split_shapes_equal_single_pass(cuda, name, sub, v1):
     f = torch.rand(G.vol_shape, device=cuda, generator=gen)
     g = torch.rand(G.shape, device=cuda, generator=gen)
     rng = None if v1 is None else (v1[0], G.shape[0] + v1[1])
-    out = {}
+    out, launches = {}, {}
     L = lib()
+
+    def counted(d, fn):
+        n = L.petl_launch_count()
+        out[d].append(fn())
+        launches[d].append(L.petl_launch_count() - n)
+
     try:
         for d in (0, 3):
             assert L.petl_set_dispatch(d) == 0
-            x = ops.project(G, f, torch.full(G.shape, 7.0, device=cuda), subset=sub, v1_range=rng)
-            y = ops.project_ratio(G, f, g, torch.full(G.shape, 7.0, device=cuda), subset=sub, v1_range=rng)
-            out[d] = [x, y] + [ops.backproject(G, g, subset=sub, v1_range=rng, mode=m) for m in ("reference", "adjoint")]
+            out[d], launches[d] = [], []
+            counted(d, lambda: ops.project(G, f, torch.full(G.shape, 7.0, device=cuda), subset=sub, v1_range=rng))
+            counted(d, lambda: ops.project_ratio(G, f, g, torch.full(G.shape, 7.0, device=cuda), subset=sub, v1_range=rng))
+            for m in ("reference", "adjoint"):
+                counted(d, lambda: ops.backproject(G, g, subset=sub, v1_range=rng, mode=m))
     finally:
         L.petl_set_dispatch(0)
     torch.cuda.synchronize()
     assert L.petl_device_error_flag() == 0
+    assert [a - b for a, b in zip(launches[0], launches[3])] == [1, 1, 2, 2]  # the split kernels ran
     for i, (a, b) in enumerate(zip(out[0], out[3])):
-        if name == "steep_planes" and i >= 2:  # dispatch 3 takes the first-generation backprojector: another order
+        if "planes" in name and i >= 2:  # dispatch 3 takes the first-generation backprojector: another order
             assert float((a - b).norm() / b.norm()) < 1e-6
         else:
             assert torch.equal(a, b), i
@@ -63,13 +77,16 @@ def test_flat_backprojection_shapes(cuda, nx, nz, acc):
     gen = torch.Generator(device=cuda).manual_seed(3)
     g = torch.rand(G.shape, device=cuda, generator=gen)
     f0 = torch.rand(G.vol_shape, device=cuda, generator=gen)
-    out = {}
+    out, launches = {}, {}
     try:
         for d in (0, 3):
             lib().petl_set_dispatch(d)
+            n = lib().petl_launch_count()
             out[d] = [ops.backproject(G, g, f0.clone(), mode=m, accumulate=acc, scale=0.7) for m in ("reference", "adjoint")]
+            launches[d] = lib().petl_launch_count() - n
     finally:
         lib().petl_set_dispatch(0)
+    assert launches[0] == launches[3] + 2  # z sums and gather in each
     for a, b in zip(out[0], out[3]):
         assert torch.equal(a, b)
 

@@ -254,3 +254,51 @@ def test_four_per_window_only_where_neighbours_differ_by_a_row():
                     a = np.swapaxes(d, 0, ax)
                     assert int(np.abs(a[n:] - a[:-n]).max()) <= spread(n), (T, ny, R, st, n)
     assert four > 300 and two > 300 and close > 50
+
+
+def _split_form(F, n_views, n_slopes, forward, sms=148):
+    """The launch shape that the host picks on the axes: slopes (planes) per
+    warp, consumer warps, slope groups of the forward's tail."""
+    (_, four_f, _), (_, four_b, _) = _shift_rule(F)
+    cd = lambda a, b: -(-a // b)  # noqa: E731
+    cols = cd(F["N_u0"], 64)
+    nv, nk = (4, 12) if (four_f if forward else four_b) else (2, 24)
+    for nw in (12, 4):
+        groups = 4 if nv == 4 or nw == 4 else 6
+        tail = 0
+        if forward:
+            left = cd(n_slopes, nv) % groups
+            tail = 0 if left == 0 else 1 if left == 1 else groups // 2 if 2 * left <= groups else 0
+            full = cd(n_slopes, nv) // groups if tail else cd(cd(n_slopes, nv), groups)
+            tiles = sum(n * cd(F["N_u1"], nk * min(nw // sg, cd(F["N_u1"], nk)))
+                        for n, sg in ((full, groups), (1 if tail else 0, max(tail, 1)))) * n_views * cols
+        else:
+            tiles = n_views * cols * cd(F["numY"], nv * groups) * cd(F["numZ"], nk * (nw // groups))
+        if tiles >= sms:
+            break
+    return nv, nw, tail
+
+
+def test_split_shape_cases_cover_the_launch_shapes():
+    """tests/test_gpu_split_shapes.py runs every launch shape of the split z
+    kernels: four and two slopes (planes) per warp, twelve and four warps, each
+    with rows that are multiples of 16 bytes and that are not, and tails of
+    one group and of half a block."""
+    from petl_b200 import Geometry
+    from test_gpu_split_shapes import CASES as SHAPES
+    fwd, bwd, tails = set(), set(), set()
+    for args, vol in SHAPES.values():
+        P = Geometry(*args, volume=vol).g
+        F = {k: getattr(P, k) for k, _ in P._fields_}
+        if args[0] == 90.0:  # the kernels see x and y exchanged
+            F["numX"], F["numY"], F["x_0"], F["y_0"] = F["numY"], F["numX"], F["y_0"], \
+                -(F["x_0"] + (F["numX"] - 1) * F["T_x"])
+        for sub, drop in (((0, 1), 0), ((1, 3), 0), ((2, 8), 3)):
+            views = len(range(sub[0], F["N_v0"], sub[1]))
+            nv, nw, tail = _split_form(F, views, F["N_v1"] - drop, True)
+            fwd.add((nv, nw))
+            tails.add((nv, nw, tail))
+            bwd.add(_split_form(F, views, F["N_v1"] - drop, False)[:2] + (F["N_u0"] % 4 == 0,))
+    assert fwd == {(4, 12), (4, 4), (2, 12), (2, 4)}
+    assert bwd == {(nv, nw, a) for nv in (4, 2) for nw in (12, 4) for a in (True, False)}
+    assert {(4, 12, 1), (2, 4, 1), (2, 4, 2), (2, 12, 3)} <= tails
