@@ -258,11 +258,14 @@ int petl_fbp_dev(const petl_geom* G, const float* g, float* f, int accumulate, v
 /* --- BF16 storage ---------------------------------------------------------
  * No reference counterpart (the reference stores float32 only).  Volumes and
  * planograms in bfloat16 (void* = __nv_bfloat16*), footprints accumulated in
- * FP32, results rounded to bfloat16 once.  These run the TMA-staged
- * shear-warp kernels only: axis-aligned planograms with bin pitch equal to
- * the voxel pitch, 16-byte aligned buffers, volume and planogram rows that
- * are multiples of 8 elements, and N_u0, numX <= 256 for the
- * backprojection.  Anything else is refused with an error. */
+ * FP32, results rounded to bfloat16 once.  These run the split and the
+ * TMA-staged shear-warp kernels only: axis-aligned planograms with bin pitch
+ * equal to the voxel pitch.  From 10 slopes per call on: planogram rows of up
+ * to 512 and volume rows of up to 1024 elements, shifts below three rows per slope and plane, and for the
+ * backprojection an even N_u0, a planogram aligned to a pair of elements and
+ * at most 128 slopes.  Fewer slopes: 16-byte aligned buffers, volume and
+ * planogram rows that are multiples of 8 elements, and N_u0, numX <= 256 for
+ * the backprojection.  Anything else is refused with an error. */
 int petl_project_bf16_dev(const petl_geom* G, const void* f, void* g, int iv1_begin, int iv1_end, int iv0_first,
                           int iv0_step, void* stream);
 /* ratio = (P f == 0) ? 0 : meas / (P f), all three in bfloat16 */

@@ -326,8 +326,7 @@ k_bwd_zgather(const __grid_constant__ GMaps<NM> gmaps, float* __restrict__ B, co
                 unsigned char* st = smem + size_t(slot) * A.stage;
                 const float s0 = scale(2 * i), s1 = scale(min(2 * i + 1, GV1MAX - 1));
                 if (lane == 0 && pw == 0) {
-                    s_info[slot] = ZStage{2 * i, np | (i == 0 ? kZFirst : 0) | (i == nst - 1 ? kZLast : 0), p0, vi, r0,
-                                          col0, s0, s1};
+                    s_info[slot] = ZStage{2 * i, np | (i == nst - 1 ? kZLast : 0), p0, vi, r0, col0, s0, s1};
                     if (BULK) {
                         fence_proxy_async_smem();
                         mbar_arrive_expect_tx(&full[slot], uint32_t(np) * (uint32_t(sizeof(GRec)) +

@@ -1,11 +1,13 @@
 // BF16-storage entry points: volumes and planograms held in bfloat16 (half
 // the bytes of FP32), footprints accumulated in FP32.  No reference
 // counterpart (the reference stores float32 only); they serve the storage
-// precision study and memory-bound serving.  They run the TMA-staged
-// shear-warp kernels only, so the geometry must be axis-aligned with voxel
-// pitch equal to bin pitch, and the volume rows and planogram rows must be
-// multiples of 8 elements (16 bytes); other geometries are refused with an
-// error rather than converted behind the caller's back.
+// precision study and memory-bound serving.  They run the split and the
+// TMA-staged shear-warp kernels only, so the geometry must be axis-aligned
+// with voxel pitch equal to bin pitch; from 10 slopes per call on planogram rows
+// of up to 512 and volume rows of up to 1024 elements pass, below (and where scratch cannot be allocated) the
+// volume and planogram rows must be multiples of 8 elements (16 bytes) from
+// aligned bases.  Other calls are refused with an error rather than converted
+// behind the caller's back.
 #include <cuda_bf16.h>
 
 #include <string>
@@ -38,9 +40,9 @@ int bf16_result(int rc, const char* what, shear::TableBuf& tb, cudaStream_t st)
     cudaFreeAsync(tb.base, st);
     if (rc == shear::kNotApplicable) {
         set_error(std::string(what) +
-                  ": BF16 storage needs 16-byte aligned buffers, volume and planogram rows that are multiples of 8 "
-                  "elements, N_u0 and numX at most 256 for the backprojection, and slope spreads within the tile "
-                  "bounds");
+                  ": BF16 storage needs a planogram aligned to a pair of elements, volume rows of at most 1024 and slope "
+                  "spreads within the tile bounds; with fewer than 10 slopes 16-byte aligned buffers, volume and "
+                  "planogram rows that are multiples of 8 elements, N_u0 and numX at most 256 for the backprojection");
         return -1;
     }
     if (rc == 0) note_path(2);

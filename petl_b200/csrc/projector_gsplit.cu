@@ -1,7 +1,8 @@
-// Split forward projector for any psi (voxel height equal to the u1 bin
-// pitch), the counterpart of the shear-warp split kernels
-// (projector_split.cu) for orientations whose rays are not parallel to a
-// volume axis.
+// Split forward projector for any psi with voxel height equal to the u1 bin
+// pitch, the counterpart of the shear-warp split kernels (projector_split.cu)
+// for orientations whose rays are not parallel to a volume axis; and, further
+// down, for unequal height and pitch at psi = 0 and 90 (k_uz in place of k_gz)
+// with its exact transpose (k_backproject_uz).
 //
 // The reference footprint (src/projectors.cu:11-238) of a ray at its
 // driving plane p (y = const for a y-driven view, x = const for an
@@ -14,11 +15,11 @@
 //   X[v0][p][z][u0]   = sum_a w0(t, a, u0) f(z, p, a),
 // and the two sums run as two kernels:
 //
-// * k_gx: a block stages 8 volume rows of plane p (from the volume, or from
-//   its x/y-transposed copy for x-driven views) in shared memory; a thread
-//   per column u0 evaluates the u0 taps of its ray on plane p once (the
-//   reference's tap range and box overlaps, taps with a positive weight)
-//   and applies them to the 8 rows.
+// * k_gx: a block stages 32 volume rows of plane p (8 of long axes; from the
+//   volume, or from its x/y-transposed copy for x-driven views) in shared
+//   memory for all views of the chunk; a thread per column u0 evaluates the u0
+//   taps of its ray on plane p once (the reference's tap range and box
+//   overlaps, taps with a positive weight) and applies them to the rows.
 // * k_gz: CTA = one view x 16 slopes x 64 rows x 32 columns, 16 warps of
 //   2 slopes x 32 rows, one column per lane (a last block of at most 8
 //   slopes as 8 slopes x 128 rows).  With equal pitch the u1 taps
@@ -862,8 +863,9 @@ int backproject_usplit_adjoint(const petl_geom& G, const float* g, float* f, int
 }
 
 // kNotApplicable when the layout rules fail (the caller then runs the
-// general kernel): voxel height != u1 pitch, a view whose shift range over a
-// tile exceeds the staged rows, or scratch that cannot be allocated.
+// general kernel): voxel height != u1 pitch off the axes, a view whose shift
+// range over a tile exceeds the staged rows, or scratch that cannot be
+// allocated.
 int project_gsplit(const petl_geom& G, const float* f, float* g, const ViewRange& vr, const float* meas,
                    cudaStream_t st)
 {

@@ -245,7 +245,6 @@ template <class TG, int NM, int NV, int NK>
 __global__ void __launch_bounds__(kZThreads, 1)
 k_fwd_zsum(const __grid_constant__ ZMaps maps, const __grid_constant__ ZsumArgs A)
 {
-    constexpr int WN = NK + kZSpread + 1;
     extern __shared__ __align__(128) unsigned char smem[];
     ZCtl* ctl = reinterpret_cast<ZCtl*>(smem + size_t(A.ns) * A.stage);
     ZStage* s_info = ctl->info;
@@ -337,8 +336,8 @@ k_fwd_zsum(const __grid_constant__ ZMaps maps, const __grid_constant__ ZsumArgs 
                     }
                     const int slot = j % ns, y = ya + K.pps * i, np = max(0, min(K.pps, ye - y));
                     unsigned char* st = smem + size_t(slot) * A.stage;
-                    s_info[slot] = ZStage{y, np | edge | (i == 0 ? kZFirst : 0) | (i == nst - 1 ? kZLast : 0), v1a, vi,
-                                          row0, col0, 0.0f, 0.0f};
+                    s_info[slot] =
+                        ZStage{y, np | edge | (i == nst - 1 ? kZLast : 0), v1a, vi, row0, col0, 0.0f, 0.0f};
                     fence_proxy_async_smem();
                     mbar_arrive_expect_tx(&full[slot], uint32_t(np) * (box + uint32_t(sizeof(ZRec))));
                     for (int h = 0; h < np; h++)
