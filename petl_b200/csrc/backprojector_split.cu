@@ -25,10 +25,9 @@
 // at v1 = 0 (the rebinned planogram of FBP) takes k_bwd_zflat: its z sums
 // do not depend on the plane.
 //
-// 256x256x128, planogram (65, 129, 128, 256): 7.9 ms for the z taps and 0.9
-// for the x pass (before: 12.5 and 0.9, with one 16-warp CTA per tile, tables
-// built by every CTA and scalar FMAs).  FBP's single slope: 0.42 ms (0.72 with
-// a thread per x).
+// 256x256x128, planogram (65, 129, 128, 256): 8.82 ms, of which 7.8 the z taps
+// (before: 13.4 and 12.5, with one 16-warp CTA per tile, tables built by every
+// CTA and scalar FMAs).  FBP's single slope: 0.46 ms (0.73 with a thread per x).
 // Every wait is bounded: a wait that gives up sets the device error word, the
 // CTA drains its copies in flight and returns without writing.
 #include <cuda.h>
@@ -213,11 +212,10 @@ __global__ void __launch_bounds__(256) k_gather_records(const ZgatherArgs A, int
 // that a voxel of those planes reads), a warp sums NV planes x NK rows x 2
 // columns per lane over the slopes that reach the tile, and the producer
 // stages the planogram rows of two slopes at a time with their table records.
-// Bound as k_fwd_zsum by FP32 issue (measured 820 cycles per slope for 576 of
-// packed FMAs).  At the edges of the visible range (a quarter to a third of
-// the (warp, slope) pairs) the taps are predicated per output row (reference
-// semantics) or take zeros for masked window rows (adjoint), a plane at a
-// time.
+// Bound as k_fwd_zsum (FMA pipe active on 44 % of cycles, issue slots on 58 %).
+// At the edges of the visible range the taps are predicated per output row
+// (reference semantics) or take zeros for masked window rows (adjoint), a
+// plane at a time.
 //
 // TG: planogram storage (float or bfloat16); B and the arithmetic are FP32.
 // BULK: planogram rows are multiples of 16 bytes and arrive by a tiled TMA copy

@@ -18,10 +18,9 @@
 //   slope to slope, so they form one of 15 monotone patterns: one dispatch per
 //   run of planes with the same one selects a fully unrolled form.
 //
-// 256x256x128, planogram (65, 129, 128, 256): 7.0 ms for the z taps and 0.7
-// for the x pass (before: 10.0 and 0.9, with one 16-warp CTA per tile, tables
-// built by every CTA, scalar FMAs on 8 rows per warp and tiles that started at
-// bin 0).  What the steps gave on the z taps: twelve warps x 12 rows against
+// 256x256x128, planogram (65, 129, 128, 256): 7.85 ms, of which 6.8 the z taps
+// (before: 10.9 and 10.0, with one 16-warp CTA per tile, tables built by every
+// CTA, scalar FMAs on 8 rows per warp and tiles that started at bin 0).  What the steps gave on the z taps: twelve warps x 12 rows against
 // eight x 16 9 %, tiles handed out by a counter against a fixed stride 18 % (the
 // stride of 148 met the period of the column blocks, whose last is often
 // empty), a rolled epilogue 10 %, twelve rows at a time against four 4 %, runs of
@@ -233,13 +232,14 @@ __global__ void __launch_bounds__(256) k_xshift(float* __restrict__ X, const Xsh
 // consumers across tile borders, so set-up and epilogue of a warp overlap the
 // sums of the others.
 //
-// Bound by FP32 issue: a plane costs a warp 96 packed FMAs (192 cycles of its
-// scheduler, which holds three such warps) and 16 eight-byte window loads (32
-// cycles of the SM's shared memory, of which twelve warps take 384 of the 576
-// cycles the FMAs take).  Measured 830 cycles per plane: the dispatch, the
-// window's first loads and the ring's waits are not fully covered.  4 slopes x
-// 16 rows in eight warps need fewer loads per FMA but ran at 800 cycles for
-// 512 of FMAs; 8 rows and 16 warps are bound by the loads.
+// Bound by the FMA pipe and what three warps per scheduler cannot hide: a plane
+// costs a warp 96 packed FMAs (192 cycles of its scheduler, which holds three
+// such warps) and 16 eight-byte window loads (32 cycles of the SM's shared
+// memory, of which twelve warps take 384 of the 576 cycles the FMAs take).
+// The FMA pipe is active on 41-48 % of cycles (256x256x128, 26 views): the
+// dispatch, the window's first loads, the ring's waits and the masked parts of
+// tiles are not covered.  4 slopes x 16 rows in eight warps need fewer loads
+// per FMA but ran 9 % slower; 8 rows and 16 warps are bound by the loads.
 // TG: planogram storage (float or bfloat16); X and the arithmetic are FP32.
 template <class TG, int NM, int NV, int NK>
 __global__ void __launch_bounds__(kZThreads, 1)
@@ -424,8 +424,7 @@ k_fwd_zsum(const __grid_constant__ ZMaps maps, const __grid_constant__ ZsumArgs 
                     // the offsets of consecutive slopes are monotone and (four
                     // slopes) at most one row apart: one dispatch over the
                     // patterns that occur for each run of planes with the same
-                    // one (a jump to another pattern's code costs a quarter of
-                    // the time a plane's taps take)
+                    // one (forward at 256x256x128 8.4 ms with a jump per plane, 7.8 so)
                     while (left > 0) {
 #define PETL_ZCASE(PC)                        \
     case PC:                                  \
