@@ -260,24 +260,28 @@ k_bwd_zgather(const __grid_constant__ GMaps<NM> gmaps, float* __restrict__ B, co
             const bool ok = round == 0 || ring_wait(&empty[slot], uint32_t((round - 1) & 1), A.err, s_abort, A.wait_limit);
             return __all_sync(0xffffffffu, ok && *s_abort == 0) != 0;
         };
-        int after = 0;  // the tile after the current one (first lane)
         int turn = 0;
-        // the next tile, or -1 once a wait gave up.  Several producer warps
-        // meet here after every tile, a warp that gave up included (each gets
-        // here in bounded time), and leave together.
+        // the next tile, taken when this one is staged (k_fwd_zsum), or -1 once
+        // a wait gave up.  Several producer warps meet here after every tile,
+        // a warp that gave up included (each gets here in bounded time), and
+        // leave together.
         auto next_tile = [&]() {
-            if (BULK) return dead ? -1 : __shfl_sync(0xffffffffu, after, 0);
-            if (dead) *s_abort = 1;
-            turn ^= 1;
-            if (pw == 0 && lane == 0) ctl->tile[turn] = after;
-            if (producers_or(dead)) {
-                dead = true;
-                return -1;
+            if constexpr (BULK) {
+                int t = -1;
+                if (lane == 0 && !dead) t = int(gridDim.x) + atomicAdd(A.next, 1);
+                return __shfl_sync(0xffffffffu, t, 0);
+            } else {
+                if (dead) *s_abort = 1;
+                turn ^= 1;
+                if (pw == 0 && lane == 0) ctl->tile[turn] = int(gridDim.x) + atomicAdd(A.next, 1);
+                if (producers_or(dead)) {
+                    dead = true;
+                    return -1;
+                }
+                return ctl->tile[turn];
             }
-            return ctl->tile[turn];
         };
         for (int tile = blockIdx.x; unsigned(tile) < unsigned(A.ntile); tile = next_tile()) {
-            if (pw == 0 && lane == 0) after = int(gridDim.x) + atomicAdd(A.next, 1);
             int t = tile;
             const int colblk = t % A.n_colblk;
             t /= A.n_colblk;
