@@ -818,7 +818,7 @@ int backproject_split_m(const petl_geom& G, const Members& M0, int mode, int acc
     A.T = T;
     A.err = err;
     A.wait_limit = wait_limit();
-    // twelve consumer warps, four where twelve would leave SMs without a tile
+    // twelve consumer warps, or four where these have few tiles (ztwelve)
     for (A.nw = kZWarps;; A.nw = 4) {
         A.pg = NV == 4 || A.nw == 4 ? 4 : 6;
         A.rg = A.nw / A.pg;
@@ -829,16 +829,20 @@ int backproject_split_m(const petl_geom& G, const Members& M0, int mode, int acc
         const long long nt = (long long)nv * nb * A.n_plblk * A.n_rowblk * A.n_colblk;
         if (nt > (1 << 30)) return kNotApplicable;
         A.ntile = int(nt);
-        if (A.nw == 4 || A.ntile >= sm_count()) break;
+        if (A.nw == 4 || ztwelve(A.ntile)) break;
     }
     if (A.n_rowblk > 65535) return kNotApplicable;  // k_gather_records grid.y
     A.nrb = A.rows + 1 + shift_spread(A.planes - 1, step);
     if (A.nrb > 250) return kNotApplicable;  // TMA box rows
     A.sbytes = (A.nrb + kZSpread) * kZCols * EB;  // a multiple of 128
     A.stage = (2 * A.sbytes + 2 * int(sizeof(GRec)) + 127) & ~127;
-    A.ns = std::min(kZStages, (227 * 1024 - int(sizeof(ZCtl))) / A.stage);
+    int ctas = zctas(A.nw, A.ntile);  // a ring that does not fit half an SM takes the whole
+    for (;; ctas = 1) {
+        A.ns = std::min(kZStages, (zsmem(ctas) - zctl_bytes(A.nw)) / A.stage);
+        if (A.ns >= 2 || ctas == 1) break;
+    }
     if (A.ns < 2) return kNotApplicable;
-    const size_t smem = size_t(A.ns) * A.stage + sizeof(ZCtl);
+    const size_t smem = size_t(A.ns) * A.stage + zctl_bytes(A.nw);
 
     GMaps<kMaxMembers> maps;
     std::memset(&maps, 0, sizeof(maps));
@@ -912,7 +916,7 @@ int backproject_split_m(const petl_geom& G, const Members& M0, int mode, int acc
         A.M = M;
         A.nslot = nvc * nb;
         A.ntile = A.nslot * A.n_plblk * A.n_rowblk * A.n_colblk;
-        const unsigned grid = unsigned(std::min(A.ntile, sm_count()));
+        const unsigned grid = unsigned(std::min(A.ntile, ctas * sm_count()));
         using std::integral_constant;
         if (bulk)
             e = NV == 4 ? launch(std::true_type{}, integral_constant<int, 4>{}, integral_constant<int, 12>{}, grid)

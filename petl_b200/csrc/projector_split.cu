@@ -550,6 +550,7 @@ k_fwd_zsum(const __grid_constant__ ZMaps maps, const __grid_constant__ ZsumArgs 
 struct ZPlan {
     ZsumArgs A;
     int nv, nk;        // slopes and rows per warp
+    int ctas;          // CTAs per SM
     size_t smem;
     size_t table_bytes;
 };
@@ -574,9 +575,8 @@ bool zsum_plan(const petl_geom& G, const ViewRange& vr, const ShiftStep& step, i
     if (shift_spread(P.nv - 1, step) > kZSpread) return false;
     const int nv1 = vr.iv1_end - vr.iv1_begin;
     const int ngrp = int(ceil_div(nv1, P.nv));
-    // Twelve consumer warps; four where twelve would leave SMs without a tile
-    // (an ordered subset of a small volume: a third of the rows per tile, and a
-    // warp alone on its scheduler).
+    // twelve consumer warps, or four where these have few tiles (ztwelve)
+    int tiles = 0;
     for (A.nw = kZWarps;; A.nw = 4) {
         const int sg = P.nv == 4 || A.nw == 4 ? 4 : 6;
         // full blocks of sg slope groups; a tail of at most half a block
@@ -584,7 +584,7 @@ bool zsum_plan(const petl_geom& G, const ViewRange& vr, const ShiftStep& step, i
         const int ntail = ngrp % sg;
         const int tail_sg = ntail == 0 ? 0 : ntail == 1 ? 1 : 2 * ntail <= sg ? sg / 2 : 0;
         const int v1_split = tail_sg ? vr.iv1_begin + (ngrp - ntail) * P.nv : vr.iv1_end;
-        int tiles = 0;
+        tiles = 0;
         for (int i = 0; i < 2; i++) {
             ZKind& K = A.k[i];
             K.v1_first = i ? v1_split : vr.iv1_begin;
@@ -612,22 +612,26 @@ bool zsum_plan(const petl_geom& G, const ViewRange& vr, const ShiftStep& step, i
             K.ntile = int(nt);
             tiles += K.ntile;
         }
-        if (A.nw == 4 || tiles >= sm_count()) break;
+        if (A.nw == 4 || ztwelve(tiles)) break;
     }
     // four planes per stage (longer runs of one pattern, fewer waits) where
-    // three stages fit, else two; the tail's tall planes one or two at a time
-    for (int pps = 4;; pps = 2) {
-        A.k[0].pps = pps;
-        A.k[1].pps = std::max(1, std::min(pps, A.k[0].nblk ? pps * A.k[0].pstride / A.k[1].pstride : 2));
-        A.rec_off = 0;
-        for (const ZKind& K : A.k)
-            if (K.nblk > 0) A.rec_off = std::max(A.rec_off, K.pstride * K.pps * 4);
-        A.stage = (A.rec_off + pps * int(sizeof(ZRec)) + 127) & ~127;
-        A.ns = std::min(kZStages, (227 * 1024 - int(sizeof(ZCtl))) / A.stage);
-        if (A.ns >= 3 || pps == 2) break;
+    // three stages fit, else two; the tail's tall planes one or two at a time.
+    // A ring that does not fit half an SM takes the whole
+    for (P.ctas = zctas(A.nw, tiles);; P.ctas = 1) {
+        for (int pps = 4;; pps = 2) {
+            A.k[0].pps = pps;
+            A.k[1].pps = std::max(1, std::min(pps, A.k[0].nblk ? pps * A.k[0].pstride / A.k[1].pstride : 2));
+            A.rec_off = 0;
+            for (const ZKind& K : A.k)
+                if (K.nblk > 0) A.rec_off = std::max(A.rec_off, K.pstride * K.pps * 4);
+            A.stage = (A.rec_off + pps * int(sizeof(ZRec)) + 127) & ~127;
+            A.ns = std::min(kZStages, (zsmem(P.ctas) - zctl_bytes(A.nw)) / A.stage);
+            if (A.ns >= 3 || pps == 2) break;
+        }
+        if (A.ns >= 2 || P.ctas == 1) break;
     }
     if (A.ns < 2) return false;
-    P.smem = size_t(A.ns) * A.stage + sizeof(ZCtl);
+    P.smem = size_t(A.ns) * A.stage + zctl_bytes(A.nw);
     const size_t nrec = size_t(A.k[0].nblk + A.k[1].nblk) * G.numY;
     P.table_bytes = nrec * (sizeof(ZRec) + sizeof(int)) + sizeof(int);
     return true;
@@ -756,7 +760,7 @@ int project_split_m(const petl_geom& G, const Members& M0, const ViewRange& vr, 
         A.nslot = nvc * nb;
         int tiles = 0;
         for (ZKind& K : A.k) tiles += K.ntile = A.nslot * K.nblk * K.n_rowblk * A.n_colblk;
-        kz<<<std::min(tiles, sm_count()), 32 * (A.nw + 4), P.smem, st>>>(maps, A);
+        kz<<<std::min(tiles, P.ctas * sm_count()), 32 * (A.nw + 4), P.smem, st>>>(maps, A);
         note_launch();
         e = cudaGetLastError();
         if (e == cudaSuccess && hook && hook->fn) hook->fn(hook->ctx, vi0, nvc);

@@ -8,6 +8,7 @@
 
 #include <cstdint>
 
+#include "common.cuh"
 #include "tma.cuh"
 
 namespace petl {
@@ -186,14 +187,29 @@ constexpr int kZOut = 12;
 struct ZCtl {
     ZStage info[kZStages];
     uint64_t full[kZStages], empty[kZStages];
-    // a warp's epilogue passes its accumulators through here, twelve rows at a
+    int abort;  // a warp gave up a wait: start no further copies
+    int tile[2];  // the producer warps' next tile, by turns
+    // (the CTA's consumer warps only) a warp's epilogue passes its accumulators through here, twelve rows at a
     // time, so that the code that scales, masks and stores them is one rolled
     // loop: unrolled over all accumulators it was tens of KB of straight code
     // per tile, and its instruction fetches took a fifth of the forward's time
     f2x out[kZWarps][kZOut][32];
-    int abort;  // a warp gave up a wait: start no further copies
-    int tile[2];  // the producer warps' next tile, by turns
 };
+constexpr int zctl_bytes(int nw) { return int(sizeof(ZCtl)) - (kZWarps - nw) * kZOut * 32 * int(sizeof(f2x)); }
+
+// Whether a launch of so many tiles of twelve-warp CTAs takes these, or tiles
+// of a third of the rows in four-warp CTAs, two of which share an SM where
+// there are more of them than SMs (registers: 256 threads of 128; shared memory:
+// 228 KB per SM, 1 KB per CTA reserved).  A tile's time is latency below a full
+// chip, so smaller tiles on more SMs win until twelve-warp tiles fill about
+// two thirds of them.  Forward of 4000 panels at psi = 0, time of twelve-warp
+// tiles over four-warp ones by number of tiles: 20-40 1.09, 60-80 1.07, 80-100
+// 1.04, 100-120 1.02, 120-148 0.97, 200-296 0.96, 400 0.88; two CTAs per SM
+// against one, where four-warp tiles outnumber SMs: 1.06 at 80-100 tiles, 1.13
+// at 120-148.
+inline bool ztwelve(int tiles) { return 3 * tiles >= 2 * sm_count(); }
+inline int zctas(int nw, int tiles) { return nw == 4 && tiles > sm_count() ? 2 : 1; }
+constexpr int zsmem(int ctas) { return (228 / ctas - 1) * 1024; }
 
 // Rows 12 * (i % (NK / 12)) .. + 11 of accumulator block i / (NK / 12) to the
 // warp's lane slots.

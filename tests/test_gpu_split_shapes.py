@@ -6,7 +6,7 @@ kernel in the backward, that the others do not have); which launch shape each
 case takes is in tests/test_split_bounds.py.  The cases sit where
 a shape or a rule changes: slopes steeper than one row per plane or slope
 (two per warp), planogram rows that are no multiple of 16 bytes (staged by
-column pairs), few tiles (four consumer warps), slope tails of one group,
+column pairs), few tiles (four consumer warps, one or two CTAs per SM), slope tails of one group,
 half a block and more, ragged and off-centre volumes, masked columns on
 either side, psi = 90, view subsets and slope ranges."""
 import pytest
@@ -22,6 +22,7 @@ CASES = {
     "steepest_planes": ((0.0, 60.0, 64.0, 190.0, 2.0, 0.6, 2.5), (36, 58, 98, 2.0)),         # 2.5, 50-column rows
     "tall_voxels": ((0.0, 120.0, 60.0, 60.0, 2.0, 0.6, 0.5), (60, 130, 30, 2.0)),           # steep, 66-column rows
     "rag90": ((90.0, 115.0, 71.0, 65.0, 1.5, 0.45, 0.2), (75, 71, 38, 1.5, 1.5, 3.0, -4.5, 1.5)),
+    "few_tiles": ((0.0, 250.0, 48.0, 56.0, 1.5, 0.5, 0.25), (64, 64, 32, 1.5)),             # a subset of 8: two CTAs per SM
     "wide": ((0.0, 300.0, 128.0, 32.0, 1.0, 0.5, 0.25), (130, 40, 20, 1.0)),                # 278 columns, volume narrower
     "one_row_block": ((0.0, 128.0, 64.0, 13.0, 1.0, 0.3, 0.1), (30, 34, 11, 1.0, 1.0, 6.0, 0.0, 0.0)),
 }

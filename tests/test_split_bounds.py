@@ -258,7 +258,7 @@ def test_four_per_window_only_where_neighbours_differ_by_a_row():
 
 def _split_form(F, n_views, n_slopes, forward, sms=148):
     """The launch shape that the host picks on the axes: slopes (planes) per
-    warp, consumer warps, slope groups of the forward's tail."""
+    warp, consumer warps, slope groups of the forward's tail, CTAs per SM."""
     (_, four_f, _), (_, four_b, _) = _shift_rule(F)
     cd = lambda a, b: -(-a // b)  # noqa: E731
     cols = cd(F["N_u0"], 64)
@@ -274,19 +274,19 @@ def _split_form(F, n_views, n_slopes, forward, sms=148):
                         for n, sg in ((full, groups), (1 if tail else 0, max(tail, 1)))) * n_views * cols
         else:
             tiles = n_views * cols * cd(F["numY"], nv * groups) * cd(F["numZ"], nk * (nw // groups))
-        if tiles >= sms:
+        if 3 * tiles >= 2 * sms:
             break
-    return nv, nw, tail
+    return nv, nw, tail, 2 if nw == 4 and tiles > sms else 1
 
 
 def test_split_shape_cases_cover_the_launch_shapes():
     """tests/test_gpu_split_shapes.py runs every launch shape of the split z
-    kernels: four and two slopes (planes) per warp, twelve and four warps, each
-    with rows that are multiples of 16 bytes and that are not, and tails of
+    kernels: four and two slopes (planes) per warp, twelve and four warps (one
+    and two CTAs per SM), each with rows that are multiples of 16 bytes and that are not, and tails of
     one group and of half a block."""
     from petl_b200 import Geometry
     from test_gpu_split_shapes import CASES as SHAPES
-    fwd, bwd, tails = set(), set(), set()
+    fwd, bwd, tails, bctas = set(), set(), set(), set()
     for args, vol in SHAPES.values():
         P = Geometry(*args, volume=vol).g
         F = {k: getattr(P, k) for k, _ in P._fields_}
@@ -295,10 +295,13 @@ def test_split_shape_cases_cover_the_launch_shapes():
                 -(F["x_0"] + (F["numX"] - 1) * F["T_x"])
         for sub, drop in (((0, 1), 0), ((1, 3), 0), ((2, 8), 3)):
             views = len(range(sub[0], F["N_v0"], sub[1]))
-            nv, nw, tail = _split_form(F, views, F["N_v1"] - drop, True)
-            fwd.add((nv, nw))
+            nv, nw, tail, ctas = _split_form(F, views, F["N_v1"] - drop, True)
+            fwd.add((nv, nw, ctas))
             tails.add((nv, nw, tail))
-            bwd.add(_split_form(F, views, F["N_v1"] - drop, False)[:2] + (F["N_u0"] % 4 == 0,))
-    assert fwd == {(4, 12), (4, 4), (2, 12), (2, 4)}
+            nv, nw, _, ctas = _split_form(F, views, F["N_v1"] - drop, False)
+            bwd.add((nv, nw, F["N_u0"] % 4 == 0))
+            bctas.add((nv, nw, ctas))
+    assert fwd == {(4, 12, 1), (4, 4, 1), (4, 4, 2), (2, 12, 1), (2, 4, 1), (2, 4, 2)}
     assert bwd == {(nv, nw, a) for nv in (4, 2) for nw in (12, 4) for a in (True, False)}
+    assert bctas == {(4, 12, 1), (4, 4, 1), (4, 4, 2), (2, 12, 1), (2, 4, 1), (2, 4, 2)}
     assert {(4, 12, 1), (2, 4, 1), (2, 4, 2), (2, 12, 3)} <= tails
