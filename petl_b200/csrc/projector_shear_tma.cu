@@ -630,7 +630,9 @@ k_bwd_tma(const __grid_constant__ CUtensorMap gmap, const TG* __restrict__ gsrc,
     // weights of view v0: (S w0, S w1) per live slope and plane.  The global
     // loads of S for the next view are issued at the start of a view
     // (load_S) and stored after its stages (store_w), so their latency hides
-    // behind the view's work; at most kWPT elements per thread.
+    // behind the view's work; kWPT elements per thread, which is all of them
+    // with 512 threads (the elements beyond that, of CTAs for short rows, are
+    // loaded where they are stored).
     constexpr int kWPT = (BV1CAP * NP + 511) / 512;
     float s_pre[kWPT];
     auto load_S = [&](int v0) {
@@ -640,7 +642,7 @@ k_bwd_tma(const __grid_constant__ CUtensorMap gmap, const TG* __restrict__ gsrc,
             s_pre[i] = e < nlive * NP ? __ldg(&A.T.S[size_t(s_v1[e / NP]) * G.N_v0 + v0]) : 0.0f;
         }
     };
-    auto store_w = [&]() {
+    auto store_w = [&](int v0) {
 #pragma unroll
         for (int i = 0; i < kWPT; i++) {
             const int e = tid + i * int(blockDim.x);
@@ -648,6 +650,10 @@ k_bwd_tma(const __grid_constant__ CUtensorMap gmap, const TG* __restrict__ gsrc,
                 const float S = s_pre[i], w = s_w[e];
                 Wt[e] = make_float2(S * (1.0f - w), S * w);
             }
+        }
+        for (int e = tid + kWPT * int(blockDim.x); e < nlive * NP; e += blockDim.x) {
+            const float S = __ldg(&A.T.S[size_t(s_v1[e / NP]) * G.N_v0 + v0]), w = s_w[e];
+            Wt[e] = make_float2(S * (1.0f - w), S * w);
         }
     };
     // x shifts of the CTA's planes for every view, staged once
@@ -700,7 +706,7 @@ k_bwd_tma(const __grid_constant__ CUtensorMap gmap, const TG* __restrict__ gsrc,
     if (my_next < ns - 1) my_next += nwarps;
     if (n_v0 > 0) {
         load_S(A.vr.iv0_first);
-        store_w();
+        store_w(A.vr.iv0_first);
     }
     __syncthreads();
 
@@ -827,7 +833,7 @@ k_bwd_tma(const __grid_constant__ CUtensorMap gmap, const TG* __restrict__ gsrc,
                 Fv[q][k] += fmaf(wx1, zm, wx0 * z0);
             }
         }
-        if (iv + 1 < n_v0) store_w();
+        if (iv + 1 < n_v0) store_w(v0 + A.vr.iv0_step);
         __syncthreads();
     }
     if (aborted) {

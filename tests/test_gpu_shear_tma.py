@@ -233,3 +233,28 @@ def test_single_slope_backprojection(cuda, name, mode):
     assert L.petl_device_error_flag() == 0
     want = _np(base) + 0.5 * a
     assert np.abs(_np(out) - want).max() <= 1e-6 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("mode", ["reference", "adjoint"])
+@pytest.mark.parametrize("cols,slopes", [(26, 19), (32, 41), (58, 45)])
+def test_narrow_planograms_with_many_slopes(cuda, cols, slopes, mode):
+    """The single-pass backprojector's CTAs for short rows have fewer threads
+    than ray scales (slopes x planes) to load: every one counts, against the
+    first-generation kernel (sums in another order)."""
+    import torch
+    from petl_b200 import Geometry, lib, ops
+    # R = 56 bins, steepest slope (slopes - 1) / 2 bins over R
+    G = Geometry(0.0, 112.0, cols - 16.0 + 0.5, 100.0, 1.0, 8.0 / 56.0, (slopes - 0.5) / 112.0, volume=(21, 23, 14, 1.0))
+    assert G.shape[0] == slopes and G.shape[3] == cols
+    g = torch.rand(G.shape, device=cuda, generator=torch.Generator(device=cuda).manual_seed(8)) + 0.1
+    L = lib()
+    out = {}
+    try:
+        for d in (2, 3):
+            assert L.petl_set_dispatch(d) == 0
+            out[d] = ops.backproject(G, g, mode=mode)
+            assert L.petl_last_projector_path() == d - 1
+    finally:
+        L.petl_set_dispatch(0)
+    assert L.petl_device_error_flag() == 0
+    assert float((out[3] - out[2]).norm() / out[2].norm()) < 1e-6
