@@ -1,9 +1,9 @@
 """The split forward for unequal voxel height and u1 pitch on an axis-aligned
 planogram against the FP64 oracle and the general kernels: bins taller and
 lower than voxels (0 to 3 whole voxels in a bin, the unrolled forms, and
-more), psi = 0 and 90, ragged and off-centre volumes, rays that miss the
-volume on most planes, a volume wider than the panels, view subsets, slope
-ranges and the MLEM ratio."""
+more), calls too small for the split form (a ray per thread), psi = 0 and 90,
+ragged and off-centre volumes, rays that miss the volume on most planes, a
+volume wider than the panels, view subsets, slope ranges and the MLEM ratio."""
 import numpy as np
 import pytest
 
@@ -21,6 +21,8 @@ CASES = {
     "one_whole": ((90.0, 100.0, 75.0, 27.0, 1.5, 0.45, 0.2), (52, 60, 18, 1.5, 1.1, 3.0, -4.5, 1.5), 3),
     "two_whole": ((0.0, 100.0, 40.0, 44.0, 2.0, 0.4, 0.2), (50, 20, 61, 0.9, 0.75), 3),
     "four_whole": ((0.0, 100.0, 40.0, 44.0, 2.0, 0.4, 0.2), (30, 20, 90, 1.0, 0.45), 3),
+    "few_rays": ((0.0, 40.0, 12.0, 10.0, 1.6, 0.5, 0.25), (14, 12, 9, 1.0, 1.2, 1.0, 0.0, -2.0), 3),
+    "few_rays90": ((90.0, 40.0, 12.0, 10.0, 1.6, 0.5, 0.25), (13, 15, 21, 0.6, 0.45, -1.0, 2.0, 0.0), 3),
     "too_many_rows": ((0.0, 100.0, 40.0, 44.0, 4.0, 0.4, 0.2), (30, 20, 90, 1.0, 0.45), 0),
 }
 
