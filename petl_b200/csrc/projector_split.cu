@@ -18,7 +18,7 @@
 //   slope to slope, so they form one of 15 monotone patterns: one dispatch per
 //   run of planes with the same one selects a fully unrolled form.
 //
-// 256x256x128, planogram (65, 129, 128, 256): 7.85 ms, of which 6.8 the z taps
+// 256x256x128, planogram (65, 129, 128, 256): 7.88 ms, of which 6.8 the z taps
 // (before: 10.9 and 10.0, with one 16-warp CTA per tile, tables built by every
 // CTA, scalar FMAs on 8 rows per warp and tiles that started at bin 0).  What the steps gave on the z taps: twelve warps x 12 rows against
 // eight x 16 9 %, tiles handed out by a counter against a fixed stride 18 % (the
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(256) k_xshift(float* __restrict__ X, const Xsh
 // costs a warp 96 packed FMAs (192 cycles of its scheduler, which holds three
 // such warps) and 16 eight-byte window loads (32 cycles of the SM's shared
 // memory, of which twelve warps take 384 of the 576 cycles the FMAs take).
-// The FMA pipe is active on 41-48 % of cycles (256x256x128, 26 views): the
+// The FMA pipe is active on 44-48 % of cycles (256x256x128, 26 views): the
 // dispatch, the window's first loads, the ring's waits and the masked parts of
 // tiles are not covered.  4 slopes x 16 rows in eight warps need fewer loads
 // per FMA but ran 9 % slower; 8 rows and 16 warps are bound by the loads.
